@@ -950,9 +950,10 @@ static inline bool use_row_fft(const jgcm_mesh* m, int C, bool inverse = false) 
 }
 static inline size_t row_fft_smem(const jgcm_mesh* m) { return (size_t)RF_WARPS * 32 * (m->nlon + 1) * sizeof(float); }
 
-// Fourier -> spectral: Gaussian quadrature per m.  grid (ceil(Cout/CT), N+1), 256 threads.
-// Shared memory holds, for 4 input slots, the hemisphere-symmetric and -antisymmetric
+// Fourier -> spectral: Gaussian quadrature per m.  grid (ceil(Cout/CT), N+1, row chunks), <= 256 threads.
+// Shared memory holds, for the input slots in use, the hemisphere-symmetric and -antisymmetric
 // combinations g(mu_j) +/- g(-mu_j) of the tile's columns.
+constexpr int G2S_BLOCKS_PER_SM = 2;  // the row split's aim (launch_g2s)
 // four consecutive table weights in one 16-byte load (the address is 16-byte aligned: nh is a
 // multiple of 4 and the tables start aligned)
 __device__ __forceinline__ void ld4(const float* p, float (&w)[4]) {
@@ -967,39 +968,67 @@ __device__ __forceinline__ void ld4(const double* p, double (&w)[4]) {
 // QL lanes per output (4: a quad splits the latitude sum and combines it with two shuffles, for
 // launches too small to fill the device; 1: a lane sums its output alone, half the instructions per
 // output, for launches with many outputs).
+// A block takes CT columns of one m and RC of its rows n (blockIdx.z: which RC): a one-layer model has
+// one column per m, and with all rows in one block its analysis kept N + 1 of the SMs busy with a
+// serial load of three whole weight blocks, in a tile of 4 to 16 columns of which one was used
+// (barotropic T42 FP64 41.3 us, shallow water T85 FP32 33.2 us, FP64 163 us; with the rows split and
+// the tile no wider than the launch's columns 12.2, 12.3 and 31.6 us, launch and event included).  The weight rows are constants: they are staged by asynchronous copies before the
+// dependency wait, at a pitch one 16-byte chunk longer than a row, so that the rows read by a warp's
+// quads start in different banks.  Only the tables (`tabs`) and input slots (`slots`) that the plan
+// uses are staged.
+enum { G2S_TAB_PW = 1, G2S_TAB_AB = 2, G2S_TAB_P = 4 };
+__host__ __device__ inline int g2s_ntab(int tabs) { return (tabs & G2S_TAB_PW ? 1 : 0) + (tabs & G2S_TAB_AB ? 2 : 0) + (tabs & G2S_TAB_P ? 1 : 0); }
+__host__ __device__ inline int bits4(int x) { return (x & 1) + (x >> 1 & 1) + (x >> 2 & 1) + (x >> 3 & 1); }
+
 template <typename T, int QL>
 __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb, const V2<T>* __restrict__ F,
-                                                      int ns, int nlat, int Cin, int CT, int stage) {
-  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+                                                      int ns, int nlat, int Cin, int CT, int RC, int slots, int tabs,
+                                                      int stage) {
   using V = V2<T>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int m = blockIdx.y;
   const int nh = nlat >> 1;
-  const int K = ns + 1 - m;
+  const int r0 = blockIdx.z * RC, K = min(RC, ns + 1 - m - r0);  // rows n = m + r0 .. m + r0 + K - 1
+  if (K <= 0) return;
   const int C = plan.C;
   const int cbase = blockIdx.x * CT;
-  V* S = (V*)smem;              // [4][nh][CT] symmetric      (column fastest: no bank conflicts)
-  V* A = S + 4 * CT * nh;       // [4][nh][CT] antisymmetric
+  const int nslot = bits4(slots);
+  V* S = (V*)smem;                  // [nslot][nh][CT] symmetric  (column fastest: no bank conflicts)
+  V* A = S + nslot * CT * nh;       // [nslot][nh][CT] antisymmetric
   const size_t mrow = (size_t)m * (ns + 1);
-  // quadrature rows n = m..ns of this m ([K][nh]); staged once per block when they fit
-  const T* tPW = tb.PW + (mrow + m) * nh;
-  const T* tCA = tb.CA + (mrow + m) * nh;
-  const T* tCB = tb.CB + (mrow + m) * nh;
+  const size_t toff = (mrow + m + r0) * nh;
+  // quadrature rows of this block ([K][pitch]); staged once per block when they fit
+  const T *tPW = tb.PW + toff, *tCA = tb.CA + toff, *tCB = tb.CB + toff, *tP = tb.P + toff;
+  int wp = nh;
   if (stage) {
-    T* sPW = (T*)(A + 4 * CT * nh);
-    T* sCA = sPW + K * nh;
-    T* sCB = sCA + K * nh;
-    for (int i = threadIdx.x; i < K * nh; i += blockDim.x) {
-      sPW[i] = tPW[i];
-      sCA[i] = tCA[i];
-      sCB[i] = tCB[i];
+    constexpr int ce = 16 / (int)sizeof(T);
+    wp = nh + ce;
+    T* dst = (T*)(A + nslot * CT * nh);
+    const T* src[4] = {tPW, tCA, tCB, tP};
+    const T** use[4] = {&tPW, &tCA, &tCB, &tP};
+    const int nchunk = nh / ce;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      if (!(tabs & (t == 0 ? G2S_TAB_PW : t == 3 ? G2S_TAB_P : G2S_TAB_AB))) continue;
+      if (nh % ce == 0) {
+        for (int i = threadIdx.x; i < K * nchunk; i += blockDim.x) {
+          const int r = i / nchunk, c = i - r * nchunk;
+          cp_async16(dst + r * wp + c * ce, src[t] + (size_t)r * nh + c * ce);
+        }
+      } else {
+        for (int i = threadIdx.x; i < K * nh; i += blockDim.x) dst[i / nh * wp + i % nh] = src[t][i];
+      }
+      *use[t] = dst;
+      dst += RC * wp;
     }
-    tPW = sPW;
-    tCA = sCA;
-    tCB = sCB;
+    cp_async_commit();
   }
-  for (int i = threadIdx.x; i < 4 * CT * nh; i += blockDim.x) {
-    int slot = i / (CT * nh), rem = i - slot * CT * nh, jh = rem / CT, cl = rem - jh * CT, c = cbase + cl;
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  for (int i = threadIdx.x; i < nslot * CT * nh; i += blockDim.x) {
+    int pos = i / (CT * nh), rem = i - pos * CT * nh, jh = rem / CT, cl = rem - jh * CT, c = cbase + cl;
+    int slot = 0;  // the pos-th slot in use
+    for (int left = pos; slot < 3; slot++)
+      if ((slots >> slot & 1) && left-- == 0) break;
     V s, a;
     s.x = s.y = a.x = a.y = 0;
     if (c < C) {
@@ -1016,9 +1045,10 @@ __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb
         a.y = x.y - y.y;
       }
     }
-    S[(slot * nh + jh) * CT + cl] = s;
-    A[(slot * nh + jh) * CT + cl] = a;
+    S[i] = s;
+    A[i] = a;
   }
+  if (stage) cp_async_wait_all();
   __syncthreads();
   // each output is summed by QL threads (latitudes jh = q, q+QL, ...), then combined with masked
   // shuffles; the QL lanes never straddle loop iterations (blockDim is a multiple of 4)
@@ -1031,17 +1061,18 @@ __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb
   };
   for (int i = threadIdx.x; i < K * CT * QL; i += blockDim.x) {
     const int q = i & (QL - 1), o = i / QL;
-    int r = o / CT, cl = o - r * CT, n = m + r, c = cbase + cl;
+    int r = o / CT, cl = o - r * CT, n = m + r0 + r, c = cbase + cl;
     if (c >= C) continue;  // whole quad
     int k;
     const SpecOutGroup& g = group_of(plan.g, plan.ng, c, &k);
-    const bool even = (r & 1) == 0;
-    const T* pw = tPW + r * nh;
-    const T* ca = tCA + r * nh;
-    const T* cb = tCB + r * nh;
+    const bool even = ((r0 + r) & 1) == 0;
+    const T* pw = tPW + r * wp;
+    const T* ca = tCA + r * wp;
+    const T* cb = tCB + r * wp;
+    auto at = [&](int slot) { return bits4(slots & ((1 << slot) - 1)) * nh * CT + cl; };  // the slot's column
     const size_t sidx = (mrow + n) * g.L + k;
     auto plain = [&](int slot) -> V {
-      const V* src = (even ? S : A) + slot * nh * CT + cl;
+      const V* src = (even ? S : A) + at(slot);
       T sr = 0, si = 0;
       if (QL == 1) {  // a lane walks every latitude: weights four at a time, same order of sums
         for (int jh = 0; jh < nh; jh += 4) {
@@ -1072,8 +1103,8 @@ __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb
     };
     // alpha operator: i * sum CA (A) + sign * sum CB (B), all latitudes folded by parity
     auto alpha = [&](int slotA, int slotB, T sign) -> V {
-      const V* sa = (even ? S : A) + slotA * nh * CT + cl;
-      const V* sb = (even ? A : S) + slotB * nh * CT + cl;
+      const V* sa = (even ? S : A) + at(slotA);
+      const V* sb = (even ? A : S) + at(slotB);
       T ar = 0, ai = 0, br = 0, bi = 0;
       if (QL == 1) {  // weights four at a time, same order of sums
         for (int jh = 0; jh < nh; jh += 4) {
@@ -1110,8 +1141,8 @@ __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb
     };
     // adjoint of the synthesis: unweighted quadrature with P, c_m nlon, row N+1 kept
     auto plain_adj = [&]() -> V {
-      const V* src = (even ? S : A) + cl;
-      const T* p = tb.P + (mrow + n) * nh;
+      const V* src = (even ? S : A) + at(0);
+      const T* p = tP + r * wp;
       T sr = 0, si = 0;
 #pragma unroll 4
       for (int jh = q; jh < nh; jh += QL) {
@@ -1196,6 +1227,17 @@ static inline int fft_ct(const jgcm_mesh* m) {
   return m->tune[3] > 0 ? m->tune[3] : m->nlon >= 1024 ? 1 : 1024 / m->nlon;
 }
 
+// A tile no wider than a launch of C columns needs (halved while half of it still holds them all): the
+// tile's further columns would be transformed as zeros (barotropic T42 FP64, 2 and 3 columns in tiles of
+// 8: synthesis 14.5 -> 10.3 us, inverse FFT 14.4 -> 12.5 us, event included)
+static inline int fit_ct(int ct, int C) {
+  while (ct > 1 && ct / 2 >= C) ct /= 2;
+  return ct;
+}
+
+// threads of a shared-memory FFT block: one per butterfly of a stage, two warps at least
+static inline int fft_threads(const jgcm_mesh* m, int fc) { return std::max(64, std::min(256, fc * m->nlon / 4)); }
+
 // The plans' FP32 copies of their FP64 scalars (pick<T> in the kernels), filled here so that
 // every plan builder stays in FP64.
 static S2GPlan with_f32(const S2GPlan& p) {
@@ -1238,7 +1280,7 @@ static int launch_s2g_into(jgcm_mesh* m, const S2GPlan& sp0, const IFFTPlan& ip,
   const S2GPlan sp = with_f32(sp0);
   JG_TRY(configure_smem<T>());
   Tables<T> tb = tables<T>(m);
-  const int nh = m->nh, ct = s2g_ct(m);
+  const int nh = m->nh, ct = m->tune[1] ? s2g_ct(m) : fit_ct(s2g_ct(m), sp.C);
   if (std::is_same<T, float>::value && m->tc.on && !m->simt_legendre) {
     JG_TRY(launch_s2g_legendre_tc(m, sp, fbuf, st));
   } else {
@@ -1257,7 +1299,7 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
   using V = V2<T>;
   const IFFTPlan ip = with_f32(ip0);
   Tables<T> tb = tables<T>(m);
-  const int fc = fft_ct(m);
+  const int fc = m->tune[3] > 0 ? fft_ct(m) : fit_ct(fft_ct(m), ip.C);
   if (std::is_same<T, float>::value && use_row_fft(m, ip.C, true)) {  // many rows: a row per thread
     dim3 gr((ip.C + 32 * RF_WARPS - 1) / (32 * RF_WARPS), m->nlat);
     const Tables<float> tf = tables<float>(m);
@@ -1287,7 +1329,7 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
   }
   size_t sm2 = align16((size_t)(fc * m->nlon + m->nlon) * sizeof(T)) + (size_t)(m->N + 1) * fc * sizeof(V);
   dim3 g2((ip.C + fc - 1) / fc, m->nlat);
-  JG_CUDA(launch_pdl(k_ifft<T>, g2, 256, sm2, st, ip, tb, (const V*)fbuf, m->N, m->nlat, m->nlon, m->logn - 1, fc));
+  JG_CUDA(launch_pdl(k_ifft<T>, g2, fft_threads(m, fc), sm2, st, ip, tb, (const V*)fbuf, m->N, m->nlat, m->nlon, m->logn - 1, fc));
   mark(st);
   JG_CUDA(cudaGetLastError());
   return JGCM_OK;
@@ -1325,7 +1367,7 @@ int launch_fft_only(jgcm_mesh* m, const FFTPlan& fp0, cudaStream_t st, void* fbu
   }
   JG_ARG(fp.C <= cap && fp.C > 0, "bad FFT plan");
   Tables<T> tb = tables<T>(m);
-  const int fc = fft_ct(m);
+  const int fc = m->tune[3] > 0 ? fft_ct(m) : fit_ct(fft_ct(m), fp.C);
   if (std::is_same<T, float>::value && use_row_fft(m, fp.C)) {  // many rows: a row per thread
     dim3 gr((fp.C + 32 * RF_WARPS - 1) / (32 * RF_WARPS), m->nlat);
     const Tables<float> tf = tables<float>(m);
@@ -1368,7 +1410,7 @@ int launch_fft_only(jgcm_mesh* m, const FFTPlan& fp0, cudaStream_t st, void* fbu
   }
   size_t sm = (size_t)(fc * m->nlon + m->nlon) * sizeof(T);
   dim3 g((fp.C + fc - 1) / fc, m->nlat);
-  JG_CUDA(launch_pdl(k_fft<T>, g, 256, sm, st, fp, tb, (V*)fbuf, m->N, m->nlat, m->nlon, m->logn - 1, fc));
+  JG_CUDA(launch_pdl(k_fft<T>, g, fft_threads(m, fc), sm, st, fp, tb, (V*)fbuf, m->N, m->nlat, m->nlon, m->logn - 1, fc));
   mark(st);
   JG_CUDA(cudaGetLastError());
   return JGCM_OK;
@@ -1388,18 +1430,37 @@ int launch_g2s(jgcm_mesh* m, const FFTPlan& fp, const G2SPlan& gp0, cudaStream_t
   if (std::is_same<T, float>::value && m->tc.on && !adj && !m->simt_legendre)
     return launch_g2s_legendre_tc(m, gp, fp.C, st, fbuf);
   Tables<T> tb = tables<T>(m);
-  const int nh = m->nh, ct = g2s_ct(m);
-  size_t sm = (size_t)8 * ct * nh * sizeof(V);
-  const size_t tab = (size_t)3 * (m->ns + 1) * nh * sizeof(T);
-  const int stage = sm + tab <= kSmemBudget;
-  if (stage) sm += tab;
-  dim3 g((gp.C + ct - 1) / ct, m->N + 1);
+  const int nh = m->nh, K0 = m->ns + 1;
+  int slots = 0, tabs = 0;
+  for (int i = 0; i < gp.ng; i++) {
+    const SpecOutGroup& g = gp.g[i];
+    slots |= (g.colA >= 0) | (g.colB >= 0) << 1 | (g.colE >= 0) << 2 | (g.colH >= 0) << 3;
+    if (g.op == G2S_ADJ_S2G) tabs |= G2S_TAB_P;
+    else if (g.op == G2S_PLAIN) tabs |= G2S_TAB_PW;
+    else tabs |= G2S_TAB_AB | (g.colE >= 0 ? G2S_TAB_PW : 0);
+  }
   // one lane per output once the launch has outputs for every thread the device holds
   const size_t outputs = (size_t)gp.C * (m->N + 1) * (m->N + 2) / 2;
-  if (outputs >= (size_t)m->sm_count * 2048 && nh % 4 == 0)
-    JG_CUDA(launch_pdl(k_g2s_legendre<T, 1>, g, 256, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, stage));
+  const int ql = outputs >= (size_t)m->sm_count * 2048 && nh % 4 == 0 ? 1 : 4;
+  // the column tile, no wider than the launch's columns (unless it is tuned)
+  const int ct = m->tune[2] ? g2s_ct(m) : fit_ct(g2s_ct(m), gp.C);
+  // rows per block: all of an m's, or fewer where the launch would leave SMs without a block: halved
+  // while the grid has less than G2S_BLOCKS_PER_SM blocks per SM and a block more than one row per
+  // quad of a warp
+  const int tiles = (gp.C + ct - 1) / ct;
+  int rc = K0;
+  while ((size_t)tiles * (m->N + 1) * ((K0 + rc - 1) / rc) < (size_t)G2S_BLOCKS_PER_SM * m->sm_count && rc * ct * ql > 64)
+    rc = (rc + 1) / 2;
+  size_t sm = (size_t)2 * bits4(slots) * ct * nh * sizeof(V);
+  const size_t tab = (size_t)g2s_ntab(tabs) * rc * (nh + 16 / sizeof(T)) * sizeof(T);
+  const int stage = sm + tab <= kSmemBudget;
+  if (stage) sm += tab;
+  dim3 g(tiles, m->N + 1, (K0 + rc - 1) / rc);
+  const int threads = std::min(256, (rc * ct * ql + 31) / 32 * 32);
+  if (ql == 1)
+    JG_CUDA(launch_pdl(k_g2s_legendre<T, 1>, g, threads, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, rc, slots, tabs, stage));
   else
-    JG_CUDA(launch_pdl(k_g2s_legendre<T, 4>, g, 256, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, stage));
+    JG_CUDA(launch_pdl(k_g2s_legendre<T, 4>, g, threads, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, rc, slots, tabs, stage));
   mark(st);
   JG_CUDA(cudaGetLastError());
   return JGCM_OK;

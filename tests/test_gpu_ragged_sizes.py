@@ -1,0 +1,52 @@
+"""Every transform entry point at the edges of the launch rules: one column, column counts that fill no
+tile, latitude counts that are no power of two (and whose half is no multiple of a 16-byte chunk), rows
+of one m that do not divide into the row chunks.
+
+Tolerances: the transforms' own (tests/test_gpu_transforms.py): FP64 1e-12, FP32 5e-6 relative L2.
+"""
+import numpy as np
+import pytest
+
+from jgcm import configs
+from test_gpu_transforms import TOL, _grid, _meshes, _spec
+
+pytestmark = pytest.mark.gpu
+
+CASES = [(5, 10, 16, 1), (7, 12, 16, 3), (21, 36, 64, 5), (31, 48, 128, 13), (42, 64, 128, 1), (63, 96, 256, 7),
+         (85, 128, 256, 1), (106, 160, 512, 2)]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("case", CASES)
+def test_transforms(jg, orc, case, prec):
+    N, nlat, nlon, nd = case
+    gm, om = _meshes(jg, orc, N, nlat, nlon, nd, prec)
+    for nlev in sorted({nd, 1}):
+        s, s2, g, g2 = _spec(om, nlev, 3, False), _spec(om, nlev, 4, False), _grid(om, nlev, 5), _grid(om, nlev, 6)
+        calls = [("Trans_Spherical_To_Grid", (s,), "g"), ("Trans_Grid_To_Spherical", (g,), "s"),
+                 ("UV_Grid_From_Vor_Div", (s, s2), "gg"), ("Vor_Div_From_Grid_UV", (g, g2), "ss"),
+                 ("Compute_Gradients", (s,), "gg"), ("Trans_Spherical_To_Grid_Adjoint", (g,), "s"),
+                 ("Trans_Grid_To_Spherical_Adjoint", (s,), "g")]
+        for name, ins, outs in calls:
+            a = [gm.grid(nlev) if o == "g" else gm.spectral(nlev) for o in outs]
+            b = [om.grid(nlev) if o == "g" else om.spectral(nlev) for o in outs]
+            getattr(jg, name)(gm, *ins, *a)
+            getattr(orc, name)(om, *ins, *b)
+            for x, y in zip(a, b):
+                assert configs.rel_l2(x, y) < TOL[prec], (name, nlev)
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 5e-5)])
+@pytest.mark.parametrize("N,nlat,nlon", [(21, 36, 64), (42, 64, 128), (63, 96, 256)])
+def test_one_layer_steps(jg, orc, N, nlat, nlon, prec, tol):
+    """Barotropic steps (the fused leapfrog epilogue behind the split rows) against the oracle, at the
+    barotropic step tolerances."""
+    params = dict(configs.PARAMS["barotropic_t42"], dt=1200)
+    gm, om = _meshes(jg, orc, N, nlat, nlon, 1, prec)
+    gmod, omod = jg.Model(gm, params), orc.Model(om, params)
+    configs.init_barotropic_rh4(orc, om, omod)
+    configs.copy_state(omod, gmod, "barotropic")
+    gmod.step(6)
+    omod.step(6)
+    for f in configs.PROGNOSTIC["barotropic"]:
+        assert configs.rel_l2(gmod.get(f), omod.get(f)) < tol, f
