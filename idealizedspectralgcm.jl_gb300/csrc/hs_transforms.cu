@@ -26,16 +26,6 @@ namespace jgcm {
 
 namespace {
 
-// one 16-byte load of four consecutive table weights (16-byte aligned rows)
-__device__ __forceinline__ void ld4w(const float* p, float (&w)[4]) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-}
-__device__ __forceinline__ void ld4w(const double* p, double (&w)[4]) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
-  w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
-}
-
 template <typename T>
 struct HSAnaArgs {
   const V2<T>* F;                       // Fourier buffer [m][j][Cin]
@@ -173,7 +163,7 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
     for (int jh = 0; jh < nh; jh += 4) {
       T w[NP][4];
 #pragma unroll
-      for (int u = 0; u < NP; u++) ld4w(pw[u] + jh, w[u]);
+      for (int u = 0; u < NP; u++) ld4(pw[u] + jh, w[u]);
 #pragma unroll
       for (int v = 0; v < 4; v++) {
         const V x = src[(size_t)(jh + v) * jstride];
@@ -211,9 +201,9 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
     T wP[NP][4], wA[NP][4], wB[NP][4];
 #pragma unroll
     for (int u = 0; u < NP; u++) {
-      ld4w(pw[u] + jh, wP[u]);
-      ld4w(ca[u] + jh, wA[u]);
-      ld4w(cb[u] + jh, wB[u]);
+      ld4(pw[u] + jh, wP[u]);
+      ld4(ca[u] + jh, wA[u]);
+      ld4(cb[u] + jh, wB[u]);
     }
 #pragma unroll
     for (int v = 0; v < 4; v++) {

@@ -270,6 +270,7 @@ struct jgcm_mesh {
   int refs;           // 1 for the caller's handle + 1 per live model built on the mesh
   int device;         // CUDA device the mesh lives on
   int sm_count;       // its SMs (152 on GB300): the size thresholds of the kernel choices
+  int host_direct;    // the device reads and writes ordinary host memory through the host's page tables
   std::string name;
   std::vector<float> twf_host;  // the FP32 twiddle table (cos, sin of 2π t / nlon, t < nlon/2) on the host
 };
@@ -350,6 +351,12 @@ int launch_fft_only(jgcm_mesh* m, const FFTPlan& fp, cudaStream_t st, void* fbuf
 // the inverse FFT of Fourier coefficients already staged in fbuf ((N+1) x nlat x ip.C)
 template <typename T>
 int launch_ifft_only(jgcm_mesh* m, const IFFTPlan& ip, cudaStream_t st, void* fbuf = nullptr, int cap = 0);
+// Host arrays (reference layout, FP64) of the entry points, as the address that the kernels read or write.
+// host_in: `src` itself where the device can read it, else its copy in `stage` (queued on `st`).  host_out:
+// `dst` itself where the device can write it, else `stage`; host_out_done then queues the copy back.
+int host_in(jgcm_mesh* m, const double* src, size_t n, double* stage, cudaStream_t st, const double** use);
+int host_out(jgcm_mesh* m, double* dst, size_t n, double* stage, double** use);
+int host_out_done(double* dst, const double* use, size_t n, cudaStream_t st);
 int spec_host_to_dev(jgcm_mesh* m, const double* d_host_layout, void* d_native, int L, cudaStream_t st);
 int spec_dev_to_host(jgcm_mesh* m, const void* d_native, double* d_host_layout, int L, cudaStream_t st);
 int grid_host_to_dev(jgcm_mesh* m, const double* d_src, void* d_native, size_t n, cudaStream_t st);

@@ -317,6 +317,12 @@ extern "C" int jgcm_mesh_create(int num_fourier, int num_spherical, int nlat, in
   int dev = 0;
   MCHK(cuda(cudaGetDevice(&dev), "cudaGetDevice"));
   MCHK(cuda(cudaDeviceGetAttribute(&m->sm_count, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
+  {
+    int pageable = 0, tables = 0;
+    MCHK(cuda(cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev), "cudaDeviceGetAttribute"));
+    MCHK(cuda(cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev), "cudaDeviceGetAttribute"));
+    m->host_direct = pageable && tables;
+  }
   size_t T3 = (size_t)(m->N + 1) * (m->ns + 1) * nlat;
   MCHK(cuda(cudaMalloc(&m->d_sinth, nlat * 8), "alloc"));
   MCHK(cuda(cudaMalloc(&m->d_wts, nlat * 8), "alloc"));

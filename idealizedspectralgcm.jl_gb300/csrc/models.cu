@@ -2635,12 +2635,11 @@ extern "C" int jgcm_model_get_field(jgcm_model* md, const char* name, double* ho
                                                     md->nd, G, md->P.rdgas, md->P.grav);
     JG_CUDA(cudaGetLastError());
     JG_CUDA(cudaMemcpyAsync(host, (double*)md->g_diag + f.off, n * 8, cudaMemcpyDeviceToHost, st));
-  } else if (f.spec) {
-    JG_TRY(spec_dev_to_host(m, f.ptr, stage, f.L, st));
-    JG_CUDA(cudaMemcpyAsync(host, stage, n * 8, cudaMemcpyDeviceToHost, st));
   } else {
-    JG_TRY(grid_dev_to_host(m, f.ptr, stage, n, st));
-    JG_CUDA(cudaMemcpyAsync(host, stage, n * 8, cudaMemcpyDeviceToHost, st));
+    double* dst;
+    JG_TRY(host_out(m, host, n, stage, &dst));
+    JG_TRY(f.spec ? spec_dev_to_host(m, f.ptr, dst, f.L, st) : grid_dev_to_host(m, f.ptr, dst, n, st));
+    JG_TRY(host_out_done(host, dst, n, st));
   }
   JG_CUDA(cudaStreamSynchronize(st));
   return JGCM_OK;
@@ -2658,11 +2657,12 @@ extern "C" int jgcm_model_set_field(jgcm_model* md, const char* name, const doub
   cudaStream_t st = m->stream;
   double* stage = n <= 4 * m->stage_slot ? m->d_stage : md->q_stage;  // tracer fields may need their own
   JG_CUDA(cudaStreamSynchronize(st));
-  JG_CUDA(cudaMemcpyAsync(stage, host, n * 8, cudaMemcpyHostToDevice, st));
+  const double* src;
+  JG_TRY(host_in(m, host, n, stage, st, &src));
   if (f.spec)
-    JG_TRY(spec_host_to_dev(m, stage, f.ptr, f.L, st));
+    JG_TRY(spec_host_to_dev(m, src, f.ptr, f.L, st));
   else
-    JG_TRY(grid_host_to_dev(m, stage, f.ptr, n, st));
+    JG_TRY(grid_host_to_dev(m, src, f.ptr, n, st));
   if (!strcmp(name, "spe_lnps_n")) md->sw_adv_from_n = 1;
   md->grad_ready = 0;  // the gradients of the current level are recomputed by the next step
   JG_CUDA(cudaStreamSynchronize(st));

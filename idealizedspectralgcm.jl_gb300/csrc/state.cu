@@ -37,29 +37,22 @@ struct PackList {
   int spec[NSTATE];
 };
 
+// One block row (blockIdx.y) per field; its blocks walk a spectrum's transposition tiles (spec_tile_*) or
+// a grid's values, in pairs (every field is an even number of values at an even offset).
 template <typename T>
 __global__ void __launch_bounds__(256) k_state_h2d(PackList p, const double* __restrict__ src, int N, int ns,
                                                    size_t G1) {
   const int f = blockIdx.y, L = p.L[f];
   const double* s = src + p.off[f];
   if (p.spec[f]) {
-    V2<T>* d = (V2<T>*)p.dev[f];
-    const size_t total = (size_t)(N + 1) * (ns + 1) * L;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-      const int k = (int)(t % L);
-      const size_t mn = t / L;
-      const int n = (int)(mn % (ns + 1)), m = (int)(mn / (ns + 1));
-      const size_t h = 2 * ((size_t)m + (size_t)(N + 1) * ((size_t)n + (size_t)(ns + 1) * k));
-      V2<T> v;
-      v.x = (n >= m) ? (T)s[h] : (T)0;
-      v.y = (n >= m) ? (T)s[h + 1] : (T)0;
-      d[t] = v;
+    const int mt = (N + 32) / 32, kt = (L + 31) / 32;
+    for (int t = blockIdx.x; t < mt * kt * (ns + 1); t += gridDim.x) {
+      const int n = t / (mt * kt), r = t - n * mt * kt;
+      spec_tile_h2d<T>((const double2*)s, (V2<T>*)p.dev[f], N, ns, L, r / kt * 32, n, r % kt * 32);
+      __syncthreads();  // the tile's shared memory is free for the next one
     }
   } else {
-    T* d = (T*)p.dev[f];
-    const size_t total = G1 * L;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x)
-      d[t] = (T)s[t];
+    cast_pairs<double, T>(s, (T*)p.dev[f], G1 * L / 2);
   }
 }
 
@@ -68,21 +61,14 @@ __global__ void __launch_bounds__(256) k_state_d2h(PackList p, double* __restric
   const int f = blockIdx.y, L = p.L[f];
   double* d = dst + p.off[f];
   if (p.spec[f]) {
-    const V2<T>* s = (const V2<T>*)p.dev[f];
-    const size_t total = (size_t)(N + 1) * (ns + 1) * L;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-      const int m = (int)(t % (N + 1));
-      const size_t r = t / (N + 1);
-      const int n = (int)(r % (ns + 1)), k = (int)(r / (ns + 1));
-      const V2<T> v = s[((size_t)m * (ns + 1) + n) * L + k];
-      d[2 * t] = (double)v.x;
-      d[2 * t + 1] = (double)v.y;
+    const int mt = (N + 32) / 32, kt = (L + 31) / 32;
+    for (int t = blockIdx.x; t < mt * kt * (ns + 1); t += gridDim.x) {
+      const int n = t / (mt * kt), r = t - n * mt * kt;
+      spec_tile_d2h<T>((const V2<T>*)p.dev[f], (double2*)d, N, ns, L, r / kt * 32, n, r % kt * 32);
+      __syncthreads();  // the tile's shared memory is free for the next one
     }
   } else {
-    const T* s = (const T*)p.dev[f];
-    const size_t total = G1 * L;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x)
-      d[t] = (double)s[t];
+    cast_pairs<T, double>((const T*)p.dev[f], d, G1 * L / 2);
   }
 }
 
@@ -221,11 +207,12 @@ extern "C" int jgcm_model_set_state(jgcm_model* md, const double* packed) {
   PackList p;
   size_t n = 0;
   JG_TRY(pack_list(md, &p, &n));
-  JG_CUDA(cudaMemcpyAsync(md->state_stage, packed, n * 8, cudaMemcpyHostToDevice, st));
+  const double* src;
+  JG_TRY(host_in(m, packed, n, md->state_stage, st, &src));
   const dim3 g(64, NSTATE);
   const size_t G1 = grid_elems(m, 1);
-  if (is_fp64(m)) k_state_h2d<double><<<g, 256, 0, st>>>(p, md->state_stage, m->N, m->ns, G1);
-  else k_state_h2d<float><<<g, 256, 0, st>>>(p, md->state_stage, m->N, m->ns, G1);
+  if (is_fp64(m)) k_state_h2d<double><<<g, 256, 0, st>>>(p, src, m->N, m->ns, G1);
+  else k_state_h2d<float><<<g, 256, 0, st>>>(p, src, m->N, m->ns, G1);
   JG_CUDA(cudaGetLastError());
   md->grad_ready = 0;  // the gradients of the new c level are recomputed by the next step
   JG_CUDA(cudaStreamSynchronize(st));
@@ -240,12 +227,14 @@ extern "C" int jgcm_model_get_state(jgcm_model* md, double* packed) {
   PackList p;
   size_t n = 0;
   JG_TRY(pack_list(md, &p, &n));
+  double* dst;
+  JG_TRY(host_out(m, packed, n, md->state_stage, &dst));
   const dim3 g(64, NSTATE);
   const size_t G1 = grid_elems(m, 1);
-  if (is_fp64(m)) k_state_d2h<double><<<g, 256, 0, st>>>(p, md->state_stage, m->N, m->ns, G1);
-  else k_state_d2h<float><<<g, 256, 0, st>>>(p, md->state_stage, m->N, m->ns, G1);
+  if (is_fp64(m)) k_state_d2h<double><<<g, 256, 0, st>>>(p, dst, m->N, m->ns, G1);
+  else k_state_d2h<float><<<g, 256, 0, st>>>(p, dst, m->N, m->ns, G1);
   JG_CUDA(cudaGetLastError());
-  JG_CUDA(cudaMemcpyAsync(packed, md->state_stage, n * 8, cudaMemcpyDeviceToHost, st));
+  JG_TRY(host_out_done(packed, dst, n, st));
   JG_CUDA(cudaStreamSynchronize(st));
   return JGCM_OK;
 }

@@ -19,6 +19,85 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// four consecutive values in 16-byte loads and stores (the address is 16-byte aligned)
+__device__ __forceinline__ void ld4(const float* p, float (&w)[4]) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+}
+__device__ __forceinline__ void ld4(const double* p, double (&w)[4]) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
+}
+
+// np pairs of values converted along blockIdx.x, CAST_U pairs in flight per thread: every load and store
+// instruction of a warp is one run of consecutive pairs (a store to host memory that leaves gaps in its
+// sectors, four values per thread, ran at half the rate)
+constexpr int CAST_U = 4;
+template <typename A, typename B>
+__device__ __forceinline__ void cast_pairs(const A* __restrict__ src, B* __restrict__ dst, size_t np) {
+  const V2<A>* __restrict__ s = reinterpret_cast<const V2<A>*>(src);
+  V2<B>* __restrict__ d = reinterpret_cast<V2<B>*>(dst);
+  for (size_t t = (size_t)blockIdx.x * blockDim.x * CAST_U + threadIdx.x; t < np;
+       t += (size_t)gridDim.x * blockDim.x * CAST_U) {
+    V2<A> x[CAST_U];
+#pragma unroll
+    for (int u = 0; u < CAST_U; u++)
+      if (t + (size_t)u * blockDim.x < np) x[u] = s[t + (size_t)u * blockDim.x];
+#pragma unroll
+    for (int u = 0; u < CAST_U; u++)
+      if (t + (size_t)u * blockDim.x < np) {
+        V2<B> y;
+        y.x = (B)x[u].x;
+        y.y = (B)x[u].y;
+        d[t + (size_t)u * blockDim.x] = y;
+      }
+  }
+}
+
+// Spectra between the host layout [k][n][m] (FP64 pairs, m fastest) and the device layout [m][n][k]: one
+// total wavenumber's 32 x 32 tile of the (k, m) matrix transposed through shared memory by 256 threads,
+// both sides in runs of consecutive pairs.  Entries n < m are not read and become zero.
+template <typename T>
+__device__ __forceinline__ void spec_tile_h2d(const double2* __restrict__ src, V2<T>* __restrict__ dst, int N, int ns,
+                                              int L, int m0, int n, int k0) {
+  __shared__ V2<T> tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int q = ty; q < 32; q += 8) {
+    const int k = k0 + q, m = m0 + tx;
+    V2<T> v;
+    v.x = v.y = 0;
+    if (k < L && m <= N && m <= n) {
+      const double2 x = src[((size_t)k * (ns + 1) + n) * (N + 1) + m];
+      v.x = (T)x.x;
+      v.y = (T)x.y;
+    }
+    tile[q][tx] = v;
+  }
+  __syncthreads();
+  for (int q = ty; q < 32; q += 8) {
+    const int m = m0 + q, k = k0 + tx;
+    if (k < L && m <= N) dst[((size_t)m * (ns + 1) + n) * L + k] = tile[tx][q];
+  }
+}
+template <typename T>
+__device__ __forceinline__ void spec_tile_d2h(const V2<T>* __restrict__ src, double2* __restrict__ dst, int N, int ns,
+                                              int L, int m0, int n, int k0) {
+  __shared__ V2<T> tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int q = ty; q < 32; q += 8) {
+    const int m = m0 + q, k = k0 + tx;
+    if (k < L && m <= N) tile[tx][q] = src[((size_t)m * (ns + 1) + n) * L + k];
+  }
+  __syncthreads();
+  for (int q = ty; q < 32; q += 8) {
+    const int k = k0 + q, m = m0 + tx;
+    if (k < L && m <= N) {
+      const V2<T> v = tile[q][tx];
+      dst[((size_t)k * (ns + 1) + n) * (N + 1) + m] = make_double2((double)v.x, (double)v.y);
+    }
+  }
+}
+
 template <typename G>
 __device__ __forceinline__ const G& group_of(const G* g, int ng, int c, int* k) {
   int i = 0;

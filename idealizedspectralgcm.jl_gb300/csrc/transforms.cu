@@ -22,6 +22,8 @@
 #include <mutex>
 #include <type_traits>
 
+#include <unistd.h>
+
 #include "jgcm_internal.cuh"
 #include "transform_ops.cuh"
 
@@ -954,17 +956,6 @@ static inline size_t row_fft_smem(const jgcm_mesh* m) { return (size_t)RF_WARPS 
 // Shared memory holds, for the input slots in use, the hemisphere-symmetric and -antisymmetric
 // combinations g(mu_j) +/- g(-mu_j) of the tile's columns.
 constexpr int G2S_BLOCKS_PER_SM = 2;  // the row split's aim (launch_g2s)
-// four consecutive table weights in one 16-byte load (the address is 16-byte aligned: nh is a
-// multiple of 4 and the tables start aligned)
-__device__ __forceinline__ void ld4(const float* p, float (&w)[4]) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
-}
-__device__ __forceinline__ void ld4(const double* p, double (&w)[4]) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
-  w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
-}
-
 // QL lanes per output (4: a quad splits the latitude sum and combines it with two shuffles, for
 // launches too small to fill the device; 1: a lane sums its output alone, half the instructions per
 // output, for launches with many outputs).
@@ -1477,36 +1468,25 @@ template int launch_fft_only<double>(jgcm_mesh*, const FFTPlan&, cudaStream_t, v
 
 // ------------------------------------------------------------------------------------------
 // Layout / precision conversion between the reference host layout (FP64) and device layout.
+// Spectra: host [k][n][m] <-> device [m][n][k], a transposition of each total wavenumber's (k, m) matrix
+// through shared memory (spec_tile_*, transform_ops.cuh).  grid (m tiles, ns + 1, level tiles).
 template <typename T>
-__global__ void k_spec_h2d(const double* __restrict__ src, V2<T>* __restrict__ dst, int N, int ns, int L) {
-  size_t total = (size_t)(N + 1) * (ns + 1) * L;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    int k = (int)(t % L);
-    size_t mn = t / L;
-    int n = (int)(mn % (ns + 1)), m = (int)(mn / (ns + 1));
-    size_t h = 2 * ((size_t)m + (size_t)(N + 1) * ((size_t)n + (size_t)(ns + 1) * k));
-    V2<T> v;
-    v.x = (n >= m) ? (T)src[h] : (T)0;
-    v.y = (n >= m) ? (T)src[h + 1] : (T)0;
-    dst[t] = v;
-  }
+__global__ void __launch_bounds__(256) k_spec_h2d(const double2* __restrict__ src, V2<T>* __restrict__ dst, int N,
+                                                  int ns, int L) {
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  spec_tile_h2d<T>(src, dst, N, ns, L, blockIdx.x * 32, blockIdx.y, blockIdx.z * 32);
 }
 template <typename T>
-__global__ void k_spec_d2h(const V2<T>* __restrict__ src, double* __restrict__ dst, int N, int ns, int L) {
-  size_t total = (size_t)(N + 1) * (ns + 1) * L;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    int m = (int)(t % (N + 1));
-    size_t r = t / (N + 1);
-    int n = (int)(r % (ns + 1)), k = (int)(r / (ns + 1));
-    V2<T> v = src[((size_t)m * (ns + 1) + n) * L + k];
-    dst[2 * t] = (double)v.x;
-    dst[2 * t + 1] = (double)v.y;
-  }
+__global__ void __launch_bounds__(256) k_spec_d2h(const V2<T>* __restrict__ src, double2* __restrict__ dst, int N,
+                                                  int ns, int L) {
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  spec_tile_d2h<T>(src, dst, N, ns, L, blockIdx.x * 32, blockIdx.y, blockIdx.z * 32);
 }
+// n values, an even number, both sides 16-byte aligned
 template <typename A, typename B>
-__global__ void k_cast(const A* __restrict__ src, B* __restrict__ dst, size_t n) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-    dst[t] = (B)src[t];
+__global__ void __launch_bounds__(256) k_cast(const A* __restrict__ src, B* __restrict__ dst, size_t n) {
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  cast_pairs<A, B>(src, dst, n / 2);
 }
 // Fourier buffer [m][j][c] -> host [c][j][m] (modes 0..N)
 template <typename T>
@@ -1528,39 +1508,83 @@ static inline int nblk(size_t n) {
 }
 
 int spec_host_to_dev(jgcm_mesh* m, const double* src, void* dst, int L, cudaStream_t st) {
-  size_t n = spec_elems(m, L);
-  if (is_fp64(m))
-    k_spec_h2d<double><<<nblk(n), 256, 0, st>>>(src, (double2*)dst, m->N, m->ns, L);
-  else
-    k_spec_h2d<float><<<nblk(n), 256, 0, st>>>(src, (float2*)dst, m->N, m->ns, L);
-  JG_CUDA(cudaGetLastError());
+  const dim3 g((m->N + 32) / 32, m->ns + 1, (L + 31) / 32);
+  const double2* s2 = (const double2*)src;
+  JG_CUDA(is_fp64(m) ? launch_pdl(k_spec_h2d<double>, g, 256, 0, st, s2, (double2*)dst, m->N, m->ns, L)
+                     : launch_pdl(k_spec_h2d<float>, g, 256, 0, st, s2, (float2*)dst, m->N, m->ns, L));
   return JGCM_OK;
 }
 int spec_dev_to_host(jgcm_mesh* m, const void* src, double* dst, int L, cudaStream_t st) {
-  size_t n = spec_elems(m, L);
-  if (is_fp64(m))
-    k_spec_d2h<double><<<nblk(n), 256, 0, st>>>((const double2*)src, dst, m->N, m->ns, L);
-  else
-    k_spec_d2h<float><<<nblk(n), 256, 0, st>>>((const float2*)src, dst, m->N, m->ns, L);
-  JG_CUDA(cudaGetLastError());
+  const dim3 g((m->N + 32) / 32, m->ns + 1, (L + 31) / 32);
+  double2* d2 = (double2*)dst;
+  JG_CUDA(is_fp64(m) ? launch_pdl(k_spec_d2h<double>, g, 256, 0, st, (const double2*)src, d2, m->N, m->ns, L)
+                     : launch_pdl(k_spec_d2h<float>, g, 256, 0, st, (const float2*)src, d2, m->N, m->ns, L));
   return JGCM_OK;
 }
 int grid_host_to_dev(jgcm_mesh* m, const double* src, void* dst, size_t n, cudaStream_t st) {
-  if (is_fp64(m))
-    JG_CUDA(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToDevice, st));
-  else
-    k_cast<double, float><<<nblk(n), 256, 0, st>>>(src, (float*)dst, n);
-  JG_CUDA(cudaGetLastError());
+  JG_CUDA(is_fp64(m) ? launch_pdl(k_cast<double, double>, nblk(n / 8), 256, 0, st, src, (double*)dst, n)
+                     : launch_pdl(k_cast<double, float>, nblk(n / 8), 256, 0, st, src, (float*)dst, n));
   return JGCM_OK;
 }
 int grid_dev_to_host(jgcm_mesh* m, const void* src, double* dst, size_t n, cudaStream_t st) {
-  if (is_fp64(m))
-    JG_CUDA(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToDevice, st));
-  else
-    k_cast<float, double><<<nblk(n), 256, 0, st>>>((const float*)src, dst, n);
-  JG_CUDA(cudaGetLastError());
+  JG_CUDA(is_fp64(m) ? launch_pdl(k_cast<double, double>, nblk(n / 8), 256, 0, st, (const double*)src, dst, n)
+                     : launch_pdl(k_cast<float, double>, nblk(n / 8), 256, 0, st, (const float*)src, dst, n));
   return JGCM_OK;
 }
+
+// ------------------------------------------------------------------------------------------
+// Host arrays.  On a device that shares the host's page tables (Grace: NVLink-C2C, coherent) the
+// conversion kernels read and write the caller's arrays in place: a pageable cudaMemcpyAsync goes
+// through the driver a call at a time, and the data crosses the device's memory once more (winds of T63L13
+// from host spectra, FP32, 1.7 MB in and 5.1 MB out: 121 -> 70 us; T85L20 FP64 269 -> 159 us; one level of
+// T21 31 -> 22 us).  Every page of the array is touched by this thread first: pages that were never written are mapped before the device
+// meets them, and an address that is not the process's to read or write faults here, in the calling
+// thread, as it did in the copy, and never on the device.  Arrays that are not 16-byte aligned (the
+// kernels move pairs), device pointers and other devices keep the copy.
+static bool host_direct(const jgcm_mesh* m, const void* p) {
+  if (!m->host_direct || ((uintptr_t)p & 15)) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeManaged ||
+         (at.type == cudaMemoryTypeHost && at.devicePointer == p);
+}
+static size_t page_bytes() {
+  static const size_t b = (size_t)sysconf(_SC_PAGESIZE);
+  return b;
+}
+int host_in(jgcm_mesh* m, const double* src, size_t n, double* stage, cudaStream_t st, const double** use) {
+  JG_ARG(src != nullptr, "input array is NULL");
+  if (host_direct(m, src)) {
+    const volatile char* p = (const volatile char*)src;
+    for (size_t o = 0; o < n * 8; o += page_bytes()) (void)p[o];
+    (void)p[n * 8 - 1];
+    *use = src;
+    return JGCM_OK;
+  }
+  JG_CUDA(cudaMemcpyAsync(stage, src, n * 8, cudaMemcpyHostToDevice, st));
+  *use = stage;
+  return JGCM_OK;
+}
+int host_out(jgcm_mesh* m, double* dst, size_t n, double* stage, double** use) {
+  JG_ARG(dst != nullptr, "output array is NULL");
+  if (host_direct(m, dst)) {
+    volatile char* p = (volatile char*)dst;
+    for (size_t o = 0; o < n * 8; o += page_bytes()) p[o] = p[o];
+    p[n * 8 - 1] = p[n * 8 - 1];
+    *use = dst;
+  } else {
+    *use = stage;
+  }
+  return JGCM_OK;
+}
+int host_out_done(double* dst, const double* use, size_t n, cudaStream_t st) {
+  if (use != dst) JG_CUDA(cudaMemcpyAsync(dst, use, n * 8, cudaMemcpyDeviceToHost, st));
+  return JGCM_OK;
+}
+
 int fourier_dev_to_host(jgcm_mesh* m, int L, double* dst, cudaStream_t st) {
   size_t n = (size_t)(m->N + 1) * m->nlat * L;
   if (is_fp64(m))

@@ -50,3 +50,44 @@ def test_one_layer_steps(jg, orc, N, nlat, nlon, prec, tol):
     omod.step(6)
     for f in configs.PROGNOSTIC["barotropic"]:
         assert configs.rel_l2(gmod.get(f), omod.get(f)) < tol, f
+
+
+def _shifted(a):
+    """a copy of `a` whose data start 8 bytes past a 16-byte boundary (FP64 arrays need no more)"""
+    raw = np.zeros(a.nbytes // 8 + 3)
+    off = 1 if raw.ctypes.data % 16 == 0 else 2
+    b = raw[off:off + a.nbytes // 8].view(a.dtype).reshape(a.shape, order="F")
+    b[...] = a
+    assert b.ctypes.data % 16 == 8 and b.flags.f_contiguous
+    return b
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+@pytest.mark.parametrize("case", [(7, 12, 16, 3), (42, 64, 128, 1), (42, 64, 128, 20)])
+def test_host_arrays_off_the_pair_alignment(jg, orc, case, prec):
+    """Arrays that the kernels do not read or write in place (8 bytes off a 16-byte boundary) give the
+    results of those that they do, bit for bit; so does a fresh output whose pages nobody has touched."""
+    N, nlat, nlon, nd = case
+    gm, om = _meshes(jg, orc, N, nlat, nlon, nd, prec)
+    s, g = _spec(om, nd, 3, False), _grid(om, nd, 5)
+    for name, ins, outs in (("UV_Grid_From_Vor_Div", (s, 2 * s), (gm.grid(nd), gm.grid(nd))),
+                            ("Vor_Div_From_Grid_UV", (g, 2 * g), (gm.spectral(nd), gm.spectral(nd))),
+                            ("Add_Horizontal_Advection", (s, g, 2 * g), (g.copy(order="F"),))):
+        off = [_shifted(x) for x in outs]
+        getattr(jg, name)(gm, *[np.asfortranarray(x) for x in ins], *outs)
+        getattr(jg, name)(gm, *[_shifted(x) for x in ins], *off)
+        for a, b in zip(outs, off):
+            assert np.array_equal(a, b), name
+
+
+def test_packed_state_off_the_pair_alignment(jg):
+    params = configs.PARAMS["hs_t21l10"]
+    mesh = configs.make_mesh(jg, "hs_t21l10", precision="fp32")
+    md = jg.Model(mesh, params)
+    configs.init_held_suarez(jg, mesh, md)
+    a, b = md.get_state(), _shifted(np.zeros(md.state_size()))
+    md.get_state(out=b)
+    assert np.array_equal(a, b)
+    md.set_state(2.0 * a)
+    md.set_state(b)
+    assert np.array_equal(md.get_state(), a)
