@@ -2949,12 +2949,35 @@ extern "C" int jgcm_spectral_initialize_fields(jgcm_model* md, const double* gri
 // ------------------------------------------------------------------------------------------
 // Member copies between models of one mesh and one parameter set (ensembles, member-major).
 namespace {
-// spectral [m][n][ne*L] member slices: dst member dm <- src member sm, L innermost levels each
-template <typename V>
-__global__ void k_spec_member_copy(V* dst, int dne, int dm, const V* src, int sne, int sm, size_t S, int L) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < S * L; q += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = q / L, k = q - r * L;
-    dst[(r * dne + dm) * L + k] = src[(r * sne + sm) * L + k];
+// The fields of a member copy, moved by one launch (blockIdx.y: the field).  As one call per field (26 to
+// 36 copies and launches of a few us each) a member's copy was bound by the host: 124 us for T21L20 FP32,
+// 12.5 us as one launch.  A grid field's member slice is one run (16-byte words: nlon is a power
+// of two from 8 on); a spectral field [m][n][ne L] has a run of L values per mode.
+struct MemberCopy {
+  struct Field {
+    void* dst;
+    const void* src;
+    int L, spec;
+  } f[36];
+  int n, dne, dm, sne, sm;
+};
+template <typename T>
+__global__ void __launch_bounds__(256) k_member_copy(MemberCopy c, size_t S, size_t G1) {
+  const MemberCopy::Field& f = c.f[blockIdx.y];
+  const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  if (f.spec) {
+    const unsigned L = f.L, total = (unsigned)(S * L);
+    const V2<T>* src = (const V2<T>*)f.src;
+    V2<T>* dst = (V2<T>*)f.dst;
+    for (unsigned q = (unsigned)t0; q < total; q += (unsigned)step) {
+      const unsigned r = q / L, k = q - r * L;
+      dst[((size_t)r * c.dne + c.dm) * L + k] = src[((size_t)r * c.sne + c.sm) * L + k];
+    }
+  } else {
+    const size_t words = f.L * G1 * sizeof(T) / 16;
+    const uint4* src = (const uint4*)f.src + c.sm * words;
+    uint4* dst = (uint4*)f.dst + c.dm * words;
+    for (size_t q = t0; q < words; q += step) dst[q] = src[q];
   }
 }
 }  // namespace
@@ -2977,44 +3000,40 @@ extern "C" int jgcm_model_copy_member(jgcm_model* dst, int dst_member, jgcm_mode
   jgcm_mesh* m = dst->mesh;
   cudaStream_t st = m->stream;
   const int nd = dst->nd;
-  const size_t ts = tsize(m), G1 = grid_elems(m, 1), S = (size_t)(m->N + 1) * (m->ns + 1);
-  auto grid = [&](void* d, const void* s_, int L) -> int {  // member slices are contiguous
-    JG_CUDA(cudaMemcpyAsync((char*)d + (size_t)dst_member * L * G1 * ts, (const char*)s_ + (size_t)src_member * L * G1 * ts,
-                            (size_t)L * G1 * ts, cudaMemcpyDeviceToDevice, st));
-    return JGCM_OK;
-  };
-  auto spec = [&](void* d, const void* s_, int L) -> int {
-    int nb = (int)std::min<size_t>((S * L + 255) / 256, 1024);
-    if (is_fp64(m))
-      k_spec_member_copy<double2><<<nb, 256, 0, st>>>((double2*)d, dst->ne, dst_member, (const double2*)s_, src->ne,
-                                                      src_member, S, L);
-    else
-      k_spec_member_copy<float2><<<nb, 256, 0, st>>>((float2*)d, dst->ne, dst_member, (const float2*)s_, src->ne,
-                                                     src_member, S, L);
-    JG_CUDA(cudaGetLastError());
-    return JGCM_OK;
-  };
+  const size_t G1 = grid_elems(m, 1), S = (size_t)(m->N + 1) * (m->ns + 1);
+  MemberCopy c;
+  c.n = 0;
+  c.dne = dst->ne;
+  c.dm = dst_member;
+  c.sne = src->ne;
+  c.sm = src_member;
+  auto add = [&](void* d, const void* s_, int L, int spec) { c.f[c.n++] = {d, s_, L, spec}; };
   for (int w = 0; w < 3; w++) {  // logical levels p, c, n
     const int ld = lvl(dst, w), ls = lvl(src, w);
-    JG_TRY(spec(dst->spe_vor[ld], src->spe_vor[ls], nd));
-    JG_TRY(spec(dst->spe_div[ld], src->spe_div[ls], nd));
-    JG_TRY(spec(dst->spe_t[ld], src->spe_t[ls], nd));
-    JG_TRY(spec(dst->spe_lnps[ld], src->spe_lnps[ls], 1));
-    JG_TRY(grid(dst->grid_u[ld], src->grid_u[ls], nd));
-    JG_TRY(grid(dst->grid_v[ld], src->grid_v[ls], nd));
-    JG_TRY(grid(dst->grid_t[ld], src->grid_t[ls], nd));
-    JG_TRY(grid(dst->grid_ps[ld], src->grid_ps[ls], 1));
+    add(dst->spe_vor[ld], src->spe_vor[ls], nd, 1);
+    add(dst->spe_div[ld], src->spe_div[ls], nd, 1);
+    add(dst->spe_t[ld], src->spe_t[ls], nd, 1);
+    add(dst->spe_lnps[ld], src->spe_lnps[ls], 1, 1);
+    add(dst->grid_u[ld], src->grid_u[ls], nd, 0);
+    add(dst->grid_v[ld], src->grid_v[ls], nd, 0);
+    add(dst->grid_t[ld], src->grid_t[ls], nd, 0);
+    add(dst->grid_ps[ld], src->grid_ps[ls], 1, 0);
     if (dst->nq) {
-      JG_TRY(spec(dst->spe_q[ld], src->spe_q[ls], nd * dst->nq));
-      JG_TRY(grid(dst->grid_q[ld], src->grid_q[ls], nd * dst->nq));
+      add(dst->spe_q[ld], src->spe_q[ls], nd * dst->nq, 1);
+      add(dst->grid_q[ld], src->grid_q[ls], nd * dst->nq, 0);
     }
   }
-  JG_TRY(grid(dst->grid_vor, src->grid_vor, nd));
-  JG_TRY(grid(dst->grid_div, src->grid_div, nd));
-  JG_TRY(grid(dst->grid_t_eq, src->grid_t_eq, nd));
-  JG_TRY(grid(dst->grid_lnps, src->grid_lnps, 1));
-  JG_TRY(grid(dst->grid_geopots, src->grid_geopots, 1));
-  JG_TRY(grid(dst->grid_h_eq, src->grid_h_eq, 1));
+  add(dst->grid_vor, src->grid_vor, nd, 0);
+  add(dst->grid_div, src->grid_div, nd, 0);
+  add(dst->grid_t_eq, src->grid_t_eq, nd, 0);
+  add(dst->grid_lnps, src->grid_lnps, 1, 0);
+  add(dst->grid_geopots, src->grid_geopots, 1, 0);
+  add(dst->grid_h_eq, src->grid_h_eq, 1, 0);
+  const size_t most = std::max(G1 * tsize(m) / 16, S) * nd;  // work items of the largest field but the tracers
+  const dim3 g((unsigned)std::min<size_t>((most + 255) / 256, 128), c.n);
+  if (is_fp64(m)) k_member_copy<double><<<g, 256, 0, st>>>(c, S, G1);
+  else k_member_copy<float><<<g, 256, 0, st>>>(c, S, G1);
+  JG_CUDA(cudaGetLastError());
   dst->grad_ready = 0;
   if (dst->ne == 1) {  // a one-member model takes the source's time-step state
     dst->init_step = src->init_step;
