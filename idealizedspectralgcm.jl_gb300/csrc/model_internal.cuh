@@ -66,6 +66,7 @@ struct jgcm_model {
   jgcm::VertCoef* d_vc;  // device copy read by the column and semi-implicit kernels
   double* div_mat;  // host nd*nd column-major
   double* d_W;      // device [2][N+1][nd][nd] (transposed: [c][r])
+  float2* d_W2;     // FP32 path: the same as pairs hi + lo
   int2* d_pairs;    // (m, n) pairs with n >= m
   int npairs;
   double *d_partials, *d_scalars;

@@ -617,6 +617,7 @@ struct ImplArgs {
   const T *damping, *dfac;  // [m][n]: damping, 1/(1 + Δt' damping) for this step
   const double* eig64;      // [m][n]: -n(n+1)/a², FP64
   const double* W;                // [N+1][c][r]
+  const float2* W2;               // FP32 path: W as pairs hi + lo
   const int2* pairs;
   int npairs, nd, L, ne, ns, N, init_step, dt;  // spectral innermost index e*nd + k of L = ne*nd
   double xi, ps_ref, kappa, rdgas, robert;
@@ -713,7 +714,13 @@ __device__ __forceinline__ void lf(int init, int Dt, R rob, R d, R f, R& dq, R q
   }
 }
 
-// R is the precision of the vertical algebra (FP64 on the FP64 path; selectable on the FP32 path).
+// R is the precision of the vertical algebra, the state's.  The wave-matrix product is formed to FP64
+// accuracy in both: FP64 products and sums on the FP64 path; on the FP32 path, whose right-hand side and
+// result are FP32, W_n as pairs hi + lo and the row sums as pairs (ds_add_prod: error-free products and
+// additions, ~2^-46 of the sum of magnitudes before the result is rounded to FP32).  An FP64 instruction
+// holds a sub-partition for ~64 cycles, the pair's ten FP32 ones for ten: with FP64 products this kernel
+// was bound by them from a few members on (128 x T21L20 95 -> 64 us, 32 x T42L20 90 -> 60 us, one T42L20 member 11.4 -> 9.8 us, event included; the
+// results against 64 bits as before: one member bit for bit, the ensembles 2.4e-6 and 2.5e-6 in the worst field).
 // DENSE: the FP64 wave-matrix products of the block's modes are spread over all its threads, one
 // (mode, component, row) output each, instead of one mode per warp, whose 32 - nd idle lanes the
 // FP64 pipe executes all the same (for launches with many modes: member ensembles).
@@ -796,6 +803,26 @@ __global__ void __launch_bounds__(256) k_hs_implicit(ImplArgs<T> a, const VertCo
     if (n <= a.N) {
       ddiv.x = act ? (R)s_o[w][0][k] : (R)0;
       ddiv.y = act ? (R)s_o[w][1][k] : (R)0;
+    }
+  } else if constexpr (std::is_same<R, float>::value) {
+    if (n <= a.N) {
+      const float2* W = a.W2 + (size_t)n * nd * nd;
+      float xh = 0, xl = 0, yh = 0, yl = 0;
+      for (int c0 = 0; c0 < nd; c0 += 8) {  // 8 loads in flight; nd is warp-uniform
+        float2 wv[8];
+#pragma unroll
+        for (int cc = 0; cc < 8; cc++) wv[cc] = (act && c0 + cc < nd) ? W[(size_t)(c0 + cc) * nd + k] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int cc = 0; cc < 8; cc++) {
+          if (c0 + cc < nd) {
+            const float bx = __shfl_sync(FULL, ddiv.x, c0 + cc), by = __shfl_sync(FULL, ddiv.y, c0 + cc);
+            ds_add_prod(xh, xl, bx, wv[cc].x, wv[cc].y);
+            ds_add_prod(yh, yl, by, wv[cc].x, wv[cc].y);
+          }
+        }
+      }
+      ddiv.x = act ? xh + xl : 0.f;
+      ddiv.y = act ? yh + yl : 0.f;
     }
   } else if (n <= a.N) {
     const double* W = a.W + (size_t)n * nd * nd;
@@ -1453,7 +1480,7 @@ void model_free(jgcm_model* md) {
   void* ps[] = {md->grid_vor, md->grid_div, md->grid_lnps, md->grid_t_eq, md->grid_geopots, md->grid_h_eq,
                 md->spe_zero, md->spe_dvor, md->spe_ddiv, md->spe_dlnps, md->spe_dt, md->g_dlps, md->g_dtps,
                 md->g_dlT, md->g_dtT, md->g_ducos, md->g_dvcos, md->g_dt, md->g_energy, md->g_dlnps, md->g_diag,
-                md->g_tdev, md->coriolis, md->damping, md->dfac[0], md->dfac[1], md->d_W, md->d_pairs, md->d_partials,
+                md->g_tdev, md->coriolis, md->damping, md->dfac[0], md->dfac[1], md->d_W, md->d_W2, md->d_pairs, md->d_partials,
                 md->d_scalars, md->d_counter, md->d_vc, md->fbuf, md->diag};
   for (auto p : ps)
     if (p) cudaFree(p);
@@ -1461,6 +1488,13 @@ void model_free(jgcm_model* md) {
   if (md->ev0) cudaEventDestroy(md->ev0);
   if (md->ev1) cudaEventDestroy(md->ev1);
   delete md;
+}
+
+__global__ void k_split_pairs(const double* in, float2* out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float hi = (float)in[i];
+  out[i] = make_float2(hi, (float)(in[i] - (double)hi));
 }
 
 int build_wave(jgcm_model* md) {
@@ -1480,6 +1514,11 @@ int build_wave(jgcm_model* md) {
   for (int s = 0; s < 2; s++) {
     k_wave_matrices<<<N + 1, 128, 2 * nd * nd * 8, m->stream>>>(d_div, d_eig0, xis[s], nd, N,
                                                                  md->d_W + (size_t)s * (N + 1) * nd * nd, d_status);
+    JG_CUDA(cudaGetLastError());
+  }
+  if (md->d_W2) {
+    const int n = 2 * (N + 1) * nd * nd;
+    k_split_pairs<<<(n + 255) / 256, 256, 0, m->stream>>>(md->d_W, md->d_W2, n);
     JG_CUDA(cudaGetLastError());
   }
   int st = 0;
@@ -1538,6 +1577,7 @@ int model_alloc(jgcm_model* md) {
   JG_TRY(alloc(&md->coriolis, (size_t)m->nlat * ts));
   JG_TRY(alloc(&md->damping, (size_t)(N + 1) * (ns + 1) * ts));
   JG_TRY(alloc((void**)&md->d_W, 2 * (size_t)(N + 1) * nd * nd * 8));
+  if (!is_fp64(m)) JG_TRY(alloc((void**)&md->d_W2, 2 * (size_t)(N + 1) * nd * nd * sizeof(float2)));
   std::vector<int2> pairs;
   for (int mm = 0; mm <= N; mm++)
     for (int n = mm; n <= ns; n++) pairs.push_back(make_int2(mm, n));
@@ -1973,6 +2013,7 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
   ia.damping = (const T*)md->damping;
   ia.dfac = (const T*)md->dfac[md->init_step ? 0 : 1];
   ia.W = md->d_W + (md->init_step ? 0 : (size_t)(m->N + 1) * nd * nd);
+  ia.W2 = md->d_W2 ? md->d_W2 + (md->init_step ? 0 : (size_t)(m->N + 1) * nd * nd) : nullptr;
   ia.pairs = md->d_pairs;
   ia.npairs = md->npairs;
   ia.nd = nd;
@@ -1999,8 +2040,10 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
   // vertical algebra in the state precision (FP64 algebra on the FP32 path measured no more
   // accurate: its error is set by FP32 storage); the wave-matrix solve is FP64 in both
   // 4 modes per block: (N+1)(N+2)/2 + N+1 modes at T42 make 248 blocks, every SM's FP64 units busy;
-  // member ensembles (from 4 members) spread the FP64 products densely over each block
-  if (E >= 4)
+  // FP64 member ensembles (from 4 members) spread the FP64 products densely over each block
+  if constexpr (std::is_same<T, float>::value)
+    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, md->d_vc));
+  else if (E >= 4)
     JG_CUDA(launch_pdl(k_hs_implicit<T, T, true>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, md->d_vc));
   else
     JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, md->d_vc));
@@ -3647,6 +3690,7 @@ ImplArgs<T> si_args(jgcm_model* md, void* const* in, void* const* out) {
   ia.damping = (const T*)md->damping;
   ia.dfac = (const T*)md->dfac[md->init_step ? 0 : 1];
   ia.W = md->d_W + (md->init_step ? 0 : (size_t)(m->N + 1) * md->nd * md->nd);
+  ia.W2 = md->d_W2 ? md->d_W2 + (md->init_step ? 0 : (size_t)(m->N + 1) * md->nd * md->nd) : nullptr;
   ia.pairs = md->d_pairs;
   ia.npairs = md->npairs;
   ia.nd = md->nd;
