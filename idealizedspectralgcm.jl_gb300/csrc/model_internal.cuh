@@ -25,6 +25,20 @@ struct VertCoef {  // Vert_Coordinate (even_sigma) and the semi-implicit referen
   // path forms the column sums of T_k Δa_k, T_k Δb_k to FP64 accuracy from them
   float dak_hi[JGCM_MAX_ND], dak_lo[JGCM_MAX_ND], dbk_hi[JGCM_MAX_ND], dbk_lo[JGCM_MAX_ND];
 };
+// The same in the state precision T, rounded once on the host: a conversion in a kernel, like every FP64
+// instruction, holds a sub-partition for ~64 cycles, and every block of the column, fixer and
+// semi-implicit kernels staged its coefficients through up to 14 of them on one warp.
+template <typename T>
+struct VertT {
+  T ak[JGCM_MAX_ND + 1], bk[JGCM_MAX_ND + 1], dak[JGCM_MAX_ND], dbk[JGCM_MAX_ND];
+  // column kernel, sigma coordinates: ln p_k - ln ps, p_k / ps, exp(kappa (ln p_k - ln ps)), the log
+  // differences, 1 / Δb_k, Δb_k / (Δb_k + Δb_{k+1}), (b_{k-1/2} dlp_m + b_{k+1/2} dlp_p) / Δb_k
+  T cf[JGCM_MAX_ND], sf[JGCM_MAX_ND], ek[JGCM_MAX_ND], dlp_p[JGCM_MAX_ND], dlp[JGCM_MAX_ND], rdb[JGCM_MAX_ND],
+      w1[JGCM_MAX_ND], x1[JGCM_MAX_ND];
+  // semi-implicit kernel: the reference column
+  T dpr[JGCM_MAX_ND], rdpr[JGCM_MAX_ND], dlnp[JGCM_MAX_ND], dlnpp[JGCM_MAX_ND], tref[JGCM_MAX_ND], tdh[JGCM_MAX_ND],
+      hk[JGCM_MAX_ND];
+};
 }  // namespace jgcm
 
 struct jgcm_model {
@@ -63,7 +77,8 @@ struct jgcm_model {
   void* dfac[2];             // [m][n] in T: 1/(1 + Δt d) (init step), 1/(1 + 2Δt d) (afterwards)
   // FP64 semi-implicit data
   jgcm::VertCoef vc;
-  jgcm::VertCoef* d_vc;  // device copy read by the column and semi-implicit kernels
+  jgcm::VertCoef* d_vc;  // device copy
+  void* d_vt;            // its VertT of the state precision, read by the column, fixer and semi-implicit kernels
   double* div_mat;  // host nd*nd column-major
   double* d_W;      // device [2][N+1][nd][nd] (transposed: [c][r])
   float2* d_W2;     // FP32 path: the same as pairs hi + lo

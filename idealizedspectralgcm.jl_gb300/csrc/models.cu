@@ -183,7 +183,7 @@ struct HSColArgs {
   double inv_2n;  // 1 / (2 nlon), exact (nlon is a power of two)
   // the physics constants in T, formed on the host with the kernel's own T arithmetic (no FP64 ->
   // FP32 conversion per thread: those run on the FP64 pipe)
-  T sb, R, kap, cp_t, kv0, ka, ks, kt0, dTy, dthz, kappa_t;
+  T sb, R, kap, cp_t, rcp, kv0, ka, ks, kt0, dTy, dthz, kappa_t;
 };
 
 template <typename T>
@@ -192,6 +192,7 @@ void hs_col_consts(HSColArgs<T>& a) {
   a.sb = (T)a.sigma_b;
   a.R = (T)a.rdgas;
   a.cp_t = (T)a.cp;
+  a.rcp = (T)(1.0 / a.cp);
   a.kap = a.R / a.cp_t;
   a.kv0 = ((T)a.k_f / day) / ((T)1.0 - a.sb);
   a.ka = (T)a.k_a / day;
@@ -242,41 +243,56 @@ __device__ __forceinline__ R seg_excl_suffix(R x, int s) {  // sum over the lane
 // D_k = ln(p_{k+1/2} / p_{k-1/2}) = log1p(Δp_k / p_{k-1/2}) (no difference of two large logarithms),
 // ln p_{k+1/2} - ln p_k = 1 - p_{k-1/2} D_k / Δp_k, ln p_k - ln p_{k-1/2} = D_k - that; the top level
 // has ln p_1 = ln p_{3/2} - 1.  Sigma coordinates read the same quantities as per-level constants.
+// Sigma coordinates (Δp_k = Δb_k ps): the mass divergence, the mass flux and the layer thickness all carry
+// one factor ps, which cancels in every tendency, and ∇ ln p_k is a per-level multiple of ∇ ln ps; so the
+// kernel works per unit of ps and a point needs no division and no transcendental (the column one log
+// and one exp; T_eq's power is exp(κ cf_k) exp(κ ln(ps / p0))).  With a quotient per layer and interface,
+// an exp per point and the coefficients converted per block: T42L20 FP64 66.1 -> 44.1 us, FP32 14.4 -> 12.8 us,
+// 32 members 92.4 -> 84.5 us (event included).
 template <typename T, int S, bool HYB>
 __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeof(T) == 4 ? 6 : 1)
-    k_hs_column(HSColArgs<T> a, const VertCoef* __restrict__ vcp) {
+    k_hs_column(HSColArgs<T> a, const VertCoef* __restrict__ vcp, const VertT<T>* __restrict__ vtp) {
   const VertCoef& vc = *vcp;
+  const VertT<T>& vt = *vtp;
   __shared__ double red[2][HS_CT / 32];
-  // the vertical coefficients in the state precision, staged once per block (constants: staged
-  // before the dependency wait; on the FP32 path this also keeps the FP64 -> FP32 conversions out of
-  // the level loops)
-  __shared__ T s_dak[JGCM_MAX_ND], s_dbk[JGCM_MAX_ND], s_bk[JGCM_MAX_ND + 1], s_cf[JGCM_MAX_ND],
-      s_dlpp[JGCM_MAX_ND], s_dlpm[JGCM_MAX_ND], s_dlp[JGCM_MAX_ND], s_sf[JGCM_MAX_ND];
-  __shared__ T s_lb1;
-  __shared__ T s_ak[JGCM_MAX_ND + 1];  // hybrid coordinates: a_k in the state precision
-  __shared__ double s_dak64[JGCM_MAX_ND], s_dbk64[JGCM_MAX_ND];  // FP64 layer coefficients: the energy integral
-  __shared__ float s_dah[JGCM_MAX_ND], s_dal[JGCM_MAX_ND], s_dbh[JGCM_MAX_ND], s_dbl[JGCM_MAX_ND];  // as FP32 pairs
+  // the vertical coefficients, staged once per block (constants: staged before the dependency wait)
+  __shared__ T s_dbk[JGCM_MAX_ND], s_bk[JGCM_MAX_ND + 1], s_cf[JGCM_MAX_ND], s_ek[JGCM_MAX_ND], s_dlpp[JGCM_MAX_ND],
+      s_dlp[JGCM_MAX_ND], s_rdb[JGCM_MAX_ND], s_w1[JGCM_MAX_ND], s_x1[JGCM_MAX_ND], s_kv[JGCM_MAX_ND], s_kt[JGCM_MAX_ND];
+  __shared__ T s_dak[HYB ? JGCM_MAX_ND : 1], s_ak[HYB ? JGCM_MAX_ND + 1 : 1];  // hybrid coordinates
+  // FP64 layer coefficients (the energy integral), as FP32 pairs on the FP32 path
+  __shared__ double s_dak64[sizeof(T) == 8 ? JGCM_MAX_ND : 1], s_dbk64[sizeof(T) == 8 ? JGCM_MAX_ND : 1];
+  __shared__ float s_dah[JGCM_MAX_ND], s_dal[JGCM_MAX_ND], s_dbh[JGCM_MAX_ND], s_dbl[JGCM_MAX_ND];
   const int nd = a.nd, nlon = a.nlon, nlat = a.nlat;
   for (int q = threadIdx.x; q <= nd; q += blockDim.x) {
-    s_bk[q] = (T)vc.bk[q];
-    s_ak[q] = (T)vc.ak[q];
+    s_bk[q] = vt.bk[q];
+    if constexpr (HYB) s_ak[q] = vt.ak[q];
     if (q < nd) {
-      s_dak64[q] = vc.dak[q];
-      s_dbk64[q] = vc.dbk[q];
-      s_dah[q] = vc.dak_hi[q];
-      s_dal[q] = vc.dak_lo[q];
-      s_dbh[q] = vc.dbk_hi[q];
-      s_dbl[q] = vc.dbk_lo[q];
-      s_dak[q] = (T)vc.dak[q];
-      s_dbk[q] = (T)vc.dbk[q];
-      s_cf[q] = (T)vc.cf[q];
-      s_dlpp[q] = (T)vc.dlp_p[q];
-      s_dlpm[q] = (T)vc.dlp_m[q];
-      s_dlp[q] = (T)vc.dlp[q];
-      s_sf[q] = (T)vc.sf[q];
+      if constexpr (sizeof(T) == 8) {
+        s_dak64[q] = vc.dak[q];
+        s_dbk64[q] = vc.dbk[q];
+      } else {
+        s_dah[q] = vc.dak_hi[q];
+        s_dal[q] = vc.dak_lo[q];
+        s_dbh[q] = vc.dbk_hi[q];
+        s_dbl[q] = vc.dbk_lo[q];
+      }
+      s_dbk[q] = vt.dbk[q];
+      if constexpr (HYB) {
+        s_dak[q] = vt.dak[q];
+      } else {
+        s_cf[q] = vt.cf[q];
+        s_ek[q] = vt.ek[q];
+        s_dlpp[q] = vt.dlp_p[q];
+        s_dlp[q] = vt.dlp[q];
+        s_rdb[q] = vt.rdb[q];
+        s_w1[q] = vt.w1[q];
+        s_x1[q] = vt.x1[q];
+        const T sg = vt.sf[q] - a.sb, smax = sg > (T)0 ? sg : (T)0;  // HS_Forcing! (sigma = p_k / ps)
+        s_kv[q] = a.kv0 * smax;
+        s_kt[q] = a.kt0 * smax;
+      }
     }
   }
-  if (threadIdx.x == 0) s_lb1 = (T)vc.lb[1];
   __syncthreads();
   pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
   const int seg = threadIdx.x % S, i = blockIdx.x * (HS_CT / S) + threadIdx.x / S, j = blockIdx.y, e = blockIdx.z;
@@ -290,16 +306,24 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
   const T* __restrict__ t_c = a.t_c + cL;
   const T* __restrict__ dvgp = a.div + cL;
   const T sj = a.sinj[j], s2 = sj * sj, c2 = (T)1.0 - s2, c4 = c2 * c2, cj = a.cosj[j], fj = a.coriolis[j];
-  const T sb = a.sb, R = a.R, kap = a.kap, cp = a.cp_t;
-  const T kv0 = a.kv0, ka = a.ka, kt0 = a.kt0;
-  const T ln_pref = (T)11.512925464970229;  // ln 1e5 (HS_Forcing.jl:49 p_ref)
+  const T R = a.R, kap = a.kap, ka = a.ka;
   const T tDt = (T)a.Dt;
   const T ps = act ? a.ps_c[c1] : (T)1, psp = act ? a.ps_p[c1] : (T)0;
-  // ∇ps / cos θ = (∇ ln ps / cos θ) ps (Spectral_Dynamics.jl:259-264)
-  const T dlps = act ? a.dlps[c1] * ps : (T)0, dtps = act ? a.dtps[c1] * ps : (T)0;
+  // ∇ps / cos θ = (∇ ln ps / cos θ) ps (Spectral_Dynamics.jl:259-264), per unit of ps on sigma levels
+  const T gps = HYB ? ps : (T)1;
+  const T dlps = act ? a.dlps[c1] * gps : (T)0, dtps = act ? a.dtps[c1] * gps : (T)0;
   const T gs = act ? a.geopots[c1] : (T)0;
   // ---- pressure variables from ps_c (Pressure_Variables!, Press_And_Geopot.jl:36-67)
-  const T lnps = log(ps);
+  T lr = 0, e0 = 0;  // sigma levels: ln(ps / p0) (p0 = 1e5, HS_Forcing.jl:49) and exp(κ of it)
+  if constexpr (!HYB) {
+    lr = log(ps * (T)1.0e-5);
+    e0 = exp(a.kappa_t * lr);
+  }
+  // Δp_k, and the mass divergence of level k (both per unit of ps on sigma levels)
+  auto layer = [&](int k) -> T { return HYB ? s_dak[HYB ? k : 0] + s_dbk[k] * ps : s_dbk[k]; };
+  auto mass_div = [&](int k, T u, T v, T dvg, T dp) -> T {
+    return HYB ? dvg * dp + s_dbk[k] * (u * dlps + v * dtps) : dp * (dvg + (u * dlps + v * dtps));
+  };
   // the level's log-pressure differences: dlnp = ln p_{k+1/2} - ln p_{k-1/2} (k = 0: ln p_{3/2}),
   // dlpp = ln p_{k+1/2} - ln p_k, dlpm = ln p_k - ln p_{k-1/2} (k = 0: ln p_1), lnpf = ln p_k
   auto logs = [&](int k, T& dlnp, T& dlpp, T& dlpm, T& lnpf) {
@@ -317,11 +341,11 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
         dlpm = dlnp - dlpp;
         lnpf = lph - dlpp;
       }
-    } else {
-      dlnp = k == 0 ? s_lb1 + lnps : s_dlp[k];
+    } else {  // (k = 0: ln p_{3/2} multiplies empty sums only, and no sigma formula reads dlpm)
+      dlnp = s_dlp[k];
       dlpp = s_dlpp[k];
-      lnpf = s_cf[k] + lnps;
-      dlpm = k == 0 ? lnpf : s_dlpm[k];
+      lnpf = s_cf[k] + lr;  // relative to ln p0
+      dlpm = 0;
     }
   };
   // ---- pass 1: Compute_Geopotential! (Press_And_Geopot.jl:71-111) on T - T0_k with T0_k the level's
@@ -346,7 +370,7 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
       logs(k, dlnp, dlpp, dlpm, lnpf);
       termS += R * td * dlnp;
       if constexpr (HYB) term0S += R * t0 * dlnp;
-      dmeanS += dvg * (s_dak[k] + s_dbk[k] * ps) + s_dbk[k] * (u * dlps + v * dtps);
+      dmeanS += mass_div(k, u, v, dvg, layer(k));
     }
   const T tot = seg_sum<S>(dmeanS);
   T rs = seg_excl_suffix<S>(termS, seg);  // sum_{r >= k1} R (T_r - T0_r) dlnp_r
@@ -381,12 +405,12 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
   if (act && k0 < k1) {
     T incl = incl0, Mlo = 0, flu = 0, flv = 0, flt = 0;  // M and the advective fluxes at k0-1/2
     T u = u_c[(size_t)k0 * G], v = v_c[(size_t)k0 * G], t = t_c[(size_t)k0 * G];
-    T dp = s_dak[k0] + s_dbk[k0] * ps;
+    T dp = layer(k0);
     if (k0 > 0) {  // the level above the segment: M_{k0-1/2} and its fluxes
       const size_t x = (size_t)(k0 - 1) * G;
-      const T um = u_c[x], vm = v_c[x], tm = t_c[x], dpm = s_dak[k0 - 1] + s_dbk[k0 - 1] * ps;
+      const T um = u_c[x], vm = v_c[x], tm = t_c[x], dpm = layer(k0 - 1);
       Mlo = -incl0 + tot * s_bk[k0];
-      const T w = dpm / (dpm + dp);
+      const T w = HYB ? dpm / (dpm + dp) : s_w1[k0 - 1];
       flu = Mlo * (um + (u - um) * w);
       flv = Mlo * (vm + (v - vm) * w);
       flt = Mlo * (tm + (t - tm) * w);
@@ -413,28 +437,35 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
         u1 = u_c[x + G];
         v1 = v_c[x + G];
         t1 = t_c[x + G];
-        dp1 = s_dak[k + 1] + s_dbk[k + 1] * ps;
+        dp1 = layer(k + 1);
       }
-      const T rdp = (T)1 / dp;
+      const T rdp = HYB ? (T)1 / dp : s_rdb[k];
       T dlnp, dlnp_p, dlnp_m, lnpf;  // ln p_{k+1/2} - ln p_k, ln p_k - ln p_{k-1/2} (ln p_{1/2} = 0)
       logs(k, dlnp, dlnp_p, dlnp_m, lnpf);
       // HS_Forcing! on the previous level (sigma = p_k / ps: sf[k] in sigma coordinates)
-      T sg;
-      if constexpr (HYB) sg = exp(lnpf) / ps - sb;
-      else sg = s_sf[k] - sb;
-      const T smax = sg > (T)0 ? sg : (T)0;
-      const T k_v = kv0 * smax;
+      T k_v, k_t, lpn, pk;  // lpn = ln(p / p0), pk = (p / p0)^κ
+      if constexpr (HYB) {
+        const T sg = exp(lnpf) / ps - a.sb, smax = sg > (T)0 ? sg : (T)0;
+        k_v = a.kv0 * smax;
+        k_t = a.kt0 * smax;
+        lpn = lnpf - (T)11.512925464970229;
+        pk = exp(a.kappa_t * lpn);
+      } else {
+        k_v = s_kv[k];
+        k_t = s_kt[k];
+        lpn = lnpf;
+        pk = s_ek[k] * e0;
+      }
       T du = -k_v * up, dv = -k_v * vp;
-      T dt = -((up + (T)0.5 * du * tDt) * du + (vp + (T)0.5 * dv * tDt) * dv) / cp;
-      const T lpn = lnpf - ln_pref;  // ln(p / p_ref)
-      T teq = ((T)315.0 - a.dTy * s2 - a.dthz * c2 * lpn) * exp(a.kappa_t * lpn);
+      T dt = -((up + (T)0.5 * du * tDt) * du + (vp + (T)0.5 * dv * tDt) * dv) * a.rcp;
+      T teq = ((T)315.0 - a.dTy * s2 - a.dthz * c2 * lpn) * pk;
       teq = teq > (T)200.0 ? teq : (T)200.0;
-      dt = dt - (ka + kt0 * smax * c4) * (tp - teq);
+      dt = dt - (ka + k_t * c4) * (tp - teq);
       // Compute_Corrections_Init: column energy integral with ps_p
       {
         const T ua = up + tDt * du, va = vp + tDt * dv;
         const T te = tp + tDt * dt;
-        col_e += ((T)0.5 * (ua * ua + va * va)) * (s_dak[k] + s_dbk[k] * psp);
+        col_e += ((T)0.5 * (ua * ua + va * va)) * (HYB ? s_dak[HYB ? k : 0] + s_dbk[k] * psp : s_dbk[k]);
         if constexpr (std::is_same<T, float>::value) {
           if constexpr (HYB) ds_add_prod(ah, al, te, s_dah[k], s_dal[k]);  // Δa_k = 0 on sigma levels
           ds_add_prod(bh, bl, te, s_dbh[k], s_dbl[k]);
@@ -445,20 +476,20 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
         }
       }
       // Four_In_One! (Spectral_Dynamics.jl:88-183)
-      const T x1 = (s_bk[k] * dlnp_m + s_bk[k + 1] * dlnp_p) * rdp;
+      const T x1 = HYB ? (s_bk[k] * dlnp_m + s_bk[k + 1] * dlnp_p) * rdp : s_x1[k];
       const T dlnp_dl = x1 * dlps, dlnp_dt = x1 * dtps;
       du = du - R * t * dlnp_dl;
       dv = dv - R * t * dlnp_dt;
-      const T dmean = dvg * dp + s_dbk[k] * (u * dlps + v * dtps);
+      const T dmean = mass_div(k, u, v, dvg, dp);
       const T excl = incl;
       incl += dmean;
       const T x5 = -(excl * dlnp + dmean * dlnp_p) * rdp + u * dlnp_dl + v * dlnp_dt;
       dt = dt + kap * t * x5;
       // M_{k+1/2} = -sum_{r<=k} D_r + B_{k+1/2} sum_r D_r, zero at the surface
       const T Mhi = below ? -incl + tot * s_bk[k + 1] : (T)0;
-      if (o_mh) o_mh[x] = Mhi;
+      if (o_mh) o_mh[x] = HYB ? Mhi : Mhi * ps;
       // Vert_Advection! (second_centered_wts): flux at k+1/2 with weight dp_k / (dp_k + dp_{k+1})
-      const T w1 = dp / (dp + dp1);
+      const T w1 = HYB ? dp / (dp + dp1) : s_w1[k];
       const T fhu = below ? Mhi * (u + (u1 - u) * w1) : (T)0;
       const T fhv = below ? Mhi * (v + (v1 - v) * w1) : (T)0;
       const T fht = below ? Mhi * (t + (t1 - t) * w1) : (T)0;
@@ -488,11 +519,12 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
     col_ta = (double)ah + (double)al;
     col_tb = (double)bh + (double)bl;
   }
+  if constexpr (!HYB) col_e *= psp;
   double col_ed = (double)col_e + a.cp * (col_ta + col_tb * (double)psp);
   col_ed = seg_sum<S>(col_ed);
   double accp = 0.0, acce = 0.0;
   if (act && seg == 0) {
-    a.dlnps[c1] = (-tot) / ps;  // grid_δlnps = grid_δps / ps (Spectral_Dynamics.jl:279)
+    a.dlnps[c1] = HYB ? (-tot) / ps : -tot;  // grid_δlnps = grid_δps / ps (Spectral_Dynamics.jl:279)
     accp = (double)psp;
     acce = col_ed;
   }
@@ -539,13 +571,12 @@ struct TracerArgs {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(128) k_hs_tracers(TracerArgs<T> a, const VertCoef* __restrict__ vcp) {
-  const VertCoef& vc = *vcp;
+__global__ void __launch_bounds__(128) k_hs_tracers(TracerArgs<T> a, const VertT<T>* __restrict__ vtp) {
   __shared__ T s_dak[JGCM_MAX_ND], s_dbk[JGCM_MAX_ND];
   const int nd = a.nd;
   for (int q = threadIdx.x; q < nd; q += blockDim.x) {
-    s_dak[q] = (T)vc.dak[q];
-    s_dbk[q] = (T)vc.dbk[q];
+    s_dak[q] = vtp->dak[q];
+    s_dbk[q] = vtp->dbk[q];
   }
   __syncthreads();
   pdl_wait();  // programmatic dependent launch: the column kernel's mass flux is complete
@@ -589,19 +620,21 @@ inline int hs_lanes(const jgcm_mesh* m, int ne, int nd) {
 }
 
 template <typename T, bool HYB>
-int launch_hs_column_v(const HSColArgs<T>& a, const jgcm_mesh* m, int ne, int S, const VertCoef* vc, cudaStream_t st) {
+int launch_hs_column_v(const HSColArgs<T>& a, const jgcm_mesh* m, int ne, int S, const VertCoef* vc, const VertT<T>* vt,
+                       cudaStream_t st) {
   const int cpb = HS_CT / S;  // columns per block
   dim3 g((m->nlon + cpb - 1) / cpb, m->nlat, ne);
-  if (S == 1) JG_CUDA(launch_pdl(k_hs_column<T, 1, HYB>, g, HS_CT, 0, st, a, vc));
-  else if (S == 2) JG_CUDA(launch_pdl(k_hs_column<T, 2, HYB>, g, HS_CT, 0, st, a, vc));
-  else if (S == 4) JG_CUDA(launch_pdl(k_hs_column<T, 4, HYB>, g, HS_CT, 0, st, a, vc));
-  else JG_CUDA(launch_pdl(k_hs_column<T, 8, HYB>, g, HS_CT, 0, st, a, vc));
+  if (S == 1) JG_CUDA(launch_pdl(k_hs_column<T, 1, HYB>, g, HS_CT, 0, st, a, vc, vt));
+  else if (S == 2) JG_CUDA(launch_pdl(k_hs_column<T, 2, HYB>, g, HS_CT, 0, st, a, vc, vt));
+  else if (S == 4) JG_CUDA(launch_pdl(k_hs_column<T, 4, HYB>, g, HS_CT, 0, st, a, vc, vt));
+  else JG_CUDA(launch_pdl(k_hs_column<T, 8, HYB>, g, HS_CT, 0, st, a, vc, vt));
   return JGCM_OK;
 }
 template <typename T>
-int launch_hs_column(const HSColArgs<T>& a, const jgcm_mesh* m, int ne, int S, const VertCoef* vc, bool hybrid,
-                     cudaStream_t st) {
-  return hybrid ? launch_hs_column_v<T, true>(a, m, ne, S, vc, st) : launch_hs_column_v<T, false>(a, m, ne, S, vc, st);
+int launch_hs_column(const HSColArgs<T>& a, const jgcm_mesh* m, int ne, int S, const VertCoef* vc, const VertT<T>* vt,
+                     bool hybrid, cudaStream_t st) {
+  return hybrid ? launch_hs_column_v<T, true>(a, m, ne, S, vc, vt, st)
+                : launch_hs_column_v<T, false>(a, m, ne, S, vc, vt, st);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -652,23 +685,21 @@ struct CX {
 // staged once per block (the same FP64 expressions, rounded once instead of in every warp)
 template <typename R>
 struct VertR {
-  R dpr[JGCM_MAX_ND], rdpr[JGCM_MAX_ND], dlnp[JGCM_MAX_ND], dlnpp[JGCM_MAX_ND], tref[JGCM_MAX_ND],
-      bk1[JGCM_MAX_ND], tdh[JGCM_MAX_ND], dh[JGCM_MAX_ND], df[JGCM_MAX_ND], hk[JGCM_MAX_ND];
+  R dpr[JGCM_MAX_ND], rdpr[JGCM_MAX_ND], dlnp[JGCM_MAX_ND], dlnpp[JGCM_MAX_ND], tref[JGCM_MAX_ND], bk1[JGCM_MAX_ND],
+      tdh[JGCM_MAX_ND], hk[JGCM_MAX_ND];
 };
 
 template <typename R>
-__device__ __forceinline__ void stage_vert(const VertCoef& vc, int nd, double ps_ref, VertR<R>& v) {
+__device__ __forceinline__ void stage_vert(const VertT<R>& vt, int nd, VertR<R>& v) {
   for (int k = threadIdx.x; k < nd; k += blockDim.x) {
-    v.dpr[k] = (R)vc.dp_ref[k];
-    v.rdpr[k] = (R)vc.rdp_ref[k];
-    v.dlnp[k] = (R)(vc.lnph_ref[k + 1] - vc.lnph_ref[k]);
-    v.dlnpp[k] = (R)(vc.lnph_ref[k + 1] - vc.lnpf_ref[k]);
-    v.tref[k] = (R)vc.t_ref[k];
-    v.bk1[k] = (R)vc.bk[k + 1];
-    v.tdh[k] = k + 1 <= nd - 1 ? (R)(vc.t_ref[k + 1] - vc.t_ref[k]) : (R)0;
-    v.dh[k] = (R)(vc.lnph_ref[k + 1] - vc.lnph_ref[k]);
-    v.df[k] = (R)(vc.lnph_ref[k + 1] - vc.lnpf_ref[k]);
-    v.hk[k] = (R)(vc.h[k] * ps_ref);
+    v.dpr[k] = vt.dpr[k];
+    v.rdpr[k] = vt.rdpr[k];
+    v.dlnp[k] = vt.dlnp[k];
+    v.dlnpp[k] = vt.dlnpp[k];
+    v.tref[k] = vt.tref[k];
+    v.bk1[k] = vt.bk[k + 1];
+    v.tdh[k] = vt.tdh[k];
+    v.hk[k] = vt.hk[k];
   }
 }
 
@@ -725,10 +756,9 @@ __device__ __forceinline__ void lf(int init, int Dt, R rob, R d, R f, R& dq, R q
 // (mode, component, row) output each, instead of one mode per warp, whose 32 - nd idle lanes the
 // FP64 pipe executes all the same (for launches with many modes: member ensembles).
 template <typename T, typename R, bool DENSE = false>
-__global__ void __launch_bounds__(256) k_hs_implicit(ImplArgs<T> a, const VertCoef* __restrict__ vcp) {
-  const VertCoef& vc = *vcp;
+__global__ void __launch_bounds__(256) k_hs_implicit(ImplArgs<T> a, const VertT<R>* __restrict__ vtp) {
   __shared__ VertR<R> vr;
-  stage_vert<R>(vc, a.nd, a.ps_ref, vr);  // constants: staged before the dependency wait
+  stage_vert<R>(*vtp, a.nd, vr);  // constants: staged before the dependency wait
   __syncthreads();
   pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
   using C = CX<R>;
@@ -764,11 +794,11 @@ __global__ void __launch_bounds__(256) k_hs_implicit(ImplArgs<T> a, const VertCo
   C t2 = {tp.x - tc.x + xi * dtt.x, tp.y - tc.y + xi * dtt.y};
   C l2 = {lp.x - lc.x + xi * dl.x, lp.y - lc.y + xi * dl.y};
   // Linear_Geopot_δt! :213-241
-  R dh = vr.dh[k];
+  R dh = vr.dlnp[k];
   R tmx = act ? Rg * (t2.x * dh) : (R)0, tmy = act ? Rg * (t2.y * dh) : (R)0;
   R rx = rscan_incl<R>(tmx, lane), ry = rscan_incl<R>(tmy, lane);
   R hx = shfl_dn1(rx, lane, nd, (R)0), hy = shfl_dn1(ry, lane, nd, (R)0);  // Φ_{k+1/2}
-  R df = vr.df[k];
+  R df = vr.dlnpp[k];
   R gx = hx + Rg * (t2.x * df), gy = hy + Rg * (t2.y * df);
   R hk = vr.hk[k];
   ddiv.x = ddiv.x - eig * (gx + hk * l2.x);
@@ -940,7 +970,7 @@ __device__ __forceinline__ double corr_col_share(const CorrArgs<T>& a, const dou
 // CL: the first fold level in thread-block clusters (launched with a cluster shape), else in
 // groups of CORR_GS blocks
 template <typename T, bool CL>
-__global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const VertCoef* __restrict__ vcp) {
+__global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const VertCoef* __restrict__ vcp, const VertT<T>* __restrict__ vtp) {
   const VertCoef& vc = *vcp;
   // block = 32 consecutive columns of one latitude row x 8 level groups: warp ks reads levels
   // ks, ks + 8, ... of the 32 columns (coalesced rows)
@@ -949,8 +979,8 @@ __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const Ver
   __shared__ double s_dak64[JGCM_MAX_ND], s_dbk64[JGCM_MAX_ND];  // and in FP64 (the c_p T sums)
   __shared__ float s_dah[JGCM_MAX_ND], s_dal[JGCM_MAX_ND], s_dbh[JGCM_MAX_ND], s_dbl[JGCM_MAX_ND];  // FP32 pairs
   for (int q = threadIdx.x; q < a.nd; q += blockDim.x) {
-    s_dak[q] = (T)vc.dak[q];
-    s_dbk[q] = (T)vc.dbk[q];
+    s_dak[q] = vtp->dak[q];
+    s_dbk[q] = vtp->dbk[q];
     s_dak64[q] = vc.dak[q];
     s_dbk64[q] = vc.dbk[q];
     s_dah[q] = vc.dak_hi[q];
@@ -1427,6 +1457,46 @@ void vertical_setup(jgcm_model* md) {
     }
 }
 
+int alloc(void** p, size_t bytes);
+
+// The vertical coefficients of the kernels, each formed in FP64 and rounded once.
+template <typename T>
+int build_vert_t(jgcm_model* md) {
+  const VertCoef& vc = md->vc;
+  const int nd = md->nd;
+  std::vector<VertT<T>> h(1);
+  VertT<T>& v = h[0];
+  memset(&v, 0, sizeof(v));
+  for (int k = 0; k <= nd; k++) {
+    v.ak[k] = (T)vc.ak[k];
+    v.bk[k] = (T)vc.bk[k];
+  }
+  for (int k = 0; k < nd; k++) {
+    v.dak[k] = (T)vc.dak[k];
+    v.dbk[k] = (T)vc.dbk[k];
+    if (!vc.hybrid) {
+      v.cf[k] = (T)vc.cf[k];
+      v.sf[k] = (T)vc.sf[k];
+      v.ek[k] = (T)std::exp(md->P.kappa * vc.cf[k]);
+      v.dlp_p[k] = (T)vc.dlp_p[k];
+      v.dlp[k] = (T)vc.dlp[k];
+      v.rdb[k] = (T)(1.0 / vc.dbk[k]);
+      if (k + 1 < nd) v.w1[k] = (T)(vc.dbk[k] / (vc.dbk[k] + vc.dbk[k + 1]));
+      v.x1[k] = (T)((vc.bk[k] * vc.dlp_m[k] + vc.bk[k + 1] * vc.dlp_p[k]) / vc.dbk[k]);
+    }
+    v.dpr[k] = (T)vc.dp_ref[k];
+    v.rdpr[k] = (T)vc.rdp_ref[k];
+    v.dlnp[k] = (T)(vc.lnph_ref[k + 1] - vc.lnph_ref[k]);
+    v.dlnpp[k] = (T)(vc.lnph_ref[k + 1] - vc.lnpf_ref[k]);
+    v.tref[k] = (T)vc.t_ref[k];
+    v.tdh[k] = k + 1 <= nd - 1 ? (T)(vc.t_ref[k + 1] - vc.t_ref[k]) : (T)0;
+    v.hk[k] = (T)(vc.h[k] * md->P.ps_ref);
+  }
+  JG_TRY(alloc(&md->d_vt, sizeof(v)));
+  JG_CUDA(cudaMemcpy(md->d_vt, &v, sizeof(v), cudaMemcpyHostToDevice));
+  return JGCM_OK;
+}
+
 // ------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void k_fill_damping(const double* eig, T* out, int N, int ns, double coef, int order, double dt_eff) {
@@ -1481,7 +1551,7 @@ void model_free(jgcm_model* md) {
                 md->spe_zero, md->spe_dvor, md->spe_ddiv, md->spe_dlnps, md->spe_dt, md->g_dlps, md->g_dtps,
                 md->g_dlT, md->g_dtT, md->g_ducos, md->g_dvcos, md->g_dt, md->g_energy, md->g_dlnps, md->g_diag,
                 md->g_tdev, md->coriolis, md->damping, md->dfac[0], md->dfac[1], md->d_W, md->d_W2, md->d_pairs, md->d_partials,
-                md->d_scalars, md->d_counter, md->d_vc, md->fbuf, md->diag};
+                md->d_scalars, md->d_counter, md->d_vc, md->d_vt, md->fbuf, md->diag};
   for (auto p : ps)
     if (p) cudaFree(p);
   delete[] md->div_mat;
@@ -1613,6 +1683,7 @@ int model_alloc(jgcm_model* md) {
   vertical_setup(md);
   JG_TRY(alloc((void**)&md->d_vc, sizeof(VertCoef)));
   JG_CUDA(cudaMemcpy(md->d_vc, &md->vc, sizeof(VertCoef), cudaMemcpyHostToDevice));
+  JG_TRY(is_fp64(m) ? build_vert_t<double>(md) : build_vert_t<float>(md));
   if (md->P.kind == JGCM_HELD_SUAREZ) JG_TRY(build_wave(md));
   JG_CUDA(cudaStreamSynchronize(m->stream));
   return JGCM_OK;
@@ -1939,7 +2010,7 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
   a.inv_2n = 0.5 / m->nlon;
   a.pstride = partial_stride(m);
   hs_col_consts<T>(a);
-  JG_TRY(launch_hs_column<T>(a, m, E, md->hs_lanes, md->d_vc, md->vc.hybrid, st));
+  JG_TRY(launch_hs_column<T>(a, m, E, md->hs_lanes, md->d_vc, (const VertT<T>*)md->d_vt, md->vc.hybrid, st));
   mark(st);
   JG_CUDA(cudaGetLastError());
   if (md->nq) {  // 2'. the tracers' tendencies
@@ -1956,7 +2027,7 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
     ta.nq = md->nq;
     ta.nlat = m->nlat;
     ta.nlon = m->nlon;
-    JG_CUDA(launch_pdl(k_hs_tracers<T>, dim3((m->nlon + 127) / 128, m->nlat, E), 128, 0, st, ta, md->d_vc));
+    JG_CUDA(launch_pdl(k_hs_tracers<T>, dim3((m->nlon + 127) / 128, m->nlat, E), 128, 0, st, ta, (const VertT<T>*)md->d_vt));
     mark(st);
     JG_CUDA(cudaGetLastError());
   }
@@ -2042,11 +2113,11 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
   // 4 modes per block: (N+1)(N+2)/2 + N+1 modes at T42 make 248 blocks, every SM's FP64 units busy;
   // FP64 member ensembles (from 4 members) spread the FP64 products densely over each block
   if constexpr (std::is_same<T, float>::value)
-    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, md->d_vc));
+    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, (const VertT<T>*)md->d_vt));
   else if (E >= 4)
-    JG_CUDA(launch_pdl(k_hs_implicit<T, T, true>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, md->d_vc));
+    JG_CUDA(launch_pdl(k_hs_implicit<T, T, true>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, (const VertT<T>*)md->d_vt));
   else
-    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, md->d_vc));
+    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, (const VertT<T>*)md->d_vt));
   mark(st);
   JG_CUDA(cudaGetLastError());
   // 5. back to the grid: vor, div, u, v, T, lnps (+ ps = exp(lnps)), and the next step's gradients
@@ -2138,9 +2209,10 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
       int cx, cy;
       corr_cluster(gx, m->nlat, cx, cy);
       JG_CUDA(launch_pdl_cluster(k_hs_corr_reduce<T, true>, dim3(gx, m->nlat, E), 256, 0, st, dim3(cx, cy, 1), ca,
-                                 md->d_vc));
+                                 md->d_vc, (const VertT<T>*)md->d_vt));
     } else {
-      JG_CUDA(launch_pdl(k_hs_corr_reduce<T, false>, dim3(gx, m->nlat, E), 256, 0, st, ca, md->d_vc));
+      JG_CUDA(launch_pdl(k_hs_corr_reduce<T, false>, dim3(gx, m->nlat, E), 256, 0, st, ca, md->d_vc,
+                         (const VertT<T>*)md->d_vt));
     }
   }
   mark(st);
@@ -3793,9 +3865,9 @@ extern "C" int jgcm_model_semi_implicit_step(jgcm_model* md, const double* const
   JG_CUDA(cudaMemcpyAsync(dout[5], din[9], spec_elems(m, md->nd) * 2 * ts, cudaMemcpyDeviceToDevice, st));
   JG_CUDA(cudaMemcpyAsync(dout[7], din[11], spec_elems(m, 1) * 2 * ts, cudaMemcpyDeviceToDevice, st));
   if (is_fp64(m))
-    k_hs_implicit<double, double><<<(md->npairs + 7) / 8, 256, 0, st>>>(si_args<double>(md, din, dout), md->d_vc);
+    k_hs_implicit<double, double><<<(md->npairs + 7) / 8, 256, 0, st>>>(si_args<double>(md, din, dout), (const VertT<double>*)md->d_vt);
   else
-    k_hs_implicit<float, float><<<(md->npairs + 7) / 8, 256, 0, st>>>(si_args<float>(md, din, dout), md->d_vc);
+    k_hs_implicit<float, float><<<(md->npairs + 7) / 8, 256, 0, st>>>(si_args<float>(md, din, dout), (const VertT<float>*)md->d_vt);
   JG_CUDA(cudaGetLastError());
   for (int i = 0; i < 8; i++) {
     const size_t nn = 2 * spec_elems(m, si_levels_out(md, i));
