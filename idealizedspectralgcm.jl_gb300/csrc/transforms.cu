@@ -275,6 +275,10 @@ __device__ __forceinline__ T fft_load(const FFTPlan& plan, const GridInGroup& g,
   return x;
 }
 
+}  // namespace jgcm
+#include "zonal_fft.cuh"
+namespace jgcm {
+
 // Fourier -> grid: inverse real FFT, one column per half-length (h = nlon/2) complex transform,
 // so rounding never leaks between columns of different magnitude.  grid (ceil(C/CT), nlat),
 // 256 threads.  Row x(λ_t) = Re g_0 + 2 Re sum_{m=1}^{N} g_m e^{imλ_t}, i.e. 2 nλ Re(ifft(g)) with
@@ -583,66 +587,6 @@ __device__ __forceinline__ void ifft_store_pair(const GridOutGroup& g, const Tab
   *reinterpret_cast<P*>((T*)g.dst + idx) = v;
 }
 
-// The epilogue of one warp's row (k_ifft_w): x(λ_2i) = re[r], x(λ_2i+1) = im[r] for i = lane + 32 r,
-// the group's epilogue chosen once per row and each pair of longitudes stored as one 8- or 16-byte
-// word.  ÷cos θ as a product with 1/cos θ (within an ulp of the quotient).
-template <typename T, int V>
-__device__ __forceinline__ void ifft_store_row(const GridOutGroup& g, const Tables<T>& tb, int k, int j, int nlat,
-                                               int nlon, const T (&re)[V], const T (&im)[V], int lane) {
-  using P = V2<T>;
-  const size_t row = ((size_t)k * nlat + j) * nlon;
-  P* dst = reinterpret_cast<P*>((T*)g.dst + row);
-  auto put = [](P* d, int i, T a, T b) {
-    P v;
-    v.x = a;
-    v.y = b;
-    d[i] = v;
-  };
-  switch (g.epi) {
-    case EPI_NONE:
-#pragma unroll
-      for (int r = 0; r < V; r++) put(dst, lane + 32 * r, re[r], im[r]);
-      break;
-    case EPI_DIVCOS: {
-      const T rc = (T)1 / tb.cosj[j];
-#pragma unroll
-      for (int r = 0; r < V; r++) put(dst, lane + 32 * r, re[r] * rc, im[r] * rc);
-    } break;
-    case EPI_EXP2: {
-      const T sh = pick<T>(g.shift, g.shiftf), es = pick<T>(g.eshift, g.eshiftf);
-      P* d2 = reinterpret_cast<P*>((T*)g.dst2 + row);
-#pragma unroll
-      for (int r = 0; r < V; r++) {
-        put(dst, lane + 32 * r, re[r] + sh, im[r] + sh);
-        put(d2, lane + 32 * r, exp(re[r]) * es, exp(im[r]) * es);
-      }
-    } break;
-    case EPI_DIVCOS_MULPS: {  // level k of ps
-      const T rc = (T)1 / tb.cosj[j];
-      const P* ps = reinterpret_cast<const P*>((const T*)g.ps + row);
-#pragma unroll
-      for (int r = 0; r < V; r++) {
-        const P q = ps[lane + 32 * r];
-        put(dst, lane + 32 * r, (re[r] * rc) * q.x, (im[r] * rc) * q.y);
-      }
-    } break;
-    case EPI_ADJ_G2S: {
-      const auto sc = tb.wts[j] / (T)(2 * nlon);
-#pragma unroll
-      for (int r = 0; r < V; r++) put(dst, lane + 32 * r, (T)(re[r] * sc), (T)(im[r] * sc));
-    } break;
-    case EPI_ANOM: {
-      const T mean = ((const V2<T>*)g.ps)[k].x;
-      P* d2 = reinterpret_cast<P*>((T*)g.dst2 + row);
-#pragma unroll
-      for (int r = 0; r < V; r++) {
-        put(dst, lane + 32 * r, re[r] + mean, im[r] + mean);
-        put(d2, lane + 32 * r, re[r], im[r]);
-      }
-    } break;
-  }
-}
-
 template <typename T, int V>
 __global__ void __launch_bounds__(256) k_ifft_w(IFFTPlan plan, Tables<T> tb, const V2<T>* __restrict__ F, int N,
                                                 int nlat, int nlon) {
@@ -682,7 +626,7 @@ __global__ void __launch_bounds__(256) k_ifft_w(IFFTPlan plan, Tables<T> tb, con
   warp_fft_dit<T, V>(re, im, tb.tw, lane);
   int k;
   const GridOutGroup& g = group_of(plan.g, plan.ng, c, &k);
-  ifft_store_row<T, V>(g, tb, k, j, nlat, nlon, re, im, lane);  // z[i] = x[2i] + i x[2i+1]
+  ifft_store_row<T, V>(g, tb, k, j, nlat, nlon, re, im, lane, 32);  // z[i] = x[2i] + i x[2i+1]
 }
 
 template <typename T, int V, bool PLAIN>
@@ -751,20 +695,12 @@ __global__ void __launch_bounds__(256) k_fft_w(FFTPlan plan, Tables<T> tb, V2<T>
 // parameter and read at compile-time indices (constant-bank operands: no loads, shuffles or block
 // barriers in the transform).  A warp's 32 rows pass through padded shared memory, so that every
 // global read and write is a coalesced row (grid) or a run of 32 consecutive columns (Fourier).
-// Same arithmetic as k_fft_w / k_ifft_w: the half-length complex transform of the real row.
+// The half-length complex transform of the real row.
 template <int NLON>
 struct RowTwiddles {
   float c[NLON / 2], s[NLON / 2];  // cos, sin of 2π t / nlon
 };
 constexpr int RF_WARPS = 4;               // warps per block, 32 rows each
-// rows from which the row-per-thread kernels are used: 128 per SM (4 warps), 19456 on GB300
-static inline size_t rows_min(const jgcm_mesh* m) { return (size_t)m->sm_count * 4 * 32; }
-
-__host__ __device__ constexpr int brev_c(int x, int bits) {
-  int r = 0;
-  for (int b = 0; b < bits; b++) r |= ((x >> b) & 1) << (bits - 1 - b);
-  return r;
-}
 
 // PLAIN: every group of the plan reads its field as it is (PRO_NONE): the prologue switch, inlined
 // for each of a warp's 32 rows, leaves the instruction stream
@@ -942,13 +878,13 @@ RowTwiddles<NLON> row_twiddles(const jgcm_mesh* m) {
   return t;
 }
 
-// FFT tile knob: 0 = by size, from rows_min rows on: nlon 64 both ways, nlon 128 the inverse only
-// (its thread holds 64 complex points in 158 registers and still beats the warp FFT, 135 -> 107 us
-// at T42 x 32 members; the forward one at 165 registers does not, 80 -> 190 us, measured);
-// -1 = rows per thread always (nlon 64 and 128)
-static inline bool use_row_fft(const jgcm_mesh* m, int C, bool inverse = false) {
+// FFT tile knob: 0 = by size: nlon 64 from 128 rows per SM on (128 x T21L20: forward 35 us against 45 split
+// in registers over four threads, whose loads cover 32 bytes of a row at a time, inverse 71 against 75; at
+// nlon 128 a thread's 64 points take 152 registers: inverse 90 against 76, forward 190 against 38);
+// -1 = rows per thread always (FP32, nlon 64 and 128)
+static inline bool use_row_fft(const jgcm_mesh* m, int C) {
   if (m->tune[3] == -1) return m->nlon == 64 || m->nlon == 128;
-  return m->tune[3] == 0 && (m->nlon == 64 || (inverse && m->nlon == 128)) && (size_t)C * m->nlat >= rows_min(m);
+  return m->tune[3] == 0 && m->nlon == 64 && (size_t)C * m->nlat >= (size_t)m->sm_count * 4 * 32;
 }
 static inline size_t row_fft_smem(const jgcm_mesh* m) { return (size_t)RF_WARPS * 32 * (m->nlon + 1) * sizeof(float); }
 
@@ -956,6 +892,7 @@ static inline size_t row_fft_smem(const jgcm_mesh* m) { return (size_t)RF_WARPS 
 // Shared memory holds, for the input slots in use, the hemisphere-symmetric and -antisymmetric
 // combinations g(mu_j) +/- g(-mu_j) of the tile's columns.
 constexpr int G2S_BLOCKS_PER_SM = 2;  // the row split's aim (launch_g2s)
+constexpr int FFT_BLOCKS_PER_SM = 4;  // the column tiles' (reg_fft_shape)
 // QL lanes per output (4: a quad splits the latitude sum and combines it with two shuffles, for
 // launches too small to fill the device; 1: a lane sums its output alone, half the instructions per
 // output, for launches with many outputs).
@@ -1260,6 +1197,67 @@ static G2SPlan with_f32(const G2SPlan& p) {
   return q;
 }
 
+// The register-split FFTs (zonal_fft.cuh): nlon 64 to 1024, unless the FFT tile knob names another kernel.
+// threads per row (zonal_fft.cuh)
+static inline int reg_fft_threads(int nlon) { return nlon == 64 ? 4 : nlon <= 256 ? 8 : 16; }
+// Which kernels transform the rows of a launch of C columns (tile knob 0): the register-split FFTs (nlon 64
+// to 1024) for fields of several levels.  T42L20, one member, FP32: a warp per row 9.0 and 12.4 us (forward and
+// inverse), split 8.8 and 8.5; 32 members 76 and 180, 38 and 76; T21L7, one member, equal (6.6 and 8.2).  FP64: in
+// shared memory 35 and 66, split 27 and 47.  With few rows the split threads' longer chains show (T85 shallow
+// water FP32 a warp per row 8.3 and 8.3, split 11.9 and 10.2 us; FP64 shared 16 and 21, split 39 and 25):
+// FP64 launches of less than two warps an SM keep the shared-memory kernels, and in FP32 fields of one level
+// a warp per row -- whatever their number, so that the members of an ensemble are transformed by the kernel
+// of a model of one, rounding for rounding.
+template <typename T>
+static bool reg_fft(const jgcm_mesh* m, int C) {
+  if (m->nlon < 64 || m->tune[3] != 0) return false;
+  if (sizeof(T) == 4) return m->nd > 1 && C > 2;
+  return (size_t)C * m->nlat * reg_fft_threads(m->nlon) >= (size_t)2 * 32 * m->sm_count;
+}
+// They move pairs of values: every field has to start on a pair's boundary (a caller's device grid may not).
+template <typename T>
+static bool pairs_aligned(const IFFTPlan& p) {
+  uintptr_t a = 0;
+  for (int i = 0; i < p.ng; i++) {
+    a |= (uintptr_t)p.g[i].dst;
+    if (p.g[i].epi == EPI_EXP2 || p.g[i].epi == EPI_ANOM) a |= (uintptr_t)p.g[i].dst2;
+    if (p.g[i].epi == EPI_DIVCOS_MULPS) a |= (uintptr_t)p.g[i].ps;
+  }
+  return a % sizeof(V2<T>) == 0;
+}
+template <typename T>
+static bool pairs_aligned(const FFTPlan& p) {
+  uintptr_t a = 0;
+  for (int i = 0; i < p.ng; i++)
+    if (p.g[i].pro == PRO_NONE) a |= (uintptr_t)p.g[i].src;
+  return a % sizeof(V2<T>) == 0;
+}
+struct RegFFT {
+  int lcb, tiles, threads;
+  dim3 grid;
+  size_t smem;
+};
+template <typename T>
+static RegFFT reg_fft_shape(const jgcm_mesh* m, int C) {
+  const int H = m->nlon / 2, R2 = reg_fft_threads(m->nlon);
+  const size_t row = (size_t)(H + H / R2 + 1) * sizeof(V2<T>);
+  RegFFT r;
+  // columns per block: 32 (256-byte runs of FP32 pairs), fewer where the rows would take more than 48 KB, the
+  // grid would leave SMs without a block, or, in FP64 (bound by its arithmetic: small blocks spread evenly,
+  // T63L20 140 -> 133 us), a block would hold more than two warps; a warp at least
+  r.lcb = 5;
+  while ((row << r.lcb) > 48 * 1024 || (sizeof(T) == 8 && (R2 << r.lcb) > 64)) r.lcb--;
+  while ((R2 << r.lcb) > 32 && (size_t)((C + (1 << r.lcb) - 1) >> r.lcb) * m->nlat < (size_t)FFT_BLOCKS_PER_SM * m->sm_count)
+    r.lcb--;
+  r.tiles = (C + (1 << r.lcb) - 1) >> r.lcb;
+  r.threads = R2 << r.lcb;
+  r.smem = row << r.lcb;
+  // a block walks several tiles where the grid is many waves deep: its twiddles are loaded once
+  const int per = std::max(1, std::min(4, (int)((size_t)r.tiles * m->nlat / ((size_t)16 * m->sm_count))));
+  r.grid = dim3((r.tiles + per - 1) / per, m->nlat);
+  return r;
+}
+
 template <typename T>
 static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip, cudaStream_t st, V2<T>* fbuf);
 
@@ -1291,7 +1289,7 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
   const IFFTPlan ip = with_f32(ip0);
   Tables<T> tb = tables<T>(m);
   const int fc = m->tune[3] > 0 ? fft_ct(m) : fit_ct(fft_ct(m), ip.C);
-  if (std::is_same<T, float>::value && use_row_fft(m, ip.C, true)) {  // many rows: a row per thread
+  if (std::is_same<T, float>::value && use_row_fft(m, ip.C)) {  // many rows: a row per thread
     dim3 gr((ip.C + 32 * RF_WARPS - 1) / (32 * RF_WARPS), m->nlat);
     const Tables<float> tf = tables<float>(m);
     const float2* Ff = (const float2*)fbuf;
@@ -1303,7 +1301,21 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
     JG_CUDA(cudaGetLastError());
     return JGCM_OK;
   }
-  // the warp-register FFT wins in FP32; in FP64 the shared-memory radix-2 kernel is faster (measured)
+  if (reg_fft<T>(m, ip.C) && pairs_aligned<T>(ip)) {
+    const RegFFT r = reg_fft_shape<T>(m, ip.C);
+#define JG_IFFT_REG(HH) launch_pdl(k_ifft_reg<T, HH>, r.grid, r.threads, r.smem, st, ip, tb, (const V*)fbuf, m->N, m->nlat, r.lcb, r.tiles)
+    switch (m->nlon) {
+      case 64: JG_CUDA(JG_IFFT_REG(32)); break;
+      case 128: JG_CUDA(JG_IFFT_REG(64)); break;
+      case 256: JG_CUDA(JG_IFFT_REG(128)); break;
+      case 512: JG_CUDA(JG_IFFT_REG(256)); break;
+      default: JG_CUDA(JG_IFFT_REG(512)); break;
+    }
+#undef JG_IFFT_REG
+    mark(st);
+    JG_CUDA(cudaGetLastError());
+    return JGCM_OK;
+  }
   if (std::is_same<T, float>::value && m->nlon >= 64 && m->nlon <= 1024 && m->tune[3] == 0) {
     const size_t smw = (size_t)(m->N + 1) * FW_COLS * sizeof(V);
     dim3 gw((ip.C + FW_COLS - 1) / FW_COLS, m->nlat);
@@ -1378,8 +1390,26 @@ int launch_fft_only(jgcm_mesh* m, const FFTPlan& fp0, cudaStream_t st, void* fbu
     JG_CUDA(cudaGetLastError());
     return JGCM_OK;
   }
-  // forward: the warp-register FFT wins in FP32 from nlon = 128 on (measured)
-  if (std::is_same<T, float>::value && m->nlon >= 128 && m->nlon <= 1024 && m->tune[3] == 0) {
+  if (reg_fft<T>(m, fp.C) && pairs_aligned<T>(fp)) {
+    const RegFFT r = reg_fft_shape<T>(m, fp.C);
+    bool plain = true;
+    for (int i = 0; i < fp.ng; i++) plain = plain && fp.g[i].pro == PRO_NONE;
+#define JG_FFT_REG(HH)                                                                                                        \
+  (plain ? launch_pdl(k_fft_reg<T, HH, true>, r.grid, r.threads, r.smem, st, fp, tb, (V*)fbuf, m->N, m->nlat, r.lcb, r.tiles) \
+         : launch_pdl(k_fft_reg<T, HH, false>, r.grid, r.threads, r.smem, st, fp, tb, (V*)fbuf, m->N, m->nlat, r.lcb, r.tiles))
+    switch (m->nlon) {
+      case 64: JG_CUDA(JG_FFT_REG(32)); break;
+      case 128: JG_CUDA(JG_FFT_REG(64)); break;
+      case 256: JG_CUDA(JG_FFT_REG(128)); break;
+      case 512: JG_CUDA(JG_FFT_REG(256)); break;
+      default: JG_CUDA(JG_FFT_REG(512)); break;
+    }
+#undef JG_FFT_REG
+    mark(st);
+    JG_CUDA(cudaGetLastError());
+    return JGCM_OK;
+  }
+  if (std::is_same<T, float>::value && m->nlon >= 64 && m->nlon <= 1024 && m->tune[3] == 0) {
     const size_t smw = ((size_t)FW_COLS * (m->nlon / 2) + (size_t)(m->N + 1) * FW_COLS) * sizeof(V);
     dim3 gw((fp.C + FW_COLS - 1) / FW_COLS, m->nlat);
     bool plain = true;
