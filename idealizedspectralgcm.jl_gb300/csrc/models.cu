@@ -82,13 +82,10 @@ __device__ __forceinline__ T shfl_dn1(T x, int lane, int nd, T fill) {
 // path and to spread them over the four sub-partitions: one warp per value, lanes over partials,
 // a fixed butterfly.  The first level's units are either thread-block clusters (up to 8 blocks on
 // one GPC, folding their values through distributed shared memory at the cluster barrier) or,
-// when the grid takes more than one wave of blocks (where a cluster barrier would hold SM slots),
-// groups of CORR_GS consecutive blocks whose last block to arrive (atomic ticket) folds them.
-// Each unit publishes its values, and the last unit to arrive folds the units' values.
-constexpr int CORR_GS = 16;  // blocks per group
+// for larger grids, the few blocks per member of
+// k_hs_corr_columns.  Each unit publishes its values, and the last unit to arrive (atomic ticket)
+// folds the units' values.
 constexpr int CORR_CL = 8;   // blocks per cluster at most (the portable cluster size)
-
-__host__ __device__ inline int corr_groups(int nb) { return (nb + CORR_GS - 1) / CORR_GS; }
 
 // The fixer reduction's cluster shape over its (gx = nlon/32) x nlat grid: powers of two that
 // divide the grid, x first (the blocks of one latitude row), at most CORR_CL blocks
@@ -933,11 +930,11 @@ struct CorrArgs {
   const double* wts;
   double *partials, *scalars;  // per member: partials + e * pstride, scalars + 4 e
   T* scal_t;                   // per member: factor and correction rounded to T (for k_hs_corr_apply)
-  unsigned* counter;           // per member: corr_groups(nb) + 1 tickets
+  unsigned* counter;           // a ticket per member
   size_t pstride;
   // the column kernel's block partials (ps_p and the column energy of the previous level) at the
-  // start of the member's region, its grid (col_gx x nlat blocks); this kernel's block values at
-  // col_off (3 x nb, the group form), the first level's units' values after them (5 x the units)
+  // start of the member's region, its grid (col_gx x nlat blocks); the first level's units' values at
+  // col_off (5 x the units)
   int col_gx, col_nb;
   size_t col_off;
   int nd, nlat, nlon, do_mass, do_energy;
@@ -967,9 +964,55 @@ __device__ __forceinline__ double corr_col_share(const CorrArgs<T>& a, const dou
   return warp_sum(s);
 }
 
-// CL: the first fold level in thread-block clusters (launched with a cluster shape), else in
-// groups of CORR_GS blocks
-template <typename T, bool CL>
+// Second level, of every thread of a unit's block after its values x[0..4] (warp ks < 5, lane 0) are formed:
+// published, and the last unit to arrive folds the units' values and applies the fixes
+template <typename T>
+__device__ __forceinline__ void corr_finish(const CorrArgs<T>& a, int e, double* upart, int u, int nu, int ks, int lane,
+                                            double x) {
+  const int nd = a.nd;
+  if (ks < 5 && lane == 0) __stcg(upart + (size_t)ks * nu + u, x);  // released by ticket_last
+  if (!ticket_last(a.counter + e, (unsigned)nu)) return;
+  __shared__ double S[5];
+  for (int v = ks; v < 5; v += blockDim.x >> 5) {
+    const double t = warp_fold(upart + (size_t)v * nu, nu, lane);
+    if (lane == 0) S[v] = t;
+  }
+  __syncthreads();
+  double* scal = a.scalars + 4 * e;
+  __shared__ double s_corr;
+  // warp 0: the mass factor and spe_lnps_n(0,0) += log(factor); warp 1 (another sub-partition):
+  // the same factor and the energy correction; warp 2: the two means, off the critical path
+  if (ks == 0 && lane == 0) {
+    const double factor = a.do_mass ? S[3] / S[0] : 1.0;
+    scal[2] = factor;
+    a.scal_t[2 * e] = (T)factor;
+    if (a.do_mass) {
+      V2<T> l = a.lnps_n[e];  // spe_lnps_n[1,1,1] += log(factor)  (P_00 = 1)
+      l.x = (T)((double)l.x + log_near_one(factor));
+      a.lnps_n[e] = l;
+    }
+  } else if (ks == 1 && lane == 0) {
+    double corr = 0.0;
+    if (a.do_energy)  // one division on this warp's chain: factor S2 = S3 S2 / S0
+      corr = a.do_mass ? fma(-S[3], S[2], S[0] * (S[4] - S[1])) / ((a.cp * S[3]) * S[0])
+                       : (S[4] - S[1] - S[2]) / (a.cp * S[3]);
+    scal[3] = corr;
+    a.scal_t[2 * e + 1] = (T)corr;
+    s_corr = corr;
+  } else if (ks == 2 && lane == 0) {
+    scal[0] = S[3] * a.inv_2n;           // mean_ps_p   (Area_Weighted_Global_Mean)
+    scal[1] = S[4] * a.inv_2n / a.grav;  // mean_energy_p (Mass_Weighted_Global_Integral)
+  }
+  __syncthreads();
+  if (a.do_energy && (int)threadIdx.x < nd) {  // spe_t_n[1,1,:] .+= temperature_correction
+    V2<T> tt = a.t_spec_n[e * nd + threadIdx.x];
+    tt.x = (T)((double)tt.x + s_corr);
+    a.t_spec_n[e * nd + threadIdx.x] = tt;
+  }
+}
+
+// One block per 32 columns (small grids), the first fold level in thread-block clusters
+template <typename T>
 __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const VertCoef* __restrict__ vcp, const VertT<T>* __restrict__ vtp) {
   const VertCoef& vc = *vcp;
   // block = 32 consecutive columns of one latitude row x 8 level groups: warp ks reads levels
@@ -1067,23 +1110,12 @@ __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const Ver
   }
   // block values S0, S1, S2 (one warp each, on three sub-partitions): the level groups of each
   // column, the butterfly over the columns, the row's weight
-  const int nb = gridDim.x * gridDim.y, bid = blockIdx.y * gridDim.x + blockIdx.x, ng = corr_groups(nb);
   double* const pe = a.partials + e * a.pstride;
-  unsigned* const ctr = a.counter + (size_t)e * (ng + 1);
-  int rank = 0, nu, u;  // the first level's units (clusters or groups) and this block's unit
-  if constexpr (CL) {
-    const dim3 cd = cg::this_cluster().dim_blocks();
-    rank = (int)cg::this_cluster().block_rank();
-    const int gcx = gridDim.x / cd.x;
-    nu = gcx * (gridDim.y / cd.y);
-    u = (blockIdx.y / cd.y) * gcx + blockIdx.x / cd.x;
-  } else {
-    nu = ng;
-    u = bid / CORR_GS;
-  }
-  double* const bpart = pe + a.col_off;           // [3][nb] (groups)
-  double* const upart = bpart + (size_t)3 * nb;  // [5][nu]
-  __shared__ double s_bv[3];                      // this block's values (clusters)
+  cg::cluster_group cl = cg::this_cluster();
+  const dim3 cd = cl.dim_blocks();
+  const int rank = (int)cl.block_rank(), gcx = gridDim.x / cd.x;
+  const int nu = gcx * (gridDim.y / cd.y), u = (blockIdx.y / cd.y) * gcx + blockIdx.x / cd.x;  // this block's unit
+  __shared__ double s_bv[3];  // this block's values
   double x = 0.0;
   if (ks < 3) {
     const T ps = act ? a.ps_n[off1 + col] : (T)0;
@@ -1113,77 +1145,160 @@ __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const Ver
       x = warp_sum(x);
     }
     x *= a.wts[j];
-    if (lane == 0) {
-      if constexpr (CL)
-        s_bv[ks] = x;
-      else
-        __stcg(bpart + (size_t)ks * nb + bid, x);  // released by ticket_last
-    }
-  } else if (CL && ks < 5 && rank == 0) {
+    if (lane == 0) s_bv[ks] = x;
+  } else if (ks < 5 && rank == 0) {
     x = corr_col_share(a, pe, ks - 3, u, nu, lane);  // the leader's share, while the others finish
   }
-  // first level
-  if constexpr (CL) {
-    // every thread of every block of the cluster reaches both cluster barriers (no return before
-    // them): the first releases the blocks' values to the leader, the second keeps the blocks
-    // resident until the leader has read them
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
-    if (rank == 0 && ks < 3) {  // the cluster's blocks in rank order, the fixed butterfly
-      const double v = lane < (int)cl.num_blocks() ? *cl.map_shared_rank(&s_bv[ks], lane) : 0.0;
-      x = warp_sum(v);
-    }
-    cl.sync();
-    if (rank != 0) return;
-  } else {
-    // the group's last block folds the group's block values and its share of the column kernel's
-    const int g0 = u * CORR_GS, gn = min(CORR_GS, nb - g0);
-    if (!ticket_last(ctr + u, (unsigned)gn)) return;
-    if (ks < 3)
-      x = warp_fold(bpart + (size_t)ks * nb + g0, gn, lane);
-    else if (ks < 5)
-      x = corr_col_share(a, pe, ks - 3, u, nu, lane);
+  // first level: every thread of every block of the cluster reaches both cluster barriers (no return
+  // before them): the first releases the blocks' values to the leader, the second keeps the blocks
+  // resident until the leader has read them
+  cl.sync();
+  if (rank == 0 && ks < 3) {  // the cluster's blocks in rank order, the fixed butterfly
+    const double v = lane < (int)cl.num_blocks() ? *cl.map_shared_rank(&s_bv[ks], lane) : 0.0;
+    x = warp_sum(v);
   }
-  if (ks < 5 && lane == 0) __stcg(upart + (size_t)ks * nu + u, x);  // released by ticket_last
-  // second level: the last unit to arrive folds the units' values and applies the fixes
-  if (!ticket_last(ctr + ng, (unsigned)nu)) return;
-  __shared__ double S[5];
-  if (ks < 5) {
-    const double x = warp_fold(upart + (size_t)ks * nu, nu, lane);
-    if (lane == 0) S[ks] = x;
+  cl.sync();
+  if (rank != 0) return;
+  corr_finish<T>(a, e, pe + a.col_off, u, nu, ks, lane, x);
+}
+
+// (h + l) times the pair (wh, wl), added to the pair (sh, sl): the leading product error-free, the cross
+// terms rounded
+__device__ __forceinline__ void ds_add_mul(float& sh, float& sl, float h, float l, float wh, float wl) {
+  const float p = __fmul_rn(h, wh), pe = __fmaf_rn(h, wh, -p);
+  ds_add(sh, sl, p);
+  sl = __fadd_rn(sl, __fadd_rn(pe, __fmaf_rn(h, wl, __fmul_rn(l, wh))));
+}
+
+// The same sums for larger grids (member ensembles): a warp takes 32 consecutive columns of a
+// latitude row at a time, a thread one column with all its levels, and keeps the three sums to the end of
+// its columns, so the folds, the barriers and the ticket come once per block.  One block per 32 columns and
+// 8 level groups spent 420 instructions and three barriers per warp on 2.5 levels (128 x T21L20 and 32 x T42L20
+// 58 us for 63 MB; 29 and 31 here, 4 levels' loads in flight 40 and 42).  As there: the kinetic part in the state precision over five levels at
+// a time, c_p T and every sum beyond as FP32 pairs (FP64 on the FP64 path).
+constexpr int CORR_WARPS = 8;
+template <typename T>
+__global__ void __launch_bounds__(32 * CORR_WARPS) k_hs_corr_columns(CorrArgs<T> a, const VertCoef* __restrict__ vcp,
+                                                                     const VertT<T>* __restrict__ vtp) {
+  const VertCoef& vc = *vcp;
+  constexpr bool F = std::is_same<T, float>::value;
+  __shared__ T s_dak[JGCM_MAX_ND], s_dbk[JGCM_MAX_ND];
+  __shared__ double s_dak64[F ? 1 : JGCM_MAX_ND], s_dbk64[F ? 1 : JGCM_MAX_ND];
+  __shared__ float s_dah[JGCM_MAX_ND], s_dal[JGCM_MAX_ND], s_dbh[JGCM_MAX_ND], s_dbl[JGCM_MAX_ND];
+  for (int q = threadIdx.x; q < a.nd; q += blockDim.x) {
+    s_dak[q] = vtp->dak[q];
+    s_dbk[q] = vtp->dbk[q];
+    if constexpr (F) {
+      s_dah[q] = vc.dak_hi[q];
+      s_dal[q] = vc.dak_lo[q];
+      s_dbh[q] = vc.dbk_hi[q];
+      s_dbl[q] = vc.dbk_lo[q];
+    } else {
+      s_dak64[q] = vc.dak[q];
+      s_dbk64[q] = vc.dbk[q];
+    }
   }
   __syncthreads();
-  double* scal = a.scalars + 4 * e;
-  __shared__ double s_corr;
-  // warp 0: the mass factor and spe_lnps_n(0,0) += log(factor); warp 1 (another sub-partition):
-  // the same factor and the energy correction; warp 2: the two means, off the critical path
-  if (ks == 0 && lane == 0) {
-    const double factor = a.do_mass ? S[3] / S[0] : 1.0;
-    scal[2] = factor;
-    a.scal_t[2 * e] = (T)factor;
-    if (a.do_mass) {
-      V2<T> l = a.lnps_n[e];  // spe_lnps_n[1,1,1] += log(factor)  (P_00 = 1)
-      l.x = (T)((double)l.x + log_near_one(factor));
-      a.lnps_n[e] = l;
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  const int lane = threadIdx.x & 31, ks = threadIdx.x >> 5, nd = a.nd, e = blockIdx.y;
+  const int gx = (a.nlon + 31) / 32, units = gx * a.nlat, nu = gridDim.x, u = blockIdx.x;
+  const size_t G = (size_t)a.nlat * a.nlon, offL = (size_t)e * nd * G, off1 = (size_t)e * G;
+  double* const pe = a.partials + e * a.pstride;
+  float sh[3] = {0, 0, 0}, sl[3] = {0, 0, 0};
+  double sd[3] = {0, 0, 0};
+  constexpr int KB = F ? 10 : 5;  // levels whose loads are issued together
+  for (int q = u * CORR_WARPS + ks; q < units; q += nu * CORR_WARPS) {
+    const int j = q / gx, i = (q - j * gx) * 32 + lane;
+    if (i >= a.nlon) continue;  // no warp operation in the loop
+    const size_t col = (size_t)j * a.nlon + i;
+    const T ps = a.ps_n[off1 + col];
+    const double w = a.wts[j];
+    float kah = 0, kal = 0, kbh = 0, kbl = 0, tah = 0, tal = 0, tbh = 0, tbl = 0;  // Σ K Δa, K Δb, T Δa, T Δb
+    T ka = 0, kb = 0;
+    double ta = 0, tb = 0;
+    for (int k0 = 0; k0 < nd; k0 += KB) {
+      T uu[KB], vv[KB], tt[KB];
+#pragma unroll
+      for (int c = 0; c < KB; c++) {
+        uu[c] = vv[c] = tt[c] = 0;
+        if (k0 + c < nd) {
+          const size_t x = offL + (size_t)(k0 + c) * G + col;
+          uu[c] = a.u_n[x];
+          vv[c] = a.v_n[x];
+          tt[c] = a.t_n[x];
+        }
+      }
+      T ca = 0, cb = 0;
+#pragma unroll
+      for (int c = 0; c < KB; c++) {
+        if (k0 + c >= nd) break;
+        const int k = k0 + c;
+        if (c == KB / 2) {  // the kinetic part: at most five levels in the state precision
+          if constexpr (F) {
+            ds_add(kbh, kbl, cb);
+            if (a.has_dak) ds_add(kah, kal, ca);
+            ca = cb = 0;
+          }
+        }
+        const T K = (T)0.5 * (uu[c] * uu[c] + vv[c] * vv[c]);
+        cb += K * s_dbk[k];
+        if (a.has_dak) ca += K * s_dak[k];
+        if constexpr (F) {
+          ds_add_prod(tbh, tbl, tt[c], s_dbh[k], s_dbl[k]);
+          if (a.has_dak) ds_add_prod(tah, tal, tt[c], s_dah[k], s_dal[k]);
+        } else {
+          tb += tt[c] * s_dbk64[k];
+          if (a.has_dak) ta += tt[c] * s_dak64[k];
+        }
+      }
+      if constexpr (F) {
+        ds_add(kbh, kbl, cb);
+        if (a.has_dak) ds_add(kah, kal, ca);
+      } else {
+        kb += cb;
+        ka += ca;
+      }
     }
-  } else if (ks == 1 && lane == 0) {
-    double corr = 0.0;
-    if (a.do_energy)  // one division on this warp's chain: factor S2 = S3 S2 / S0
-      corr = a.do_mass ? fma(-S[3], S[2], S[0] * (S[4] - S[1])) / ((a.cp * S[3]) * S[0])
-                       : (S[4] - S[1] - S[2]) / (a.cp * S[3]);
-    scal[3] = corr;
-    a.scal_t[2 * e + 1] = (T)corr;
-    s_corr = corr;
-  } else if (ks == 2 && lane == 0) {
-    scal[0] = S[3] * a.inv_2n;           // mean_ps_p   (Area_Weighted_Global_Mean)
-    scal[1] = S[4] * a.inv_2n / a.grav;  // mean_energy_p (Mass_Weighted_Global_Integral)
+    if constexpr (F) {
+      const float wh = (float)w, wl = (float)(w - (double)wh);
+      ds_add_mul(kbh, kbl, tbh, tbl, a.cp_hi, a.cp_lo);  // E = K + c_p T
+      const float p = __fmul_rn(kbh, ps), pl = __fadd_rn(__fmaf_rn(kbh, ps, -p), __fmul_rn(kbl, ps));
+      ds_add_mul(sh[0], sl[0], ps, 0.f, wh, wl);
+      ds_add_mul(sh[2], sl[2], p, pl, wh, wl);
+      if (a.has_dak) {
+        ds_add_mul(kah, kal, tah, tal, a.cp_hi, a.cp_lo);
+        ds_add_mul(sh[1], sl[1], kah, kal, wh, wl);
+      }
+    } else {
+      sd[0] += ps * w;
+      sd[1] += (ka + a.cp * ta) * w;
+      sd[2] += (kb + a.cp * tb) * ps * w;
+    }
+  }
+  // the block's values: the butterfly over a warp's columns, then the warps in order
+  __shared__ double s_w[3][CORR_WARPS];
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    if constexpr (F) {
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) {
+        const float h2 = __shfl_xor_sync(FULL, sh[v], o), l2 = __shfl_xor_sync(FULL, sl[v], o);
+        ds_add(sh[v], sl[v], h2);
+        sl[v] = __fadd_rn(sl[v], l2);
+      }
+      sd[v] = (double)sh[v] + (double)sl[v];
+    } else {
+      sd[v] = warp_sum(sd[v]);
+    }
+    if (lane == 0) s_w[v][ks] = sd[v];
   }
   __syncthreads();
-  if (a.do_energy && (int)threadIdx.x < nd) {  // spe_t_n[1,1,:] .+= temperature_correction
-    V2<T> tt = a.t_spec_n[e * nd + threadIdx.x];
-    tt.x = (T)((double)tt.x + s_corr);
-    a.t_spec_n[e * nd + threadIdx.x] = tt;
-  }
+  double x = 0.0;
+  if (ks < 3)
+    for (int q = 0; q < CORR_WARPS; q++) x += s_w[ks][q];
+  else if (ks < 5)
+    x = corr_col_share(a, pe, ks - 3, u, nu, lane);
+  corr_finish<T>(a, e, pe + a.col_off, u, nu, ks, lane, x);
 }
 
 template <typename T>
@@ -1610,10 +1725,8 @@ int build_wave(jgcm_model* md) {
 size_t col_partials(const jgcm_mesh* m) { return (size_t)2 * ((m->nlon + HS_CT / 8 - 1) / (HS_CT / 8)) * m->nlat; }
 size_t partial_stride(const jgcm_mesh* m) {
   const int nb = ((m->nlon + 31) / 32) * m->nlat;  // the fixer reduction's blocks per member
-  return col_partials(m) + (size_t)3 * nb + (size_t)5 * nb;  // its block values, its units' (<= nb)
+  return col_partials(m) + (size_t)5 * nb;  // its units' values (<= nb units)
 }
-// the fixer reduction's tickets per member
-inline size_t corr_tickets(const jgcm_mesh* m) { return (size_t)corr_groups(((m->nlon + 31) / 32) * m->nlat) + 1; }
 
 int model_alloc(jgcm_model* md) {
   jgcm_mesh* m = md->mesh;
@@ -1657,7 +1770,7 @@ int model_alloc(jgcm_model* md) {
   JG_TRY(alloc((void**)&md->d_partials, (size_t)ne * partial_stride(m) * 8));
   // 4 FP64 scalars per member, then each member's factor and correction in the state precision
   JG_TRY(alloc((void**)&md->d_scalars, (size_t)6 * ne * 8));
-  JG_TRY(alloc((void**)&md->d_counter, (size_t)ne * corr_tickets(m) * sizeof(unsigned)));
+  JG_TRY(alloc((void**)&md->d_counter, (size_t)ne * sizeof(unsigned)));
   int nt = (N + 1) * (ns + 1);
   JG_TRY(alloc(&md->dfac[0], (size_t)nt * ts));
   JG_TRY(alloc(&md->dfac[1], (size_t)nt * ts));
@@ -2203,15 +2316,19 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
   ca.cp_lo = (float)(md->cp_air - (double)ca.cp_hi);
   ca.has_dak = has_dak(md);
   {
-    // clusters when the grid is one wave of blocks (8 of these per SM), groups otherwise
-    const int gx = (m->nlon + 31) / 32;
-    if ((size_t)gx * m->nlat * E <= (size_t)8 * m->sm_count) {
+    // one block per 32 columns while that is less than three blocks per SM (the shortest chain: T42L20, one
+    // member, FP64 12.3 us against 20.5; FP32 the same 12.4), else a few blocks per member (4 members 16.5 ->
+    // 12.4 us, one member of T63 14.2 -> 12.2)
+    const int gx = (m->nlon + 31) / 32, units = gx * m->nlat;
+    if ((size_t)units * E <= (size_t)3 * m->sm_count) {
       int cx, cy;
       corr_cluster(gx, m->nlat, cx, cy);
-      JG_CUDA(launch_pdl_cluster(k_hs_corr_reduce<T, true>, dim3(gx, m->nlat, E), 256, 0, st, dim3(cx, cy, 1), ca,
+      JG_CUDA(launch_pdl_cluster(k_hs_corr_reduce<T>, dim3(gx, m->nlat, E), 256, 0, st, dim3(cx, cy, 1), ca,
                                  md->d_vc, (const VertT<T>*)md->d_vt));
     } else {
-      JG_CUDA(launch_pdl(k_hs_corr_reduce<T, false>, dim3(gx, m->nlat, E), 256, 0, st, ca, md->d_vc,
+      // about four blocks of 8 warps per SM, each warp with at least one unit of 32 columns
+      const int nb = std::max(1, std::min((units + CORR_WARPS - 1) / CORR_WARPS, (4 * m->sm_count + E - 1) / E));
+      JG_CUDA(launch_pdl(k_hs_corr_columns<T>, dim3(nb, E), 32 * CORR_WARPS, 0, st, ca, md->d_vc,
                          (const VertT<T>*)md->d_vt));
     }
   }
