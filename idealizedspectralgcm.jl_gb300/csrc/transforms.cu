@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) k_s2g_legendre(S2GPlan plan, Tables<T> tb
     if (c < C) {
       int k;
       const S2GGroup& g = group_of(plan.g, plan.ng, c, &k);
-      for (int r = threadIdx.x / CT; r < K; r += rstep) X[r * CT + cl0] = s2g_input<T>(g, tb, m, m + r, ns, mrow, k);
+      s2g_column<T>(g, tb, m, ns, mrow, k, X + cl0, CT, threadIdx.x / CT, rstep, K);
     } else {
       for (int r = threadIdx.x / CT; r < K; r += rstep) X[r * CT + cl0] = V{0, 0};
     }
@@ -201,6 +201,66 @@ __global__ void __launch_bounds__(256) k_s2g_legendre(S2GPlan plan, Tables<T> tb
       F[((size_t)m * nlat + j) * C + c] = s;
       F[((size_t)m * nlat + (nlat - 1 - j)) * C + c] = nn;
     }
+  }
+}
+
+// The same synthesis for launches of many columns, FP32: a warp takes LT latitudes, a lane one of the block's
+// 32 columns at all of them.  Per row n the lane reads its input (coalesced) and the LT weights (broadcast) for
+// 2 LT multiply-adds, where a tile of 8 columns with an output per thread read two words for two and built its
+// inputs, staged the weights and looked up its groups for 8 columns at a time (T42L20, 32 members: 107 M
+// instructions for 9 M multiply-adds, 103 us; 40 us here; 128 x T21L20 87 -> 35 us).  Two columns per lane
+// measured 41 and 38 us.  Same products in the same order per output.  grid (column tiles, N + 1), 32 nh / LT
+// threads.
+template <int LT>
+__global__ void __launch_bounds__(512) k_s2g_tiles(const __grid_constant__ S2GPlan plan, Tables<float> tb,
+                                                   float2* __restrict__ F, int ns, int nlat) {
+  constexpr int CT = 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int m = blockIdx.y, nh = nlat >> 1, K = ns + 1 - m, C = plan.C;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * CT + lane;
+  const size_t mrow = (size_t)m * (ns + 1);
+  float* Ps = (float*)smem;                                                     // [K][nh]
+  float2* X = (float2*)(smem + align16((size_t)(ns + 1) * nh * sizeof(float)));  // [K][CT]
+  const float* Pm = tb.P + (mrow + m) * nh;
+  for (int i = threadIdx.x; i < K * nh / 4; i += blockDim.x) cp_async16(Ps + i * 4, Pm + i * 4);
+  cp_async_commit();
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  if (c < C) {
+    int k;
+    const S2GGroup& g = group_of(plan.g, plan.ng, c, &k);
+    s2g_column<float>(g, tb, m, ns, mrow, k, X + lane, CT, warp, blockDim.x >> 5, K);
+  }  // (a lane past the last column reads its own unset inputs and stores nothing)
+  cp_async_wait_all();
+  __syncthreads();
+  const int j0 = warp * LT;
+  float er[LT], ei[LT], qr[LT], qi[LT];  // even and odd sums
+#pragma unroll
+  for (int l = 0; l < LT; l++) er[l] = ei[l] = qr[l] = qi[l] = 0;
+  auto row = [&](int r, float(&sr)[LT], float(&si)[LT]) {
+    const float2 x = X[r * CT + lane];
+#pragma unroll
+    for (int l = 0; l < LT; l += 4) {
+      float p[4];
+      ld4(Ps + r * nh + j0 + l, p);
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        sr[l + v] += p[v] * x.x;
+        si[l + v] += p[v] * x.y;
+      }
+    }
+  };
+  int r = 0;
+  for (; r + 1 < K; r += 2) {
+    row(r, er, ei);
+    row(r + 1, qr, qi);
+  }
+  if (r < K) row(r, er, ei);
+  if (c >= C) return;
+#pragma unroll
+  for (int l = 0; l < LT; l++) {
+    const int j = j0 + l;
+    F[((size_t)m * nlat + j) * C + c] = make_float2(er[l] + qr[l], ei[l] + qi[l]);
+    F[((size_t)m * nlat + (nlat - 1 - j)) * C + c] = make_float2(er[l] - qr[l], ei[l] - qi[l]);
   }
 }
 
@@ -1132,6 +1192,8 @@ static int configure_smem() {
     JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     if (idx == 0) {
+      JG_CUDA(cudaFuncSetAttribute(k_s2g_tiles<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+      JG_CUDA(cudaFuncSetAttribute(k_s2g_tiles<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
       JG_CUDA(cudaFuncSetAttribute(k_fft_rows<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
       JG_CUDA(cudaFuncSetAttribute(k_fft_rows<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
       JG_CUDA(cudaFuncSetAttribute(k_fft_rows<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -1261,6 +1323,21 @@ static RegFFT reg_fft_shape(const jgcm_mesh* m, int C) {
 template <typename T>
 static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip, cudaStream_t st, V2<T>* fbuf);
 
+// Latitudes per thread of the tiled synthesis (k_s2g_tiles) for a launch of C columns, 0 = k_s2g_legendre
+// (FP64, a tuned tile, shapes that do not fit).  From two of its blocks per SM on (T42L20, 2 members 13.2 ->
+// 11.9 us, T63L20, one member 16.4 -> 14.4, T21L20, 8 members 12.7 -> 10.7; one member of T42L20 10.7 -> 12.0), 8
+// latitudes instead of 4 from eight blocks per SM on (4 members 16.1 us against 12.6, 32 members 40 against 43).
+template <typename T>
+static int s2g_tile_lats(const jgcm_mesh* m, int C) {
+  if (!std::is_same<T, float>::value || m->tune[1] != 0) return 0;
+  if (align16((size_t)(m->ns + 1) * m->nh * sizeof(float)) + (size_t)(m->ns + 1) * 32 * sizeof(float2) > kSmemBudget) return 0;
+  const size_t blocks = (size_t)((C + 31) / 32) * (m->N + 1);
+  if (blocks < (size_t)2 * m->sm_count) return 0;
+  auto fits = [&](int lt) { return m->nh % lt == 0 && 32 * m->nh / lt <= 512; };
+  if (blocks >= (size_t)8 * m->sm_count && fits(8)) return 8;
+  return fits(4) ? 4 : fits(8) ? 8 : 0;
+}
+
 // Legendre synthesis then inverse FFT, with the Fourier coefficients staged in `fbuf`
 // ((N+1) x nlat x C complex T).
 template <typename T>
@@ -1272,6 +1349,14 @@ static int launch_s2g_into(jgcm_mesh* m, const S2GPlan& sp0, const IFFTPlan& ip,
   const int nh = m->nh, ct = m->tune[1] ? s2g_ct(m) : fit_ct(s2g_ct(m), sp.C);
   if (std::is_same<T, float>::value && m->tc.on && !m->simt_legendre) {
     JG_TRY(launch_s2g_legendre_tc(m, sp, fbuf, st));
+  } else if (const int lt = s2g_tile_lats<T>(m, sp.C)) {
+    const size_t smt = align16((size_t)(m->ns + 1) * nh * sizeof(float)) + (size_t)(m->ns + 1) * 32 * sizeof(float2);
+    const dim3 gt((sp.C + 31) / 32, m->N + 1);
+    const Tables<float> tf = tables<float>(m);
+    if (lt == 8) JG_CUDA(launch_pdl(k_s2g_tiles<8>, gt, 32 * nh / 8, smt, st, sp, tf, (float2*)fbuf, m->ns, m->nlat));
+    else JG_CUDA(launch_pdl(k_s2g_tiles<4>, gt, 32 * nh / 4, smt, st, sp, tf, (float2*)fbuf, m->ns, m->nlat));
+    mark(st);
+    JG_CUDA(cudaGetLastError());
   } else {
     size_t sm1 = align16((size_t)(m->ns + 1) * nh * sizeof(T)) + (size_t)(m->ns + 1) * ct * sizeof(V);
     dim3 g1((sp.C + ct - 1) / ct, m->N + 1);

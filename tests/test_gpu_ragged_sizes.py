@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 CASES = [(5, 10, 16, 1), (7, 12, 16, 3), (21, 36, 64, 5), (31, 48, 128, 13), (42, 64, 128, 1), (63, 96, 256, 7),
          (85, 128, 256, 1), (106, 160, 512, 2)]
 # enough rows for the register-split FFTs at every length, column counts that leave a ragged last tile
-MANY = [(31, 48, 64, 61), (42, 64, 128, 41), (63, 96, 256, 27), (106, 160, 512, 9), (170, 256, 1024, 5)]
+MANY = [(31, 48, 64, 61), (42, 64, 128, 41), (63, 96, 256, 27), (106, 160, 512, 9), (170, 256, 1024, 5),
+        (85, 128, 256, 61)]  # the last: the tiled synthesis, too
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
