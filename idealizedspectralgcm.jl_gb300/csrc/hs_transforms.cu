@@ -61,23 +61,20 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
   // field read neighbouring words
   V* X = (V*)(smem + ((wsz * sizeof(T) + 15) & ~(size_t)15));
   // 1. the weight rows n = m..ns of both m (constants): asynchronous 16-byte copies, issued before
-  //    the dependency wait and waited for once.  A row is nh * sizeof(T) / 16 chunks (a power of
-  //    two): a warp pass copies 32 / chunks rows, or one row in passes of 32 chunks.
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  //    the dependency wait and waited for once
   {
     constexpr int ce = 16 / (int)sizeof(T);  // weights per chunk
-    const int nchunk = nh / ce, rpi = nchunk >= 32 ? 1 : 32 / nchunk;
-    const int rsub = nchunk >= 32 ? 0 : lane / nchunk, c0 = nchunk >= 32 ? lane : lane - rsub * nchunk;
+    const int nchunk = nh / ce;
     for (int s = 0; s < nm; s++) {
       const int m = s ? m2 : m1, K = s ? K2 : K1;
       const size_t src = ((size_t)m * (ns + 1) + m) * nh;
       T* dst = W + (s ? (size_t)3 * K1 * wp : 0);
-#pragma unroll
-      for (int tbl = 0; tbl < 3; tbl++) {
-        const T* from = (tbl == 0 ? tb.PW : tbl == 1 ? tb.CA : tb.CB) + src;
-        T* to = dst + (size_t)tbl * K * wp;
-        for (int r = warp * rpi + rsub; r < K; r += nw * rpi)
-          for (int c = c0; c < nchunk; c += 32) cp_async16(to + (size_t)r * wp + c * ce, from + (size_t)r * nh + c * ce);
+      for (int i = threadIdx.x; i < K * nchunk; i += blockDim.x) {
+        const int r = i / nchunk, c = i - r * nchunk;
+        const size_t to = (size_t)r * wp + c * ce, from = src + (size_t)i * ce;
+        cp_async16(dst + to, tb.PW + from);
+        cp_async16(dst + (size_t)K * wp + to, tb.CA + from);
+        cp_async16(dst + (size_t)2 * K * wp + to, tb.CB + from);
       }
     }
     cp_async_commit();
@@ -260,6 +257,161 @@ size_t hs_analysis_smem(const jgcm_mesh* m, int LG) {
 
 PerDeviceOnce g_hs_ana_smem[2];
 
+// The same analysis for launches of many columns, FP32: a block takes 32 consecutive columns (levels of
+// all members in a row) of one m, a warp four rows n of one parity (n = m + 8 i + p + 2 u, u < 4), a lane one
+// column.  Per latitude pair the lane reads its eight inputs (coalesced), folds them, and with the warp's 12
+// weights (three broadcast loads) makes 48 multiply-adds; with two rows per thread and a weight row per load
+// the shared-memory pipe was the bound (T42L20, 32 members: 68 % of its wavefronts at 22 % of the warps, 37 M
+// instructions for 7.6 M multiply-adds, 70 us; 128 x T21L20 60 us).  The Fourier rows stream through a
+// ring of AT_STAGES x AT_JC latitude pairs by asynchronous copies, and the weights are laid out for it once
+// per mesh ([m][latitude][row group][table][u], hs_tables_build): 40 and 29 us; staged and folded in step,
+// with a transposition of the weights per block, 50 and 41.  The columns of
+// δ ln ps (one per member) are tiles of their own behind the levels', with the δT slot alone.  Same sums in
+// the same order.  grid (level tiles + δ ln ps tiles, N + 1), 32 at_groups(ns + 1) threads.
+constexpr int AT_ROWS = 4, AT_JC = 8, AT_STAGES = 3;
+__host__ __device__ constexpr int at_groups(int K) { return 2 * ((K + 2 * AT_ROWS - 1) / (2 * AT_ROWS)); }
+__host__ __device__ constexpr int at_pitch(int ns) { return at_groups(ns + 1) * 3 * AT_ROWS; }  // floats per latitude
+
+__global__ void k_at_weights(Tables<float> tb, float* __restrict__ out, int N, int ns, int nh) {
+  const int wp = at_pitch(ns);
+  const size_t total = (size_t)(N + 1) * nh * wp;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    const int q = (int)(t % wp), jh = (int)(t / wp % nh), m = (int)(t / wp / nh);
+    const int g = q / (3 * AT_ROWS), tbl = q / AT_ROWS % 3, u = q % AT_ROWS, n = m + 8 * (g >> 1) + (g & 1) + 2 * u;
+    const float* from = tbl == 0 ? tb.PW : tbl == 1 ? tb.CA : tb.CB;
+    out[t] = n <= ns ? from[((size_t)m * (ns + 1) + n) * nh + jh] : 0.f;
+  }
+}
+
+// 8-byte asynchronous copy, or zeros when !live (the source address is valid either way)
+__device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc, bool live) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gsrc), "r"(live ? 8 : 0) : "memory");
+}
+
+template <int NT, int NB>
+__global__ void __launch_bounds__(NT, NB) k_hs_analysis_tiles(HSAnaArgs<float> a, Tables<float> tb,
+                                                              const float* __restrict__ wt) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int ns = a.ns, nh = a.nh, nlat = a.nlat, m = blockIdx.y, K = ns + 1 - m, G = at_groups(K), wp = at_pitch(ns);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nt = (a.L + 31) / 32;
+  const bool isp = (int)blockIdx.x >= nt;  // a tile of δ ln ps columns
+  const int col = ((int)blockIdx.x - (isp ? nt : 0)) * 32 + lane;
+  const bool live = col < (isp ? a.E : a.L);
+  float* W = (float*)smem;                                         // [nh][wp]
+  float2* X = (float2*)(smem + (size_t)nh * wp * sizeof(float));  // [stage][latitude][field][south, north][32]
+  const size_t mrow = (size_t)m * (ns + 1);
+  {
+    const float* src = wt + (size_t)m * nh * wp;
+    const int nc = G * 3;  // 16-byte chunks of a latitude's weights in use
+    for (int i = threadIdx.x; i < nh * nc; i += blockDim.x) {
+      const int jh = i / nc, c = i - jh * nc;
+      cp_async16(W + (size_t)jh * wp + c * 4, src + (size_t)jh * wp + c * 4);
+    }
+  }
+  pdl_wait();  // programmatic dependent launch: the forward FFT's coefficients are complete
+  constexpr int SZ = AT_JC * 8 * 32;  // pairs per stage
+  // the fields' columns follow one another (U, V, T, E, L apart); a δ ln ps tile has the third slot alone
+  const unsigned C = a.Cin, fs = isp ? 0u : (unsigned)a.L;
+  const unsigned o0 = (unsigned)m * nlat * C + (live ? (isp ? a.colP : a.colU) + col : 0);
+  auto fetch = [&](int j0, int stage) {
+    float2* dst = X + stage * SZ + warp * 32 + lane;
+    for (int q = warp; q < 8 * AT_JC; q += nw, dst += nw * 32) {
+      const unsigned f = q >> 1 & 3, jh = j0 + (q >> 3), j = q & 1 ? nlat - 1 - jh : jh;
+      const bool on = live && (!isp || f == 2);
+      cp_async8(dst, a.F + (o0 + j * C + (on ? f * fs : 0u)), on);
+    }
+  };
+  const int nchunk = nh / AT_JC;
+#pragma unroll
+  for (int s = 0; s < AT_STAGES - 1; s++) {
+    if (s < nchunk) fetch(s * AT_JC, s);
+    cp_async_commit();  // (the first group holds the weights, too)
+  }
+  float var[AT_ROWS], vai[AT_ROWS], vbr[AT_ROWS], vbi[AT_ROWS], dar[AT_ROWS], dai[AT_ROWS], dbr[AT_ROWS], dbi[AT_ROWS],
+      er[AT_ROWS], ei[AT_ROWS], tr[AT_ROWS], ti[AT_ROWS];
+#pragma unroll
+  for (int u = 0; u < AT_ROWS; u++)
+    var[u] = vai[u] = vbr[u] = vbi[u] = dar[u] = dai[u] = dbr[u] = dbi[u] = er[u] = ei[u] = tr[u] = ti[u] = 0;
+  // the hemisphere fold of a row's parity is south + sg north, the other parity's south - sg north (P_n^m is
+  // symmetric about the equator for n - m even)
+  const float sg = warp & 1 ? -1.f : 1.f;
+  for (int c = 0; c < nchunk; c++) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(AT_STAGES - 2) : "memory");
+    __syncthreads();  // chunk c is staged, and every warp has read chunk c - 1
+    if (c + AT_STAGES - 1 < nchunk) fetch((c + AT_STAGES - 1) * AT_JC, (c + AT_STAGES - 1) % AT_STAGES);
+    cp_async_commit();
+    if (warp < G) {
+      const float* w = W + (size_t)c * AT_JC * wp + warp * 3 * AT_ROWS;
+      const float2* x = X + (c % AT_STAGES) * SZ + lane;
+#pragma unroll 2
+      for (int jj = 0; jj < AT_JC; jj++) {
+        float wP[4], wA[4], wB[4];
+        ld4(w, wP);
+        ld4(w + AT_ROWS, wA);
+        ld4(w + 2 * AT_ROWS, wB);
+        const float2 us = x[0], un = x[32], vs = x[64], vn = x[96], ts = x[128], tn = x[160], es = x[192], en = x[224];
+        const float xux = fmaf(sg, un.x, us.x), xuy = fmaf(sg, un.y, us.y), yux = fmaf(-sg, un.x, us.x),
+                    yuy = fmaf(-sg, un.y, us.y), xvx = fmaf(sg, vn.x, vs.x), xvy = fmaf(sg, vn.y, vs.y),
+                    yvx = fmaf(-sg, vn.x, vs.x), yvy = fmaf(-sg, vn.y, vs.y), xex = fmaf(sg, en.x, es.x),
+                    xey = fmaf(sg, en.y, es.y), xtx = fmaf(sg, tn.x, ts.x), xty = fmaf(sg, tn.y, ts.y);
+#pragma unroll
+        for (int u = 0; u < AT_ROWS; u++) {
+          var[u] += (-xvy) * wA[u];
+          vai[u] += xvx * wA[u];
+          vbr[u] += yux * wB[u];
+          vbi[u] += yuy * wB[u];
+          dar[u] += (-xuy) * wA[u];
+          dai[u] += xux * wA[u];
+          dbr[u] += yvx * wB[u];
+          dbi[u] += yvy * wB[u];
+          er[u] += xex * wP[u];
+          ei[u] += xey * wP[u];
+          tr[u] += xtx * wP[u];
+          ti[u] += xty * wP[u];
+        }
+        w += wp;
+        x += 8 * 32;
+      }
+    }
+  }
+  if (warp >= G || !live) return;
+#pragma unroll
+  for (int u = 0; u < AT_ROWS; u++) {
+    const int r = 8 * (warp >> 1) + (warp & 1) + 2 * u, n = m + r;
+    if (r >= K) continue;
+    const bool last = n == ns;  // row N+1 of the analysis is zero (Trans_Grid_To_Spherical!, :288-291)
+    const float2 ot = last ? make_float2(0.f, 0.f) : make_float2(tr[u] * 0.5f, ti[u] * 0.5f);
+    if (isp) {
+      a.dlnps[(mrow + n) * a.E + col] = ot;
+      continue;
+    }
+    float2 ov = make_float2(0.f, 0.f), od = ov;
+    if (!last) {
+      const float eig = tb.eig[mrow + n];
+      ov.x = var[u] + -1.f * vbr[u];
+      ov.y = vai[u] + -1.f * vbi[u];
+      od.x = dar[u] + dbr[u];
+      od.y = dai[u] + dbi[u];
+      od.x = od.x - eig * (er[u] * 0.5f);
+      od.y = od.y - eig * (ei[u] * 0.5f);
+    }
+    const size_t sidx = (mrow + n) * a.L + col;
+    a.dvor[sidx] = ov;
+    a.ddiv[sidx] = od;
+    a.dt[sidx] = ot;
+  }
+}
+
+size_t at_smem(const jgcm_mesh* m) {
+  return (size_t)m->nh * at_pitch(m->ns) * sizeof(float) + (size_t)AT_STAGES * AT_JC * 8 * 32 * sizeof(float2);
+}
+// whether the tiled kernel serves this mesh
+bool at_fits(const jgcm_mesh* m) {
+  return m->nh % AT_JC == 0 && 32 * at_groups(m->ns + 1) <= 640 && at_smem(m) <= kSmemBudget;
+}
+
 }  // namespace
 
 // total wavenumbers per thread: two of one parity for member ensembles (each folded input loaded
@@ -290,13 +442,29 @@ int hs_analysis_levels(const jgcm_mesh* m, int nd, int E) {
   return lg_max;
 }
 
+// The tiled kernel serves an FP32 launch of E members: from five blocks per four SMs on (T42L20, 4 members
+// 15.5 -> 16.5 us, 8 members 23 -> 19, 16 members 38 -> 25, 4 members of T63L20 29.6 -> 27.4, one 14 -> 22)
+static int at_tiles(int nd, int E) { return (nd * E + 31) / 32 + (E + 31) / 32; }
+static bool at_pays(const jgcm_mesh* m, int nd, int E) {
+  return (size_t)4 * at_tiles(nd, E) * (m->N + 1) >= (size_t)5 * m->sm_count;
+}
+
+// The tiled kernel's weights, built with the first Held-Suarez model that it serves (freed with the mesh)
+int hs_tables_build(jgcm_mesh* m, int nd, int E) {
+  if (m->d_at || is_fp64(m) || !at_fits(m) || !at_pays(m, nd, E)) return JGCM_OK;
+  const size_t n = (size_t)(m->N + 1) * m->nh * at_pitch(m->ns);
+  JG_CUDA(cudaMalloc(&m->d_at, n * sizeof(float)));
+  k_at_weights<<<(int)std::min<size_t>((n + 255) / 256, 1184), 256, 0, m->stream>>>(tables<float>(m), m->d_at, m->N, m->ns, m->nh);
+  JG_CUDA(cudaGetLastError());
+  return JGCM_OK;
+}
+
 // The Held-Suarez analysis kernel serves this mesh: not tuned away (levels per block -1), SIMT
 // Legendre path, weights in 16-byte rows, shared memory within the budget.
 bool hs_analysis_fits(const jgcm_mesh* m, int nd, int E) {
   if (m->hs_levels < 0) return false;  // tuned to the general analysis kernel
   if (m->tc.on && !m->simt_legendre) return false;
-  // weight rows of a power-of-two nh/4 16-byte chunks (at most 32: one warp pass per row or more)
-  if (m->nh < 4 || m->nh > 128 || (m->nh & (m->nh - 1)) != 0) return false;
+  if (m->nh % 4 != 0) return false;  // weights four at a time (and rows of whole 16-byte chunks)
   const int LG = hs_analysis_levels(m, nd, E);
   if (LG < 1) return false;
   const size_t sm = is_fp64(m) ? hs_analysis_smem<double>(m, LG) : hs_analysis_smem<float>(m, LG);
@@ -315,6 +483,10 @@ int launch_hs_analysis(jgcm_mesh* m, const FFTPlan& fp, int colU, int colV, int 
   JG_TRY(g_hs_ana_smem[sizeof(T) == 8 ? 1 : 0].run([]() -> int {
     JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    if constexpr (std::is_same<T, float>::value) {
+      JG_CUDA(cudaFuncSetAttribute(k_hs_analysis_tiles<384, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+      JG_CUDA(cudaFuncSetAttribute(k_hs_analysis_tiles<640, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    }
     return JGCM_OK;
   }));
   HSAnaArgs<T> a;
@@ -337,6 +509,19 @@ int launch_hs_analysis(jgcm_mesh* m, const FFTPlan& fp, int colU, int colV, int 
   a.nlat = m->nlat;
   a.nh = m->nh;
   a.LG = LG;
+  if constexpr (std::is_same<T, float>::value) {
+    const int th = 32 * at_groups(m->ns + 1);
+    // (the columns in the step's order, 32-bit offsets)
+    if (m->d_at && m->hs_levels == 0 && at_pays(m, nd, E) && colV == colU + a.L && colT == colU + 2 * a.L &&
+        colE == colU + 3 * a.L && (size_t)(m->N + 1) * m->nlat * fp.C < ((size_t)1 << 31)) {
+      const dim3 gt(at_tiles(nd, E), m->N + 1);
+      JG_CUDA(th <= 384 ? launch_pdl(k_hs_analysis_tiles<384, 2>, gt, th, at_smem(m), st, a, tables<float>(m), m->d_at)
+                        : launch_pdl(k_hs_analysis_tiles<640, 1>, gt, th, at_smem(m), st, a, tables<float>(m), m->d_at));
+      mark(st);
+      JG_CUDA(cudaGetLastError());
+      return JGCM_OK;
+    }
+  }
   const int np = hs_analysis_np(E);
   const int threads = (hs_analysis_rows(m, np) * LG + 31) / 32 * 32;
   dim3 grid(m->N / 2 + 1, (nd + 1 + LG - 1) / LG, E);

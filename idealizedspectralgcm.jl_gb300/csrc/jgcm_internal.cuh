@@ -258,6 +258,7 @@ struct jgcm_mesh {
   int simt_legendre;       // tensor-core precision modes: 1 = run the Legendre contractions on the FP32
                            // SIMT kernels instead (chosen by the autotuner where they are faster)
   int hs_levels;           // levels per block of the Held-Suarez analysis kernel (0 = default)
+  float* d_at;             // weights of the tiled Held-Suarez analysis (NULL: not built)
   // workspace
   int Cmax;
   void* d_fbuf;       // Fourier buffer [m][j][c] complex T, c < Cmax
@@ -382,6 +383,7 @@ size_t simt_smem_need(const jgcm_mesh* m, int s2g, int g2s, int fft);
 // hs_transforms.cu: the Held-Suarez step's analysis as one contraction per (m pair, level group,
 // member); the forward FFT of the plan first
 bool hs_analysis_fits(const jgcm_mesh* m, int nd, int E);
+int hs_tables_build(jgcm_mesh* m, int nd, int E);
 int hs_analysis_levels(const jgcm_mesh* m, int nd, int E);
 template <typename T>
 int launch_hs_analysis(jgcm_mesh* m, const FFTPlan& fp, int colU, int colV, int colE, int colT, int colP, int nd,

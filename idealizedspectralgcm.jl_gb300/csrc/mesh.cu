@@ -253,7 +253,7 @@ static void mesh_free(jgcm_mesh* m) {
   if (!m) return;
   void* ps[] = {m->d_sinth, m->d_wts, m->d_costh, m->d_qnm, m->d_dqnm, m->d_ref2, m->d_fbuf, m->d_stage,
                 m->d_grid[0], m->d_grid[1], m->d_grid[2], m->d_grid[3], m->d_spec[0], m->d_spec[1], m->d_spec[2],
-                m->d_spec[3], m->d_red, m->d_counter, m->d_status};
+                m->d_spec[3], m->d_red, m->d_counter, m->d_status, m->d_at};
   for (auto p : ps)
     if (p) cudaFree(p);
   tc_tables_free(m);

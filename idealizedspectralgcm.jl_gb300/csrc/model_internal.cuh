@@ -78,10 +78,10 @@ struct jgcm_model {
   // FP64 semi-implicit data
   jgcm::VertCoef vc;
   jgcm::VertCoef* d_vc;  // device copy
-  void* d_vt;            // its VertT of the state precision, read by the column, fixer and semi-implicit kernels
+  void* d_vt;            // its VertT of the state precision (in d_vc's allocation): the kernels' coefficients
   double* div_mat;  // host nd*nd column-major
   double* d_W;      // device [2][N+1][nd][nd] (transposed: [c][r])
-  float2* d_W2;     // FP32 path: the same as pairs hi + lo
+  float2* d_W2;     // FP32 path: the same as pairs hi + lo (in d_W's allocation)
   int2* d_pairs;    // (m, n) pairs with n >= m
   int npairs;
   double *d_partials, *d_scalars;

@@ -12,6 +12,7 @@
 // solve runs in FP64 (one warp per spectral mode, lanes over levels) and the mass/energy
 // fixers (Spectral_Dynamics.jl:5-68) use deterministic FP64 reductions.
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -1579,9 +1580,14 @@ template <typename T>
 int build_vert_t(jgcm_model* md) {
   const VertCoef& vc = md->vc;
   const int nd = md->nd;
-  std::vector<VertT<T>> h(1);
-  VertT<T>& v = h[0];
+  struct Both {
+    VertCoef c;
+    VertT<T> t;
+  };
+  std::vector<Both> h(1);
+  VertT<T>& v = h[0].t;
   memset(&v, 0, sizeof(v));
+  h[0].c = vc;
   for (int k = 0; k <= nd; k++) {
     v.ak[k] = (T)vc.ak[k];
     v.bk[k] = (T)vc.bk[k];
@@ -1607,8 +1613,9 @@ int build_vert_t(jgcm_model* md) {
     v.tdh[k] = k + 1 <= nd - 1 ? (T)(vc.t_ref[k + 1] - vc.t_ref[k]) : (T)0;
     v.hk[k] = (T)(vc.h[k] * md->P.ps_ref);
   }
-  JG_TRY(alloc(&md->d_vt, sizeof(v)));
-  JG_CUDA(cudaMemcpy(md->d_vt, &v, sizeof(v), cudaMemcpyHostToDevice));
+  JG_TRY(alloc((void**)&md->d_vc, sizeof(Both)));
+  JG_CUDA(cudaMemcpy(md->d_vc, h.data(), sizeof(Both), cudaMemcpyHostToDevice));
+  md->d_vt = (char*)md->d_vc + offsetof(Both, t);
   return JGCM_OK;
 }
 
@@ -1665,8 +1672,8 @@ void model_free(jgcm_model* md) {
   void* ps[] = {md->grid_vor, md->grid_div, md->grid_lnps, md->grid_t_eq, md->grid_geopots, md->grid_h_eq,
                 md->spe_zero, md->spe_dvor, md->spe_ddiv, md->spe_dlnps, md->spe_dt, md->g_dlps, md->g_dtps,
                 md->g_dlT, md->g_dtT, md->g_ducos, md->g_dvcos, md->g_dt, md->g_energy, md->g_dlnps, md->g_diag,
-                md->g_tdev, md->coriolis, md->damping, md->dfac[0], md->dfac[1], md->d_W, md->d_W2, md->d_pairs, md->d_partials,
-                md->d_scalars, md->d_counter, md->d_vc, md->d_vt, md->fbuf, md->diag};
+                md->g_tdev, md->coriolis, md->damping, md->dfac[0], md->dfac[1], md->d_W, md->d_pairs, md->d_partials,
+                md->d_scalars, md->d_counter, md->d_vc, md->fbuf, md->diag};
   for (auto p : ps)
     if (p) cudaFree(p);
   delete[] md->div_mat;
@@ -1759,8 +1766,9 @@ int model_alloc(jgcm_model* md) {
   JG_TRY(alloc(&md->g_diag, grid_elems(m, 1) * (7 * (size_t)nd + 3) * 8));
   JG_TRY(alloc(&md->coriolis, (size_t)m->nlat * ts));
   JG_TRY(alloc(&md->damping, (size_t)(N + 1) * (ns + 1) * ts));
-  JG_TRY(alloc((void**)&md->d_W, 2 * (size_t)(N + 1) * nd * nd * 8));
-  if (!is_fp64(m)) JG_TRY(alloc((void**)&md->d_W2, 2 * (size_t)(N + 1) * nd * nd * sizeof(float2)));
+  const size_t nW = 2 * (size_t)(N + 1) * nd * nd;
+  JG_TRY(alloc((void**)&md->d_W, nW * (is_fp64(m) ? 8 : 16)));  // FP32: the pairs behind
+  if (!is_fp64(m)) md->d_W2 = (float2*)(md->d_W + nW);
   std::vector<int2> pairs;
   for (int mm = 0; mm <= N; mm++)
     for (int n = mm; n <= ns; n++) pairs.push_back(make_int2(mm, n));
@@ -1794,10 +1802,11 @@ int model_alloc(jgcm_model* md) {
   JG_CUDA(cudaEventCreate(&md->ev1));
   md->div_mat = new double[nd * nd]();
   vertical_setup(md);
-  JG_TRY(alloc((void**)&md->d_vc, sizeof(VertCoef)));
-  JG_CUDA(cudaMemcpy(md->d_vc, &md->vc, sizeof(VertCoef), cudaMemcpyHostToDevice));
   JG_TRY(is_fp64(m) ? build_vert_t<double>(md) : build_vert_t<float>(md));
-  if (md->P.kind == JGCM_HELD_SUAREZ) JG_TRY(build_wave(md));
+  if (md->P.kind == JGCM_HELD_SUAREZ) {
+    JG_TRY(hs_tables_build(m, nd, ne));
+    JG_TRY(build_wave(md));
+  }
   JG_CUDA(cudaStreamSynchronize(m->stream));
   return JGCM_OK;
 }

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from jgcm import configs
+from test_gpu_models import MIXED_TOL, _compare
 from test_gpu_transforms import TOL, _grid, _meshes, _spec
 
 pytestmark = pytest.mark.gpu
@@ -53,6 +54,31 @@ def test_one_layer_steps(jg, orc, N, nlat, nlon, prec, tol):
     omod.step(6)
     for f in configs.PROGNOSTIC["barotropic"]:
         assert configs.rel_l2(gmod.get(f), omod.get(f)) < tol, f
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", MIXED_TOL["fp32"])])
+@pytest.mark.parametrize("N,nlat,nlon,nd,members", [(21, 40, 64, 7, 1), (31, 48, 128, 13, 1), (31, 48, 128, 13, 29),
+                                                    (42, 64, 128, 20, 11), (63, 96, 256, 9, 1), (63, 96, 256, 9, 17)])
+def test_held_suarez_steps(jg, orc, N, nlat, nlon, nd, members, prec, tol):
+    """Held-Suarez steps on latitude counts that are no power of two, alone and as ensembles large enough
+    for the tiled Legendre kernels, whose column tiles straddle members: the first and last members against
+    the oracle, at the step tolerances."""
+    if prec == "fp64" and members > 1:
+        members = 3
+    params = configs.PARAMS["hs_t21l20"]
+    gm, om = _meshes(jg, orc, N, nlat, nlon, nd, prec)
+    omod, one = orc.Model(om, params), jg.Model(gm, params)
+    configs.init_held_suarez(orc, om, omod)
+    configs.add_hs_flow(orc, om, omod)
+    configs.copy_state(omod, one, "held_suarez")
+    ens = jg.Model(gm, params, members=members)
+    for e in range(members):
+        ens.copy_member(e, one)
+    ens.step(3)
+    omod.step(3)
+    for e in {0, members - 1}:
+        one.copy_member(0, ens, e)
+        _compare(one, omod, "held_suarez", tol)
 
 
 def _shifted(a):
