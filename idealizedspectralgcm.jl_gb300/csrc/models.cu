@@ -1,7 +1,7 @@
 // models.cu -- device-resident time stepping of the three JGCM models.
 //
 //   Barotropic_Dynamics!        Barotropic_Dynamics.jl:2-46                 4 launches / step
-//   Shallow_Water_Dynamics!     Shallow_Water_Dynamics.jl:7-179             6 launches / step
+//   Shallow_Water_Dynamics!     Shallow_Water_Dynamics.jl:7-179             4 launches / step
 //   Atmosphere_Update! (HS)     Spectral_Dynamics.jl:206-365, 452-490,
 //                               HS_Forcing.jl:1-130, Semi_Implicit.jl        8 launches / step
 //
@@ -1897,14 +1897,13 @@ int step_barotropic(jgcm_model* md, cudaStream_t st) {
   return JGCM_OK;
 }
 
-// Shallow_Water_Physics! + Shallow_Water_Dynamics! (Shallow_Water_Dynamics.jl:7-179).
-// h lives in the lnps/ps slots; the advected height is spe_h_n, which equals spe_h_c after the
-// first Time_Advance! (Shallow_Water_Dynamics.jl:147).
+// The gradients of the advected height (÷ cos θ; Compute_Gradients!, Spectral_Spherical_Mesh.jl:721-741), for a
+// state that no step synthesised: the advected height is spe_h_n, which equals spe_h_c after the first
+// Time_Advance! (Shallow_Water_Dynamics.jl:147).
 template <typename T>
-int step_shallow_water(jgcm_model* md, cudaStream_t st) {
-  jgcm_mesh* m = md->mesh;
-  const int p = lvl(md, 0), c = lvl(md, 1), n = lvl(md, 2), E = md->ne;
-  const void* h_adv = md->sw_adv_from_n ? md->spe_lnps[n] : md->spe_lnps[c];
+int issue_sw_grad(jgcm_model* md, cudaStream_t st) {
+  const int E = md->ne;
+  const void* h_adv = md->spe_lnps[lvl(md, md->sw_adv_from_n ? 2 : 1)];
   S2GPlan sp;
   memset(&sp, 0, sizeof(sp));
   sp.ng = 2;
@@ -1917,7 +1916,18 @@ int step_shallow_water(jgcm_model* md, cudaStream_t st) {
   ip.C = 2 * E;
   ip.g[0] = og(EPI_DIVCOS, md->g_dlps, E, 0 * E);
   ip.g[1] = og(EPI_DIVCOS, md->g_dtps, E, 1 * E);
-  JG_TRY(launch_s2g<T>(m, sp, ip, st, md->fbuf, md->fcap));
+  return launch_s2g<T>(md->mesh, sp, ip, st, md->fbuf, md->fcap);
+}
+
+// Shallow_Water_Physics! + Shallow_Water_Dynamics! (Shallow_Water_Dynamics.jl:7-179).
+// h lives in the lnps/ps slots.  The gradients of the height that the next step advects are synthesised
+// with the new level, in its two launches: a step is four launches of a few microseconds instead of six
+// (T85 FP32 27.2 -> 22.6 us a step, FP64 91 -> 75).
+template <typename T>
+int step_shallow_water(jgcm_model* md, cudaStream_t st) {
+  jgcm_mesh* m = md->mesh;
+  const int p = lvl(md, 0), c = lvl(md, 1), n = lvl(md, 2), E = md->ne;
+  if (!md->grad_ready) JG_TRY(issue_sw_grad<T>(md, st));
   FFTPlan fp;
   memset(&fp, 0, sizeof(fp));
   fp.ng = 4;
@@ -1957,22 +1967,26 @@ int step_shallow_water(jgcm_model* md, cudaStream_t st) {
   JG_TRY(launch_g2s<T>(m, fp, gp, st, md->fbuf, md->fcap));
   S2GPlan sp2;
   memset(&sp2, 0, sizeof(sp2));
-  sp2.ng = 5;
-  sp2.C = 5 * E;
+  sp2.ng = 7;
+  sp2.C = 7 * E;
   sp2.g[0] = sg(S2G_PLAIN, md->spe_vor[n], nullptr, E, 0 * E);
   sp2.g[1] = sg(S2G_PLAIN, md->spe_div[n], nullptr, E, 1 * E);
   sp2.g[2] = sg(S2G_PLAIN, md->spe_lnps[n], nullptr, E, 2 * E);
   sp2.g[3] = sg(S2G_UCOS, md->spe_vor[n], md->spe_div[n], E, 3 * E);
   sp2.g[4] = sg(S2G_VCOS, md->spe_vor[n], md->spe_div[n], E, 4 * E);
+  sp2.g[5] = sg(S2G_DLAM, md->spe_lnps[n], nullptr, E, 5 * E);
+  sp2.g[6] = sg(S2G_DTH, md->spe_lnps[n], nullptr, E, 6 * E);
   IFFTPlan ip2;
   memset(&ip2, 0, sizeof(ip2));
-  ip2.ng = 5;
-  ip2.C = 5 * E;
+  ip2.ng = 7;
+  ip2.C = 7 * E;
   ip2.g[0] = og(EPI_NONE, md->grid_vor, E, 0 * E);
   ip2.g[1] = og(EPI_NONE, md->grid_div, E, 1 * E);
   ip2.g[2] = og(EPI_NONE, md->grid_ps[n], E, 2 * E);
   ip2.g[3] = og(EPI_DIVCOS, md->grid_u[n], E, 3 * E);
   ip2.g[4] = og(EPI_DIVCOS, md->grid_v[n], E, 4 * E);
+  ip2.g[5] = og(EPI_DIVCOS, md->g_dlps, E, 5 * E);
+  ip2.g[6] = og(EPI_DIVCOS, md->g_dtps, E, 6 * E);
   JG_TRY(launch_s2g<T>(m, sp2, ip2, st, md->fbuf, md->fcap));
   return JGCM_OK;
 }
@@ -2371,7 +2385,7 @@ int issue(jgcm_model* md, cudaStream_t st) {
 }
 
 void after_step(jgcm_model* md) {
-  md->grad_ready = md->P.kind == JGCM_HELD_SUAREZ;
+  md->grad_ready = md->P.kind != JGCM_BAROTROPIC;
   if (md->diag_on) md->diag_steps++;
   md->rot = (md->rot + 1) % 3;
   md->init_step = 0;
@@ -2426,8 +2440,10 @@ int graph_step(jgcm_model* md) {
 
 // K steady steps through one CUDA graph (K a multiple of 3: whole time-level rotations): fewer graph
 // launches, and the step boundaries inside become ordinary (programmatic) kernel edges.
+// the gradients that the next step reads are there
+bool grads(const jgcm_model* md) { return md->P.kind == JGCM_BAROTROPIC || md->grad_ready; }
 bool steady(const jgcm_model* md) {
-  return !(md->init_step || md->sw_adv_from_n || (md->P.kind == JGCM_HELD_SUAREZ && !md->grad_ready));
+  return !(md->init_step || md->sw_adv_from_n || !grads(md));
 }
 
 int graph_steps(jgcm_model* md, int K, cudaGraphExec_t* slots) {
@@ -2473,7 +2489,7 @@ int graph_step3(jgcm_model* md) { return graph_steps(md, 3, md->graph3); }
 int graph_step24(jgcm_model* md) { return graph_steps(md, 24, md->graph24); }
 
 int model_step(jgcm_model* md) {
-  if (md->init_step || md->sw_adv_from_n || (md->P.kind == JGCM_HELD_SUAREZ && !md->grad_ready)) {
+  if (!steady(md)) {
     JG_TRY(issue(md, md->mesh->stream));
     after_step(md);
     return JGCM_OK;
@@ -2715,7 +2731,7 @@ extern "C" int jgcm_model_update_init_step(jgcm_model* md) {
 }
 
 static int launches_per_step(const jgcm_model* md) {
-  return md->P.kind == JGCM_BAROTROPIC ? 4 : md->P.kind == JGCM_SHALLOW_WATER ? 6 : md->nq ? 11 : 8;
+  return md->P.kind == JGCM_BAROTROPIC ? 4 : md->P.kind == JGCM_SHALLOW_WATER ? 4 : md->nq ? 11 : 8;
 }
 
 extern "C" int jgcm_model_launches_per_step(jgcm_model* md, int* launches) {
@@ -2730,9 +2746,8 @@ extern "C" int jgcm_model_kernel_name(jgcm_model* md, int slot, char* buf, int c
                              "s2g_legendre(vor,div,u,v,T,lnps,grad lnps,grad T)",
                              "ifft(vor,div,u,v,T,lnps,grad lnps,grad T)", "hs_corr_reduce", "hs_corr_apply"};
   static const char* bt[] = {"fft(flux)", "g2s_legendre(vor+leapfrog)", "s2g_legendre(vor,u,v)", "ifft(vor,u,v)"};
-  static const char* sw[] = {"s2g_legendre(grad h)", "ifft(grad h)", "fft(fluxes,kin,dh)",
-                             "g2s_legendre(vor,div,h+implicit+leapfrog)", "s2g_legendre(vor,div,h,u,v)",
-                             "ifft(vor,div,h,u,v)"};
+  static const char* sw[] = {"fft(fluxes,kin,dh)", "g2s_legendre(vor,div,h+implicit+leapfrog)",
+                             "s2g_legendre(vor,div,h,u,v,grad h)", "ifft(vor,div,h,u,v,grad h)"};
   static const char* hsq[] = {"hs_column", "hs_tracers", "fft(tendencies)", "g2s_legendre(vor,div,T,lnps)",
                               "fft(tracers)", "g2s_legendre(tracers)", "hs_implicit",
                               "s2g_legendre(vor,div,u,v,T,lnps,grad lnps,grad T,tracers)",
@@ -2759,7 +2774,7 @@ extern "C" int jgcm_model_kernel_times(jgcm_model* md, int nsteps, float* ms, in
   jgcm_mesh* m = md->mesh;
   const int L = launches_per_step(md);
   JG_ARG(cap >= L, "buffer too small");
-  if (md->init_step || (md->P.kind == JGCM_HELD_SUAREZ && !md->grad_ready)) JG_TRY(model_step(md));
+  while (!steady(md)) JG_TRY(model_step(md));
   struct DiagOff {  // the timed steps run without the diagnostics' reductions (and are not summed)
     jgcm_model* md;
     int saved;
@@ -2811,8 +2826,7 @@ extern "C" int jgcm_model_kernel_times(jgcm_model* md, int nsteps, float* ms, in
 extern "C" int jgcm_model_time_steps(jgcm_model* md, int nsteps, float* ms) {
   JG_ARG(md && ms && nsteps > 0, "bad arguments");
   jgcm_mesh* m = md->mesh;
-  while (md->init_step || md->sw_adv_from_n || (md->P.kind == JGCM_HELD_SUAREZ && !md->grad_ready))
-    JG_TRY(model_step(md));
+  while (!steady(md)) JG_TRY(model_step(md));
   // capture every rotation phase before timing (after a tile change the graphs are rebuilt)
   auto captured = [&]() {
     if (md->graph_gen != m->tune_gen) return false;
@@ -3373,9 +3387,12 @@ int ensemble_graph(jgcm_ensemble* en, cudaGraphExec_t* out, int nwin) {
 
 int ensemble_windows(jgcm_ensemble* en, int nwin) {
   for (auto* md : en->models)  // window graphs start from ready gradients
-    if (md->P.kind == JGCM_HELD_SUAREZ && !md->grad_ready) {
-      JG_TRY(is_fp64(md->mesh) ? issue_hs_grad<double>(md, lvl(md, 1), en->st)
-                               : issue_hs_grad<float>(md, lvl(md, 1), en->st));
+    if (!grads(md)) {
+      if (md->P.kind == JGCM_HELD_SUAREZ)
+        JG_TRY(is_fp64(md->mesh) ? issue_hs_grad<double>(md, lvl(md, 1), en->st)
+                                 : issue_hs_grad<float>(md, lvl(md, 1), en->st));
+      else
+        JG_TRY(is_fp64(md->mesh) ? issue_sw_grad<double>(md, en->st) : issue_sw_grad<float>(md, en->st));
       md->grad_ready = 1;
     }
   cudaGraphExec_t g;
@@ -3479,7 +3496,7 @@ extern "C" int jgcm_ensemble_time(jgcm_ensemble* en, int nwindows, float* ms) {
     int st = JGCM_OK;
     for (int c = 0; c < count && st == JGCM_OK; c++) {
       bool ready = true;
-      for (auto* md : en->models) ready = ready && !(md->P.kind == JGCM_HELD_SUAREZ && !md->grad_ready);
+      for (auto* md : en->models) ready = ready && grads(md);
       if (!ready) break;  // the first window prepares the gradients; its graph is captured when it runs
       cudaGraphExec_t g;
       st = ensemble_graph(en, &g, nwin);
