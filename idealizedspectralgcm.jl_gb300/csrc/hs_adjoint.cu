@@ -330,54 +330,56 @@ __global__ void k_grad_adjoint(const V2<T>* __restrict__ sl, const V2<T>* __rest
 // follows weights m >= 1 twice and the grid cotangent of fft/nlon is (1/nlon) sum_m Re(F_bar e^{im
 // lam}), so the coefficients are stored x cos_j / (c_m nlon) (c_0 = 1, c_m = 2): the grid result is
 // then the cotangent of u and v themselves.  Fourier columns [0, nd) u, [nd, 2 nd) v.
-// grid (ceil(nh*nd/256), N+1), 256 threads: one (latitude pair, level) per thread.
+// grid (ceil(nh*nd/64), N+1), 256 threads: four lanes (8 apart) per (latitude pair, level), which take the rows
+// n in turns of two and then exchange their 16 sums so that each is left with one component of u or v.  With
+// one thread per (latitude pair, level) a chain of up to N + 1 rows of loads ran on one warp per scheduler
+// (T42L20 FP64 41 us, the FP64 pipe busy for 8 of them); split 24 us.
 template <typename T>
 __global__ void __launch_bounds__(256) k_alpha_adjoint(const V2<T>* __restrict__ bvor, const V2<T>* __restrict__ bdiv,
                                                        V2<T>* __restrict__ F, Tables<T> tb, int N, int ns, int nlat,
                                                        int nlon, int nd) {
   pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
   using V = V2<T>;
-  const int m = blockIdx.y, nh = nlat >> 1;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nh * nd) return;
+  const int m = blockIdx.y, nh = nlat >> 1, lane = threadIdx.x & 31, g = lane >> 3;
+  const int i0 = blockIdx.x * 64 + (threadIdx.x >> 5) * 8 + (lane & 7);
+  const bool act = i0 < nh * nd;
+  const int i = act ? i0 : nh * nd - 1;  // every lane of a warp takes part in the exchanges
   const int k = i % nd, jh = i / nd;
   const size_t row = (size_t)m * (ns + 1);
-  // even / odd (n - m) partial sums of the CA terms and of the CB terms, u and v
-  T uae[2] = {0, 0}, uao[2] = {0, 0}, ube[2] = {0, 0}, ubo[2] = {0, 0};
-  T vae[2] = {0, 0}, vao[2] = {0, 0}, vbe[2] = {0, 0}, vbo[2] = {0, 0};
-  for (int n = m; n <= ns - 1; n++) {
+  // [u, v][re, im]: even and odd (n - m) sums of the CA terms, then of the CB terms
+  T s[2][2][4] = {};
+  auto add = [&](int n, int odd) {
     const T ca = tb.CA[(row + n) * nh + jh], cb = tb.CB[(row + n) * nh + jh];
     const V vb = bvor[(row + n) * nd + k], db = bdiv[(row + n) * nd + k];
-    const bool odd = (n - m) & 1;
-    T* ua = odd ? uao : uae;
-    T* ub = odd ? ubo : ube;
-    T* va = odd ? vao : vae;
-    T* vbb = odd ? vbo : vbe;
-    ua[0] += ca * db.y;  // -i CA div_bar
-    ua[1] -= ca * db.x;
-    ub[0] -= cb * vb.x;  // -CB vor_bar
-    ub[1] -= cb * vb.y;
-    va[0] += ca * vb.y;  // -i CA vor_bar
-    va[1] -= ca * vb.x;
-    vbb[0] += cb * db.x;  // +CB div_bar
-    vbb[1] += cb * db.y;
+    s[0][0][odd] += ca * db.y;  // -i CA div_bar
+    s[0][1][odd] -= ca * db.x;
+    s[0][0][2 + odd] -= cb * vb.x;  // -CB vor_bar
+    s[0][1][2 + odd] -= cb * vb.y;
+    s[1][0][odd] += ca * vb.y;  // -i CA vor_bar
+    s[1][1][odd] -= ca * vb.x;
+    s[1][0][2 + odd] += cb * db.x;  // +CB div_bar
+    s[1][1][2 + odd] += cb * db.y;
+  };
+#pragma unroll 2
+  for (int n = m + 2 * g; n <= ns - 1; n += 8) {
+    add(n, 0);
+    if (n + 1 <= ns - 1) add(n + 1, 1);
   }
+  const bool gv = lane & 16, gi = lane & 8;  // this lane's field (u, v) and component (re, im)
+  T h[2][4], e[4];
+#pragma unroll
+  for (int c = 0; c < 2; c++)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      h[c][q] = (gv ? s[1][c][q] : s[0][c][q]) + __shfl_xor_sync(FULL, gv ? s[0][c][q] : s[1][c][q], 16);
+#pragma unroll
+  for (int q = 0; q < 4; q++) e[q] = (gi ? h[1][q] : h[0][q]) + __shfl_xor_sync(FULL, gi ? h[0][q] : h[1][q], 8);
+  if (!act) return;
   const T sc = tb.cosj[jh] / ((m == 0 ? (T)1 : (T)2) * (T)nlon);  // exact in T: no FP64 per thread
-  const int C = 2 * nd;
-  const int jn = nlat - 1 - jh;
-  V us, un, vs, vn;
-  us.x = (uae[0] + uao[0] + ube[0] + ubo[0]) * sc;
-  us.y = (uae[1] + uao[1] + ube[1] + ubo[1]) * sc;
-  un.x = (uae[0] - uao[0] - ube[0] + ubo[0]) * sc;
-  un.y = (uae[1] - uao[1] - ube[1] + ubo[1]) * sc;
-  vs.x = (vae[0] + vao[0] + vbe[0] + vbo[0]) * sc;
-  vs.y = (vae[1] + vao[1] + vbe[1] + vbo[1]) * sc;
-  vn.x = (vae[0] - vao[0] - vbe[0] + vbo[0]) * sc;
-  vn.y = (vae[1] - vao[1] - vbe[1] + vbo[1]) * sc;
-  F[((size_t)m * nlat + jh) * C + k] = us;
-  F[((size_t)m * nlat + jn) * C + k] = un;
-  F[((size_t)m * nlat + jh) * C + nd + k] = vs;
-  F[((size_t)m * nlat + jn) * C + nd + k] = vn;
+  T* Fc = reinterpret_cast<T*>(F) + (gv ? 2 * nd : 0) + (gi ? 1 : 0) + 2 * k;
+  const size_t C2 = 4 * (size_t)nd, r0 = (size_t)m * nlat;
+  Fc[(r0 + jh) * C2] = (e[0] + e[1] + e[2] + e[3]) * sc;
+  Fc[(r0 + nlat - 1 - jh) * C2] = (e[0] - e[1] - e[2] + e[3]) * sc;
 }
 
 // ---- the column kernel --------------------------------------------------------------------------
@@ -418,224 +420,287 @@ void col_adj_consts(ColAdjArgs<T>& a) {
   a.inv_2n = 0.5 / a.nlon;
 }
 
-template <typename R>
-__device__ __forceinline__ R up1(R x, int lane) {  // value of lane - 1 (0 for lane 0)
-  R y = __shfl_up_sync(FULL, x, 1);
-  return lane == 0 ? (R)0 : y;
+// Levels of a column over the 8 lanes of a warp with the same lane % 4: lane 4 l + c holds levels l NL ...
+// l NL + NL - 1 of the warp's column c, so that a level's loads and stores of 4 columns fill a 32-byte sector in
+// FP64.  Every lane takes part in each of these.
+template <typename R, int NL>
+__device__ __forceinline__ R level_below(const R (&x)[NL], int e, int lane) {  // value of level k - 1 (0 at k = 0)
+  if (e > 0) return x[e - 1];
+  const R y = __shfl_up_sync(FULL, x[NL - 1], 4);
+  return lane < 4 ? (R)0 : y;
 }
 template <typename R>
-__device__ __forceinline__ R dn1(R x, int lane) {  // value of lane + 1 (0 for lane 31)
-  R y = __shfl_down_sync(FULL, x, 1);
-  return lane == 31 ? (R)0 : y;
-}
-template <typename R>
-__device__ __forceinline__ R wsum(R x) {
+__device__ __forceinline__ R column_sum(R x) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL, x, o);
+  for (int o = 4; o < 32; o <<= 1) x += __shfl_xor_sync(FULL, x, o);
   return x;
 }
-template <typename R>
-__device__ __forceinline__ R scan_excl(R x, int lane) {  // sum over lanes < lane
-  R s = x;
+template <typename R, int NL>
+__device__ __forceinline__ void scan_excl(const R (&x)[NL], R (&y)[NL], int lane) {  // sums over the levels < k
+  R s = x[0];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    R y = __shfl_up_sync(FULL, s, o);
-    if (lane >= o) s += y;
+  for (int e = 1; e < NL; e++) s += x[e];
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    const R z = __shfl_up_sync(FULL, s, o);
+    if (lane >= o) s += z;
   }
-  return s - x;
+  s = __shfl_up_sync(FULL, s, 4);
+  y[0] = lane < 4 ? (R)0 : s;
+#pragma unroll
+  for (int e = 1; e < NL; e++) y[e] = y[e - 1] + x[e - 1];
 }
-template <typename R>
-__device__ __forceinline__ R rscan_excl(R x, int lane) {  // sum over lanes > lane
-  R s = x;
+template <typename R, int NL>
+__device__ __forceinline__ void rscan_excl(const R (&x)[NL], R (&y)[NL], int lane) {  // sums over the levels > k
+  R s = x[0];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    R y = __shfl_down_sync(FULL, s, o);
-    if (lane + o < 32) s += y;
+  for (int e = 1; e < NL; e++) s += x[e];
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    const R z = __shfl_down_sync(FULL, s, o);
+    if (lane + o < 32) s += z;
   }
-  return s - x;
+  s = __shfl_down_sync(FULL, s, 4);
+  y[NL - 1] = lane >= 28 ? (R)0 : s;
+#pragma unroll
+  for (int e = NL - 2; e >= 0; e--) y[e] = y[e + 1] + x[e + 1];
+}
+// The column's sums of eight values at once: lane 4 l + c returns the total of value l (each exchange halves the
+// values a lane still holds: 7 additions instead of 24)
+template <typename R>
+__device__ __forceinline__ R column_sum8(const R (&v)[8], int lane) {
+  R a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const R keep = lane & 16 ? v[i + 4] : v[i], give = lane & 16 ? v[i] : v[i + 4];
+    a[i] = keep + __shfl_xor_sync(FULL, give, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const R keep = lane & 8 ? a[i + 2] : a[i], give = lane & 8 ? a[i] : a[i + 2];
+    b[i] = keep + __shfl_xor_sync(FULL, give, 8);
+  }
+  const R keep = lane & 4 ? b[1] : b[0], give = lane & 4 ? b[0] : b[1];
+  return keep + __shfl_xor_sync(FULL, give, 4);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_hs_column_adjoint(ColAdjArgs<T> a, const VertCoef* __restrict__ vcp) {
+// On the FP64 path the kernel is bound by the FP64 pipe, which a warp's idle lanes, exchanges and what every lane
+// computes for its column occupy all the same: 4 columns per warp, NL = ceil(nd / 8) levels per lane (a column
+// per warp leaves 32 - nd lanes idle and takes 5 steps per scan or sum instead of 3); the column's logarithm,
+// power and reciprocals formed once (a thread per column), the level constants from the table, and the column's
+// sums in one exchange.  T42L20 FP64: 177 us (a column per warp, everything per level), 132 (a column per
+// warp), 77.  Blocks of 64 threads (8 columns): the SMs share the columns evenly.
+template <typename T, int NL>
+__global__ void __launch_bounds__(64) k_hs_column_adjoint(ColAdjArgs<T> a, const VertT<T>* __restrict__ vtp) {
   pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
   using R = T;
-  __shared__ double pw[8][5];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __shared__ double pw[2][5];
+  __shared__ R s_col[8][4];  // per column: ln(ps / p0), (ps / p0)^kappa, 1 / ps, 1 / cos
+  if (threadIdx.x < 8) {
+    const int c = min((int)blockIdx.x * 8 + (int)threadIdx.x, a.nlat * a.nlon - 1);
+    const R p = a.ps[c], l = log(p) - (R)a.ln_p0_t;
+    s_col[threadIdx.x][0] = l;
+    s_col[threadIdx.x][1] = exp((R)a.kappa_t * l);
+    s_col[threadIdx.x][2] = (R)1 / p;
+    s_col[threadIdx.x][3] = (R)1 / (R)a.cosj[c / a.nlon];
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, lq = lane >> 2, bc = wid * 4 + (lane & 3);
   const int G = a.nlat * a.nlon, nd = a.nd;
-  const int col = blockIdx.x * 8 + wid;
+  const int col = blockIdx.x * 8 + bc;
   const bool colv = col < G;
-  const int k = lane;
-  const bool act = colv && k < nd;
-  const VertCoef& vc = *vcp;
+  const int k0 = lq * NL;  // this lane's levels: k0 + e
+  const VertT<T>& vt = *vtp;
   const int j = colv ? col / a.nlon : 0;
-  const size_t x = (size_t)(colv ? col : 0) + (size_t)G * (act ? k : 0);
-  auto ld = [&](const T* p) -> R { return act ? (R)p[x] : (R)0; };
-  const R u = ld(a.u), v = ld(a.v), t = ld(a.t), vor = ld(a.vor), div = ld(a.div);
-  const R tl = ld(a.tl), tt = ld(a.tt), up = ld(a.up), vp = ld(a.vp), tp = ld(a.tp);
-  const R DU = ld(a.DU), DV = ld(a.DV), DT = ld(a.DT), EN = ld(a.EN);
   const size_t c1 = colv ? col : 0;
-  const R ps = a.ps[c1], psp = a.psp[c1], gl = a.gl[c1], gt = a.gt[c1];
-  const R DLN = colv ? (R)a.DLN[c1] : (R)0;
-  const R Rg = (R)a.rdgas_t, kap = (R)a.kappa_t;
-  // vertical constants; lanes >= nd carry zeros (dbk = 1 keeps the divisions finite)
-  const R bk = act ? (R)vc.bk[k] : (R)0, bk1 = act ? (R)vc.bk[k + 1] : (R)0, dbk = act ? (R)vc.dbk[k] : (R)1;
-  const R rdbk = (R)1 / dbk;
-  const R dlp_p = act ? (R)vc.dlp_p[k] : (R)0, dlp_m = (act && k >= 1) ? (R)vc.dlp_m[k] : (R)0;
-  const R dlp = (act && k >= 1) ? (R)vc.dlp[k] : (R)0, sf = act ? (R)vc.sf[k] : (R)1;
-  const R cf = act ? (R)vc.cf[k] : (R)0;
-  const R X1 = (bk * dlp_m + bk1 * dlp_p) * rdbk;  // x1 ps (Four_In_One!)
+  auto act = [&](int e) { return colv && k0 + e < nd; };
+  auto at = [&](int e) { return c1 + (size_t)G * (k0 + e); };
+  auto ld = [&](const T* p, int e) -> R { return act(e) ? (R)p[at(e)] : (R)0; };
+  // vertical constants; levels >= nd carry zeros
+  auto lc = [&](const T* p, int e) -> R { return act(e) ? (R)p[k0 + e] : (R)0; };
+  const R gl = a.gl[c1], gt = a.gt[c1];
+  const R Rg = (R)a.rdgas_t, kap = (R)a.kappa_t, f = (R)a.coriolis[j];
+  R u[NL], v[NL], t[NL], DU[NL], DV[NL], DT[NL], bu[NL], bv[NL], bt[NL];
+  R q[NL], x5[NL], Mt[NL], Mb[NL], Mbar[NL], s1[NL], s2v[NL];
+#pragma unroll
+  for (int e = 0; e < NL; e++) {
+    u[e] = ld(a.u, e);
+    v[e] = ld(a.v, e);
+    t[e] = ld(a.t, e);
+    DU[e] = ld(a.DU, e);
+    DV[e] = ld(a.DV, e);
+    DT[e] = ld(a.DT, e);
+  }
   // ---- forward of the column: Four_In_One! with the mass fluxes scaled by 1/ps ----
-  const R gu = u * gl + v * gt;
-  const R q = act ? dbk * (div + gu) : (R)0;  // dmean / ps
-  const R Tex = scan_excl(q, lane);           // dmean_tot before level k, / ps
-  const R Ttot = wsum(q);
-  const R x5 = -(Tex * dlp + q * dlp_p) * rdbk + X1 * gu;
-  const R Mt = (act && k >= 1) ? (-Tex + Ttot * bk) : (R)0;  // M_half[k] / ps (k = 1..nd-1)
-  const R Mn = dn1(Mt, lane);                                 // every lane takes part in the shuffle
-  const R Mb = (k + 1 < nd) ? Mn : (R)0;                      // M_half[k+1] / ps
-  const R dbk_m1 = up1(dbk, lane);
-  const R al = (act && k >= 1) ? dbk_m1 / (dbk_m1 + dbk) : (R)0;
+#pragma unroll
+  for (int e = 0; e < NL; e++) q[e] = lc(vt.dbk, e) * (ld(a.div, e) + (u[e] * gl + v[e] * gt));  // dmean / ps
+  scan_excl(q, s1, lane);  // dmean_tot before level k, / ps
+  R Ttot = q[0];
+#pragma unroll
+  for (int e = 1; e < NL; e++) Ttot += q[e];
+  Ttot = column_sum(Ttot);
+#pragma unroll
+  for (int e = 0; e < NL; e++) {
+    x5[e] = -(s1[e] * lc(vt.dlp, e) + q[e] * lc(vt.dlp_p, e)) * lc(vt.rdb, e) +
+            lc(vt.x1, e) * (u[e] * gl + v[e] * gt);
+    Mt[e] = act(e) && k0 + e >= 1 ? -s1[e] + Ttot * (R)vt.bk[k0 + e] : (R)0;  // M_half[k] / ps (k = 1..nd-1)
+  }
+  {
+    const R next = __shfl_down_sync(FULL, Mt[0], 4);  // M_half[k+1] / ps: 0 at k = nd - 1
+#pragma unroll
+    for (int e = 0; e < NL; e++) Mb[e] = e + 1 < NL ? Mt[e + 1 < NL ? e + 1 : 0] : lane >= 28 ? (R)0 : next;
+  }
   // ---- cotangents ----
-  R bu = act ? (R)a.seed_u[x] : (R)0, bv = act ? (R)a.seed_v[x] : (R)0;
-  R bt = act ? (R)a.seed_t[x] : (R)0;
-  // absolute-vorticity fluxes: du += (vor + f) v, dv -= (vor + f) u
-  const R av = vor + (R)a.coriolis[j];
-  const R bvor = DU * v - DV * u;
-  bv += DU * av;
-  bu -= DV * av;
-  // horizontal advection of T: dT -= u dT/dlam + v dT/dth
-  bu -= DT * tl;
-  bv -= DT * tt;
-  const R btl = -DT * u, btt = -DT * v;
+#pragma unroll
+  for (int e = 0; e < NL; e++) {
+    // absolute-vorticity fluxes: du += (vor + f) v, dv -= (vor + f) u; horizontal advection of T:
+    // dT -= u dT/dlam + v dT/dth; energy = geopotential + |u|^2 / 2
+    const R av = ld(a.vor, e) + f;
+    s2v[e] = ld(a.EN, e);
+    bu[e] = ld(a.seed_u, e) - DV[e] * av - DT[e] * ld(a.tl, e) + s2v[e] * u[e];
+    bv[e] = ld(a.seed_v, e) + DU[e] * av - DT[e] * ld(a.tt, e) + s2v[e] * v[e];
+    bt[e] = ld(a.seed_t, e);
+    Mbar[e] = 0;
+  }
   // vertical advection (Vert_Advection!, dz = dp = dbk ps, w = M_half): flux_k = w_k r_int_k
-  R Mbar = 0;
-  auto vadv = [&](R r, R Rb, R& rb) {
-    const R r_m1 = up1(r, lane);
-    const R rint = (k >= 1) ? r_m1 + (r - r_m1) * al : (R)0;
-    const R qq = Rb * rdbk;
-    const R qq_m1 = up1(qq, lane);
-    const R fb = (act && k >= 1) ? qq - qq_m1 : (R)0;  // flux_k enters rdt_k (+) and rdt_{k-1} (-)
-    rb += qq * (Mb - Mt);
-    Mbar += -qq * r + ((k >= 1) ? qq_m1 * r_m1 : (R)0);
-    Mbar += fb * rint;
-    rb += fb * Mt * al;
-    rb += dn1(fb * Mt * ((R)1 - al), lane);  // r_{k-1} share of flux_k, from lane k + 1's view
+  auto vadv = [&](const R(&r)[NL], const R(&Rb)[NL], R(&rb)[NL]) {
+    R qq[NL], sh[NL];  // sh: the r_{k-1} share of flux_k, from level k's view
+#pragma unroll
+    for (int e = 0; e < NL; e++) qq[e] = Rb[e] * lc(vt.rdb, e);
+#pragma unroll
+    for (int e = 0; e < NL; e++) {
+      const R r_m1 = level_below(r, e, lane), qq_m1 = level_below(qq, e, lane);
+      const bool in = act(e) && k0 + e >= 1;
+      const R al = in ? (R)vt.w1[k0 + e - 1] : (R)0;  // Δb_{k-1} / (Δb_{k-1} + Δb_k)
+      const R rint = r_m1 + (r[e] - r_m1) * al;
+      const R fb = in ? qq[e] - qq_m1 : (R)0;  // flux_k enters rdt_k (+) and rdt_{k-1} (-)
+      const R fm = fb * Mt[e], fa = fm * al;
+      rb[e] += qq[e] * (Mb[e] - Mt[e]) + fa;
+      sh[e] = fm - fa;
+      Mbar[e] += fb * rint + qq_m1 * r_m1 - qq[e] * r[e];
+    }
+    const R next = __shfl_down_sync(FULL, sh[0], 4);
+#pragma unroll
+    for (int e = 0; e < NL; e++) rb[e] += e + 1 < NL ? sh[e + 1 < NL ? e + 1 : 0] : lane >= 28 ? (R)0 : next;
   };
   vadv(u, DU, bu);
   vadv(v, DV, bv);
   vadv(t, DT, bt);
-  // dlnps = dps / ps = -dmean_tot / ps
-  R Tbar_tot = -DLN;
-  // energy = geopotential + |u|^2 / 2: Phi_k = R (t_k dlp_p_k + sum_{l > k} t_l dlp_l)
-  bu += EN * u;
-  bv += EN * v;
-  bt += Rg * (EN * dlp_p + dlp * scan_excl(EN, lane));
+  // Phi_k = R (t_k dlp_p_k + sum_{l > k} t_l dlp_l)
+  scan_excl(s2v, s1, lane);
   // Four_In_One! reversed: M_half[k] = -tot_k + tot_nd b_k
-  R Tbar = (act && k >= 1) ? -Mbar : (R)0;
-  Tbar_tot += wsum((act && k >= 1) ? Mbar * bk : (R)0);
-  bt += kap * x5 * DT;
-  const R bx5 = kap * t * DT;
-  if (k >= 1) Tbar -= bx5 * dlp * rdbk;
-  R qbar = -bx5 * dlp_p * rdbk;
-  R gub = bx5 * X1;
-  bt -= Rg * X1 * (gl * DU + gt * DV);
-  R glb = -Rg * t * X1 * DU, gtb = -Rg * t * X1 * DV;
-  qbar += rscan_excl(act ? Tbar : (R)0, lane) + Tbar_tot;  // tot_k = sum_{l < k} dmean_l
-  const R bdiv = qbar * dbk;
-  gub += qbar * dbk;
-  bu += gub * gl;
-  bv += gub * gt;
-  glb += gub * u;
-  gtb += gub * v;
+  R mb = 0;
+  R glb = 0, gtb = 0;
+#pragma unroll
+  for (int e = 0; e < NL; e++) {
+    const bool in = act(e) && k0 + e >= 1;
+    const R dlp = lc(vt.dlp, e), dlp_p = lc(vt.dlp_p, e), rdbk = lc(vt.rdb, e), X1 = lc(vt.x1, e);  // X1 = x1 ps
+    bt[e] += Rg * (s2v[e] * dlp_p + dlp * s1[e]) + kap * x5[e] * DT[e] - Rg * X1 * (gl * DU[e] + gt * DV[e]);
+    if (in) mb += Mbar[e] * (R)vt.bk[k0 + e];
+    const R bx5 = kap * t[e] * DT[e], bxr = bx5 * rdbk, rtx = Rg * t[e] * X1;
+    Mbar[e] = in ? -Mbar[e] - bxr * dlp : (R)0;  // cotangent of tot_k
+    q[e] = -bxr * dlp_p;                         // ... of dmean_k
+    x5[e] = bx5 * X1;                            // ... of grad ln ps . u
+    glb -= rtx * DU[e];
+    gtb -= rtx * DV[e];
+  }
+  // dlnps = dps / ps = -dmean_tot / ps
+  const R Tbar_tot = column_sum(mb) - (colv ? (R)a.DLN[c1] : (R)0);
+  rscan_excl(Mbar, s1, lane);  // tot_k = sum_{l < k} dmean_l
+  const R rc = s_col[bc][3];
+#pragma unroll
+  for (int e = 0; e < NL; e++) {
+    const R bdiv = (q[e] + s1[e] + Tbar_tot) * lc(vt.dbk, e);
+    const R gub = x5[e] + bdiv;
+    glb += gub * u[e];
+    gtb += gub * v[e];
+    if (act(e)) {
+      const size_t x = at(e);
+      a.bu[x] = (T)(bu[e] + gub * gl);
+      a.bv[x] = (T)(bv[e] + gub * gt);
+      a.bt[x] = (T)bt[e];
+      a.bvor[x] = (T)(DU[e] * v[e] - DV[e] * u[e]);
+      a.bdiv[x] = (T)bdiv;
+      a.btl[x] = (T)(-DT[e] * u[e] * rc);
+      a.btt[x] = (T)(-DT[e] * v[e] * rc);
+    }
+  }
   // ---- HS_Forcing! of the p level and the energy integral of Compute_Corrections_Init ----
   const R t_zero = 315, t_strat = 200, sb = (R)a.sigma_b_t;
   const R sj = a.sinj[j], s2 = sj * sj, c2 = (R)1 - s2, c4 = c2 * c2;
-  const R Ep_bar = (R)a.sc[SC_EP_BAR], Wc = (R)(a.wts[j] * a.inv_2n);
-  const R Dt = (R)a.Dt, icp = (R)a.inv_cp_t, ig = (R)a.inv_grav_t;
-  const R lps = log(ps) - (R)a.ln_p0_t;  // one logarithm per column
-  R bup = 0, bvp = 0, btp = 0, bps_l = 0, bpsp_l = 0;
-  R pb0 = 0, pb1 = 0, pb2 = 0, pb3 = 0, pb4 = 0;
-  if (act) {
-    const R s = sf - sb, sp = s > (R)0 ? s : (R)0;  // sigma = p_k / ps
+  const R Wc = (R)(a.wts[j] * a.inv_2n), EW = (R)a.sc[SC_EP_BAR] * Wc * (R)a.inv_grav_t, EWp = EW * a.psp[c1];
+  const R Dt = (R)a.Dt, icp = (R)a.inv_cp_t, inv_day = (R)a.inv_day_t;
+  const R lps = s_col[bc][0], tz = t_zero - (R)a.dT_y_t * s2, dth = (R)a.dtheta_z_t * c2;
+  R bps = 0, bpsp = 0, pb0 = 0, pb1 = 0, pb2 = 0, pb3 = 0, pb4 = 0;
+#pragma unroll
+  for (int e = 0; e < NL; e++) {
+    if (!act(e)) continue;
+    const size_t x = at(e);
+    const int k = k0 + e;
+    const R up = a.up[x], vp = a.vp[x], tp = a.tp[x], dbk = vt.dbk[k];
+    const R s = vt.sf[k] - sb, sp = s > (R)0 ? s : (R)0;  // sigma = p_k / ps
     const R kv = (R)a.kvc_t * sp;
     const R duf = -kv * up, dvf = -kv * vp;
-    const R lpn = cf + lps;                  // ln(p_k / p0)
-    const R pk = exp(kap * lpn);             // (p_k / p0)^kappa
-    const R pn = sf * ps * (R)1.0e-5;        // p_k / p0
-    const R tpot = t_zero - (R)a.dT_y_t * s2 - (R)a.dtheta_z_t * c2 * lpn;
+    const R lpn = vt.cf[k] + lps;            // ln(p_k / p0)
+    const R pk = vt.ek[k] * s_col[bc][1];    // (p_k / p0)^kappa
+    const R tpot = tz - dth * lpn;
     const R te = tpot * pk;
     const R teq = te > t_strat ? te : t_strat;
     const R kt = (R)a.ka_t + (R)a.ktc_t * sp * c4;
     const R fr = -((up + (R)0.5 * duf * Dt) * duf + (vp + (R)0.5 * dvf * Dt) * dvf) * icp;
-    const R dTf = fr - kt * (tp - teq);
+    const R dtq = tp - teq;
+    const R dTf = fr - kt * dtq;
     const R aa = up + Dt * duf, bb = vp + Dt * dvf;
     const R enp = (R)0.5 * (aa * aa + bb * bb) + (R)a.cp_t * (tp + Dt * dTf);
-    bpsp_l = Ep_bar * Wc * ig * enp * dbk;
-    const R eb = Ep_bar * Wc * ((R)vc.dak[k] + dbk * psp) * ig;
+    bpsp += EW * enp * dbk;
+    const R eb = EWp * dbk, cpe = (R)a.cp_t * eb;
     const R ba = eb * aa, bbv = eb * bb;
-    btp += (R)a.cp_t * eb;
-    R bdTf = DT + (R)a.cp_t * Dt * eb;
-    R bduf = DU + Dt * ba;
-    R bdvf = DV + Dt * bbv;
-    bup += ba;
-    bvp += bbv;
-    const R bkt = -bdTf * (tp - teq);
-    btp -= kt * bdTf;
-    const R bteq = kt * bdTf;
-    bduf -= bdTf * (up + duf * Dt) * icp;
-    bup -= bdTf * duf * icp;
-    bdvf -= bdTf * (vp + dvf * Dt) * icp;
-    bvp -= bdTf * dvf * icp;
+    const R bdTf = DT[e] + cpe * Dt, bdi = bdTf * icp;
+    const R bduf = DU[e] + Dt * ba - bdi * aa;
+    const R bdvf = DV[e] + Dt * bbv - bdi * bb;
+    const R bkt = -bdTf * dtq, bteq = kt * bdTf;
+    a.btp[x] = (T)(cpe - bteq);
+    a.bup[x] = (T)(ba - bdi * duf - kv * bduf);
+    a.bvp[x] = (T)(bbv - bdi * dvf - kv * bdvf);
     const R bkv = -bduf * up - bdvf * vp;
-    bup -= kv * bduf;
-    bvp -= kv * bdvf;
-    const R spn = sp * (R)a.inv_1msb_t;
-    pb0 = bkv * spn * (R)a.inv_day_t;
-    pb1 = bkt * ((R)1 - spn * c4) * (R)a.inv_day_t;
-    pb2 = bkt * spn * c4 * (R)a.inv_day_t;
-    const R bte = te > t_strat ? bteq : (R)0;
-    pb3 = -s2 * pk * bte;
-    pb4 = -c2 * lpn * pk * bte;
-    // d te / d pn = (pk / pn) (kappa tpot - dtheta_z cos^2); pn = sf ps / p0
-    const R dte = pk / pn * (kap * tpot - (R)a.dtheta_z_t * c2);
-    bps_l = bte * dte * sf * (R)1.0e-5;
+    const R spn = sp * (R)a.inv_1msb_t, w = spn * c4 * bkt;
+    pb0 += bkv * spn * inv_day;
+    pb1 += (bkt - w) * inv_day;
+    pb2 += w * inv_day;
+    const R bte = te > t_strat ? bteq : (R)0, pt = pk * bte;
+    pb3 -= s2 * pt;
+    pb4 -= c2 * lpn * pt;
+    // d te / d ps = (pk / ps) (kappa tpot - dtheta_z cos^2)
+    bps += pt * (kap * tpot - dth);
   }
-  const R glb_c = wsum(act ? glb : (R)0), gtb_c = wsum(act ? gtb : (R)0);
-  const R bps_c = wsum(bps_l), bpsp_c = wsum(bpsp_l);
-  const R p0 = wsum(pb0), p1 = wsum(pb1), p2 = wsum(pb2), p3 = wsum(pb3), p4 = wsum(pb4);
-  if (act) {
-    const R rc = (R)1 / (R)a.cosj[j];
-    a.bu[x] = (T)bu;
-    a.bv[x] = (T)bv;
-    a.bt[x] = (T)bt;
-    a.bup[x] = (T)bup;
-    a.bvp[x] = (T)bvp;
-    a.btp[x] = (T)btp;
-    a.bvor[x] = (T)bvor;
-    a.bdiv[x] = (T)bdiv;
-    a.btl[x] = (T)(btl * rc);
-    a.btt[x] = (T)(btt * rc);
+  const R sums[8] = {glb, gtb, bps * s_col[bc][2], bpsp, pb0, pb1, pb2, pb3};
+  R tot = column_sum8(sums, lane), p4 = column_sum(pb4);
+  if (colv) {  // lane 4 v + c holds total v of column c
+    if (lq == 0) a.bgl[col] = (T)(tot * rc);
+    else if (lq == 1) a.bgt[col] = (T)(tot * rc);
+    else if (lq == 2) a.bps[col] = (T)((R)a.seed_ps[col] + tot);
+    else if (lq == 3) a.bpsp[col] = (T)(tot + (R)a.sc[SC_MPSP_BAR] * Wc);
   }
-  if (colv && lane == 0) {
-    const R rc = (R)1 / (R)a.cosj[j];
-    a.bps[col] = (T)((R)a.seed_ps[col] + bps_c);
-    a.bpsp[col] = (T)(bpsp_c + (R)a.sc[SC_MPSP_BAR] * Wc);
-    a.bgl[col] = (T)(glb_c * rc);
-    a.bgt[col] = (T)(gtb_c * rc);
-  }
-  if (lane == 0) {
-    pw[wid][0] = colv ? (double)p0 : 0.0;
-    pw[wid][1] = colv ? (double)p1 : 0.0;
-    pw[wid][2] = colv ? (double)p2 : 0.0;
-    pw[wid][3] = colv ? (double)p3 : 0.0;
-    pw[wid][4] = colv ? (double)p4 : 0.0;
-  }
+  tot += __shfl_xor_sync(FULL, tot, 1);
+  tot += __shfl_xor_sync(FULL, tot, 2);
+  p4 += __shfl_xor_sync(FULL, p4, 1);
+  p4 += __shfl_xor_sync(FULL, p4, 2);
+  if (lq >= 4 && !(lane & 3)) pw[wid][lq - 4] = (double)tot;
+  if (lane == 0) pw[wid][4] = (double)p4;
   __syncthreads();
-  if (threadIdx.x < 5) {
-    double sum = 0.0;
-    for (int w = 0; w < 8; w++) sum += pw[w][threadIdx.x];
-    a.ppart[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = sum;
+  if (threadIdx.x < 5) a.ppart[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = pw[0][threadIdx.x] + pw[1][threadIdx.x];
+}
+
+template <typename T>
+int launch_hs_column_adjoint(const ColAdjArgs<T>& a, const VertT<T>* vt, int blocks, cudaStream_t st) {
+  switch ((a.nd + 7) / 8) {
+    case 1: k_hs_column_adjoint<T, 1><<<blocks, 64, 0, st>>>(a, vt); break;
+    case 2: k_hs_column_adjoint<T, 2><<<blocks, 64, 0, st>>>(a, vt); break;
+    case 3: k_hs_column_adjoint<T, 3><<<blocks, 64, 0, st>>>(a, vt); break;
+    default: k_hs_column_adjoint<T, 4><<<blocks, 64, 0, st>>>(a, vt); break;
   }
+  JG_CUDA(cudaGetLastError());
+  return JGCM_OK;
 }
 
 // one block per parameter
@@ -705,7 +770,7 @@ int work_alloc(jgcm_model* md, AdjWork* w) {
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const int G = m->nlat * m->nlon;
   w->nb_col = (int)((grid_elems(m, nd) + 255) / 256);  // block partials: a thread per grid point
-  w->nb_adj = (G + 7) / 8;      // one warp per column
+  w->nb_adj = (G + 7) / 8;      // 8 columns per block
   const size_t gtot = 6 * al(G1) + 10 * al(GL);
   const size_t stot = 4 * al(S1) + 15 * al(SL);
   const size_t dtot = al(SC_N * 8) + al((size_t)(std::max(w->nb_col, w->nb_adj) + 8) * 8) +
@@ -924,7 +989,7 @@ int adjoint_step(jgcm_model* md, AdjWork* w, const StateBuf* x0, const StateBuf*
   }
   // ... and the alpha operators (vor, div from u cos, v cos) -> du, dv
   {
-    dim3 ga((m->nh * nd + 255) / 256, N + 1);
+    dim3 ga((m->nh * nd + 63) / 64, N + 1);
     JG_CUDA(launch_pdl(k_alpha_adjoint<T>, ga, 256, 0, st, (const V*)w->b_dvor, (const V*)w->b_ddiv, (V*)md->fbuf, tb, N, ns, nlat,
                                             nlon, nd));
     JG_CUDA(cudaGetLastError());
@@ -1027,7 +1092,7 @@ int adjoint_step(jgcm_model* md, AdjWork* w, const StateBuf* x0, const StateBuf*
     ca.inv_grav = 1.0 / md->P.grav;
     col_adj_consts<T>(ca);
   }
-  k_hs_column_adjoint<T><<<w->nb_adj, 256, 0, st>>>(ca, md->d_vc);
+  JG_TRY(launch_hs_column_adjoint<T>(ca, (const VertT<T>*)md->d_vt, w->nb_adj, st));
   JG_CUDA(launch_pdl(k_fold_params, 5, 256, 0, st, w->ppart, w->nb_adj, w->pbar));
   JG_CUDA(cudaGetLastError());
   // 6. the gradients' syntheses reversed, then Compute_Gradient_Cos! transposed

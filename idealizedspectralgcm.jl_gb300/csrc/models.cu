@@ -3777,12 +3777,14 @@ __device__ __forceinline__ void lf_adj(int init, R Dt, R rob, R d, R f, R qnb, R
   }
 }
 
+// One warp per (m, n) and component, four to a block: the real and imaginary parts are independent (T42L20 FP64
+// with both on one warp, eight pairs to a block: 124 blocks of long chains, 33 us; 29 so).
 template <typename T>
-__global__ void __launch_bounds__(256) k_hs_implicit_adjoint(AdjArgs<T> a) {
+__global__ void __launch_bounds__(128) k_hs_implicit_adjoint(AdjArgs<T> a) {
   pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
   using R = T;
   const int lane = threadIdx.x & 31;
-  const int pid = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), pid = w >> 1, comp = w & 1;
   if (pid >= a.npairs) return;  // whole warp
   const int2 mn = a.pairs[pid];
   const int m = mn.x, n = mn.y, nd = a.nd;
@@ -3791,73 +3793,71 @@ __global__ void __launch_bounds__(256) k_hs_implicit_adjoint(AdjArgs<T> a) {
   auto ld = [&](const V2<T>* p, int comp) -> R { return act ? (R)(comp ? p[s].y : p[s].x) : (R)0; };
   const R rob = (R)a.rob_t, Dt = (R)a.dt, d = (R)a.damping[row], f = (R)a.dfac[row], xi = (R)a.xi_t;
   const R rpsr = (R)a.rpsr_t, xipsr = (R)a.xipsr_t, eig = (R)a.eig_t[row];
-  for (int comp = 0; comp < 2; comp++) {  // real and imaginary parts are independent
-    R dvb, vpb, vcb, ddb2, dpb, dcb, dtb2, tpb, tcb;
-    lf_adj<R>(a.init_step, Dt, rob, d, f, ld(a.vn_b, comp), ld(a.vc_b, comp), dvb, vpb, vcb);
-    lf_adj<R>(a.init_step, Dt, rob, d, f, ld(a.dn_b, comp), ld(a.dc_b, comp), ddb2, dpb, dcb);
-    lf_adj<R>(a.init_step, Dt, rob, d, f, ld(a.tn_b, comp), ld(a.tc_b, comp), dtb2, tpb, tcb);
-    R dlb2 = 0, lpb = 0, lcb = 0;
-    {
-      const R lnb = comp ? (R)a.ln_b[row].y : (R)a.ln_b[row].x, lcbo = comp ? (R)a.lc_b[row].y : (R)a.lc_b[row].x;
-      lf_adj<R>(a.init_step, Dt, rob, (R)0, (R)1, lnb, lcbo, dlb2, lpb, lcb);
+  R dvb, vpb, vcb, ddb2, dpb, dcb, dtb2, tpb, tcb;
+  lf_adj<R>(a.init_step, Dt, rob, d, f, ld(a.vn_b, comp), ld(a.vc_b, comp), dvb, vpb, vcb);
+  lf_adj<R>(a.init_step, Dt, rob, d, f, ld(a.dn_b, comp), ld(a.dc_b, comp), ddb2, dpb, dcb);
+  lf_adj<R>(a.init_step, Dt, rob, d, f, ld(a.tn_b, comp), ld(a.tc_b, comp), dtb2, tpb, tcb);
+  R dlb2 = 0, lpb = 0, lcb = 0;
+  {
+    const R lnb = comp ? (R)a.ln_b[row].y : (R)a.ln_b[row].x, lcbo = comp ? (R)a.lc_b[row].y : (R)a.lc_b[row].x;
+    lf_adj<R>(a.init_step, Dt, rob, (R)0, (R)1, lnb, lcbo, dlb2, lpb, lcb);
+  }
+  // dtt2 = dtt1 + xi dtmp_b, dl2 = dl1 + xi/ps_ref dps_b, (dps_b, dtmp_b) = LPT(ddiv2)
+  R dtt1b = dtb2, dl1b = dlb2;
+  const R dtmpb = xi * dtb2, dpsb = xipsr * dlb2;
+  R ddiv2b = ddb2 + matT<R>(a.Apt, dtmpb, lane, nd) + (act ? (R)a.spt[lane] * dpsb : (R)0);
+  // ddiv2 = W_n ddiv1 (n <= N)
+  R ddiv1b = ddiv2b;
+  if (n <= a.N) {
+    const double* W = a.W + (size_t)n * nd * nd;  // W[k][c] at c*nd + k: W^T[k][c] = W[c][k] at k*nd + c
+    R y = 0;
+    for (int c = 0; c < nd; c++) {
+      R xc = __shfl_sync(FULL, ddiv2b, c);
+      if (act) y += (R)W[(size_t)lane * nd + c] * xc;
     }
-    // dtt2 = dtt1 + xi dtmp_b, dl2 = dl1 + xi/ps_ref dps_b, (dps_b, dtmp_b) = LPT(ddiv2)
-    R dtt1b = dtb2, dl1b = dlb2;
-    const R dtmpb = xi * dtb2, dpsb = xipsr * dlb2;
-    R ddiv2b = ddb2 + matT<R>(a.Apt, dtmpb, lane, nd) + (act ? (R)a.spt[lane] * dpsb : (R)0);
-    // ddiv2 = W_n ddiv1 (n <= N)
-    R ddiv1b = ddiv2b;
-    if (n <= a.N) {
-      const double* W = a.W + (size_t)n * nd * nd;  // W[k][c] at c*nd + k: W^T[k][c] = W[c][k] at k*nd + c
-      R y = 0;
-      for (int c = 0; c < nd; c++) {
-        R xc = __shfl_sync(FULL, ddiv2b, c);
-        if (act) y += (R)W[(size_t)lane * nd + c] * xc;
-      }
-      ddiv1b = act ? y : (R)0;
+    ddiv1b = act ? y : (R)0;
+  }
+  // ddiv1 = ddiv - eig (A_geo t2 + hk l2)
+  const R gb = -eig * ddiv1b;
+  const R t2b = matT<R>(a.Ageo, gb, lane, nd);
+  R hdot = act ? (R)a.hk[lane] * ddiv1b : (R)0;
+  for (int o = 16; o > 0; o >>= 1) hdot += __shfl_xor_sync(FULL, hdot, o);
+  const R l2b = -eig * hdot;
+  // t2 = tp - tc + xi dtt1, l2 = lp - lc + xi dl1
+  tpb += t2b;
+  tcb -= t2b;
+  dtt1b += xi * t2b;
+  lpb += l2b;
+  lcb -= l2b;
+  dl1b += xi * l2b;
+  // dtt1 = dtt + dtmp_a, dl1 = dl + dps_a / ps_ref, (dps_a, dtmp_a) = LPT(div_p - div_c)
+  const R qb = matT<R>(a.Apt, dtt1b, lane, nd) + (act ? (R)a.spt[lane] * (rpsr * dl1b) : (R)0);
+  dpb += qb;
+  dcb -= qb;
+  auto st = [&](V2<T>* p, R v) {
+    if (act) {
+      if (comp) p[s].y = (T)v;
+      else p[s].x = (T)v;
     }
-    // ddiv1 = ddiv - eig (A_geo t2 + hk l2)
-    const R gb = -eig * ddiv1b;
-    const R t2b = matT<R>(a.Ageo, gb, lane, nd);
-    R hdot = act ? (R)a.hk[lane] * ddiv1b : (R)0;
-    for (int o = 16; o > 0; o >>= 1) hdot += __shfl_xor_sync(FULL, hdot, o);
-    const R l2b = -eig * hdot;
-    // t2 = tp - tc + xi dtt1, l2 = lp - lc + xi dl1
-    tpb += t2b;
-    tcb -= t2b;
-    dtt1b += xi * t2b;
-    lpb += l2b;
-    lcb -= l2b;
-    dl1b += xi * l2b;
-    // dtt1 = dtt + dtmp_a, dl1 = dl + dps_a / ps_ref, (dps_a, dtmp_a) = LPT(div_p - div_c)
-    const R qb = matT<R>(a.Apt, dtt1b, lane, nd) + (act ? (R)a.spt[lane] * (rpsr * dl1b) : (R)0);
-    dpb += qb;
-    dcb -= qb;
-    auto st = [&](V2<T>* p, R v) {
-      if (act) {
-        if (comp) p[s].y = (T)v;
-        else p[s].x = (T)v;
-      }
-    };
-    st(a.dvor_b, dvb);
-    st(a.ddiv_b, ddiv1b);
-    st(a.dt_b, dtt1b);
-    st(a.vp_b, vpb);
-    st(a.vcin_b, vcb);
-    st(a.dp_b, dpb);
-    st(a.dcin_b, dcb);
-    st(a.tp_b, tpb);
-    st(a.tcin_b, tcb);
-    if (lane == 0) {
-      if (comp) {
-        a.dl_b[row].y = (T)dl1b;
-        a.lp_b[row].y = (T)lpb;
-        a.lcin_b[row].y = (T)lcb;
-      } else {
-        a.dl_b[row].x = (T)dl1b;
-        a.lp_b[row].x = (T)lpb;
-        a.lcin_b[row].x = (T)lcb;
-      }
+  };
+  st(a.dvor_b, dvb);
+  st(a.ddiv_b, ddiv1b);
+  st(a.dt_b, dtt1b);
+  st(a.vp_b, vpb);
+  st(a.vcin_b, vcb);
+  st(a.dp_b, dpb);
+  st(a.dcin_b, dcb);
+  st(a.tp_b, tpb);
+  st(a.tcin_b, tcb);
+  if (lane == 0) {
+    if (comp) {
+      a.dl_b[row].y = (T)dl1b;
+      a.lp_b[row].y = (T)lpb;
+      a.lcin_b[row].y = (T)lcb;
+    } else {
+      a.dl_b[row].x = (T)dl1b;
+      a.lp_b[row].x = (T)lpb;
+      a.lcin_b[row].x = (T)lcb;
     }
   }
 }
@@ -3971,7 +3971,7 @@ int si_adjoint_launch(jgcm_model* md, const void* const* obar, void* const* ibar
     a.ps_ref = md->P.ps_ref;
     a.robert = md->P.robert_coef;
     adj_consts<T>(a, tables<T>(m).eig);
-    return launch_pdl(k_hs_implicit_adjoint<T>, dim3((md->npairs + 7) / 8), dim3(256), 0, st, a);
+    return launch_pdl(k_hs_implicit_adjoint<T>, dim3((md->npairs + 1) / 2), dim3(128), 0, st, a);
   };
   JG_CUDA(is_fp64(m) ? launch(double()) : launch(float()));
   mark(st);
@@ -4076,7 +4076,7 @@ extern "C" int jgcm_model_semi_implicit_step_adjoint(jgcm_model* md, const doubl
     a.ps_ref = md->P.ps_ref;
     a.robert = md->P.robert_coef;
     adj_consts<T>(a, tables<T>(m).eig);
-    k_hs_implicit_adjoint<T><<<(md->npairs + 7) / 8, 256, 0, st>>>(a);
+    k_hs_implicit_adjoint<T><<<(md->npairs + 1) / 2, 128, 0, st>>>(a);
   };
   if (is_fp64(m)) launch(double());
   else launch(float());

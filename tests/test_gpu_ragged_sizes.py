@@ -9,6 +9,7 @@ import pytest
 
 from jgcm import configs
 from test_gpu_models import MIXED_TOL, _compare
+from test_hs_adjoint import _rand_like, _rms
 from test_gpu_transforms import TOL, _grid, _meshes, _spec
 
 pytestmark = pytest.mark.gpu
@@ -79,6 +80,37 @@ def test_held_suarez_steps(jg, orc, N, nlat, nlon, nd, members, prec, tol):
     for e in {0, members - 1}:
         one.copy_member(0, ens, e)
         _compare(one, omod, "held_suarez", tol)
+
+
+# the step adjoint's own tolerances (tests/test_hs_adjoint.py, ten levels); FP32 x sqrt(32 / 10) for the
+# roundings of up to 32 levels' sums
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 2e-4 * 1.8)])
+@pytest.mark.parametrize("N,nlat,nlon,nd", [(21, 36, 64, 3), (21, 32, 64, 8), (21, 32, 64, 9), (31, 48, 128, 20),
+                                            (21, 32, 64, 25), (21, 32, 64, 32)])
+def test_step_adjoint_levels(jg, orc, N, nlat, nlon, nd, prec, tol):
+    """Every number of levels per lane of the reverse column kernel, its first and last level counts, and the
+    transposed alpha operators at sizes that leave a ragged last block."""
+    params = dict(configs.PARAMS["hs_t21l10"], dt=900)
+    gm, om = _meshes(jg, orc, N, nlat, nlon, nd, prec)
+    omod = orc.Model(om, params)
+    configs.init_held_suarez(orc, om, omod)
+    configs.add_hs_flow(orc, om, omod)
+    orc.set_state(omod, orc.get_state(omod))
+    omod.step(3)
+    fields, _ = orc.get_state(omod)
+    orc.set_state(omod, (fields, False))
+    rng = np.random.default_rng(21)
+    ybar = {k: _rand_like(rng, v, 1.0 / _rms(v)) for k, v in fields.items()}
+    xb_o, pb_o = orc.HS_Step_Adjoint(omod, ybar)
+    gmod = jg.Model(gm, params)
+    for k in orc.STATE_FIELDS:
+        gmod.set(k, fields[k])
+    gmod.update_init_step()
+    xb_g, pb_g = jg.HS_Step_Adjoint(gmod, ybar)
+    for k in orc.STATE_FIELDS:
+        assert configs.rel_l2(xb_g[k], xb_o[k]) < tol, k
+    for p, x, y in zip(orc.HS_PARAMS, pb_g, pb_o):
+        assert abs(x - y) <= tol * abs(y) + 1e-30, p
 
 
 def _shifted(a):
