@@ -920,6 +920,317 @@ __global__ void __launch_bounds__(256) k_hs_implicit(ImplArgs<T> a, const VertT<
     }
 }
 
+// The same correction for launches of many (mode, member) columns: a warp takes four of them, 8 lanes each with NL =
+// ceil(nd / 8) consecutive levels (lane 4 l + c: levels l NL ... of column c), so that 32 - nd idle lanes, five-step
+// scans and two exchanges per wave-matrix term serve one column no longer.  Columns follow one another members first:
+// a warp's share a mode, and so its matrix, where the members are a multiple of four.  Global memory is read and
+// written in the fields' order (element lane + 32 i of the four columns' levels), where the leapfrogs run, too; what
+// the vertical algebra takes and gives goes through shared memory.
+// FP32 alone: bound by the pair products (60 instructions a term) at half its issue rate, against 41.6 M instructions
+// of the kernel above (25.5 M here) at T42L20 with 32 members: 55 -> 45 us, 128 members of T21L20 59 -> 47.
+template <typename R, int NL>
+struct ColLevels {  // levels of a column over the 8 lanes lane, lane ^ 4, ^ 8, ^ 16; every lane takes part
+  static __device__ __forceinline__ R sum(const R (&x)[NL]) {
+    R s = x[0];
+#pragma unroll
+    for (int i = 1; i < NL; i++) s += x[i];
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) s += __shfl_xor_sync(FULL, s, o);
+    return s;
+  }
+  static __device__ __forceinline__ void above(const R (&x)[NL], R (&y)[NL], int lane) {  // y_k = sum_{r < k} x_r
+    R s = x[0];
+#pragma unroll
+    for (int i = 1; i < NL; i++) s += x[i];
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      const R z = __shfl_up_sync(FULL, s, o);
+      if (lane >= o) s += z;
+    }
+    s = __shfl_up_sync(FULL, s, 4);
+    y[0] = lane < 4 ? (R)0 : s;
+#pragma unroll
+    for (int i = 1; i < NL; i++) y[i] = y[i - 1] + x[i - 1];
+  }
+  static __device__ __forceinline__ void below(const R (&x)[NL], R (&y)[NL], int lane) {  // y_k = sum_{r > k} x_r
+    R s = x[0];
+#pragma unroll
+    for (int i = 1; i < NL; i++) s += x[i];
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      const R z = __shfl_down_sync(FULL, s, o);
+      if (lane + o < 32) s += z;
+    }
+    s = __shfl_down_sync(FULL, s, 4);
+    y[NL - 1] = lane >= 28 ? (R)0 : s;
+#pragma unroll
+    for (int i = NL - 2; i >= 0; i--) y[i] = y[i + 1] + x[i + 1];
+  }
+  static __device__ __forceinline__ R prev(const R (&x)[NL], int i, int lane) {  // value of level k - 1 (0 at k = 0)
+    if (i > 0) return x[i - 1];
+    const R z = __shfl_up_sync(FULL, x[NL - 1], 4);
+    return lane < 4 ? (R)0 : z;
+  }
+};
+
+// Linear_Ps_T_δdiv! (Semi_Implicit.jl:271-341), one component: dtt_k, and the column total tx = -dps
+template <typename R, int NL>
+__device__ __forceinline__ void linear_ps_t_cols(const VertR<R>& vr, int k0, int lane, int nd, R kappa, const R (&d)[NL],
+                                                 R& tx, R (&dtt)[NL]) {
+  using L = ColLevels<R, NL>;
+  R dm[NL], ex[NL], mdh[NL];
+#pragma unroll
+  for (int i = 0; i < NL; i++) dm[i] = k0 + i < nd ? d[i] * vr.dpr[k0 + i] : (R)0;
+  L::above(dm, ex, lane);
+  tx = L::sum(dm);
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    const int k = min(k0 + i, nd - 1);
+    dtt[i] = -kappa * vr.tref[k] * (ex[i] * vr.dlnp[k] + dm[i] * vr.dlnpp[k]) * vr.rdpr[k];
+    // M_{k+1/2} (k <= nd-2) times (t_ref[k+1] - t_ref[k])
+    mdh[i] = k0 + i + 1 < nd ? (tx * vr.bk1[k] - (ex[i] + dm[i])) * vr.tdh[k] : (R)0;
+  }
+#pragma unroll
+  for (int i = 0; i < NL; i++)
+    dtt[i] -= (R)0.5 * (mdh[i] + L::prev(mdh, i, lane)) * vr.rdpr[min(k0 + i, nd - 1)];
+}
+
+constexpr int IMPL_CW = 4;  // warps per block
+
+template <int NL>
+__global__ void __launch_bounds__(32 * IMPL_CW) k_hs_implicit_cols(const __grid_constant__ ImplArgs<float> a,
+                                                                   const VertT<float>* __restrict__ vtp) {
+  using R = float;
+  using L = ColLevels<R, NL>;
+  using V = V2<R>;
+  __shared__ VertR<R> vr;
+  __shared__ V buf[IMPL_CW][32 * NL];
+  const int nd = a.nd;
+  stage_vert<R>(*vtp, nd, vr);  // constants: staged before the dependency wait
+  __syncthreads();
+  pdl_wait();  // programmatic dependent launch: the predecessor's output is complete
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c0 = (blockIdx.x * IMPL_CW + w) * 4, ncol = a.npairs * a.ne;
+  if (c0 >= ncol) return;  // whole warp; no block barrier follows
+  V* B = buf[w];
+  // this lane's column in the vertical algebra (lane & 3) ...
+  const int cc = min(c0 + (lane & 3), ncol - 1), pid = cc / a.ne, e = cc - pid * a.ne, k0 = (lane >> 2) * NL;
+  const int2 mn = a.pairs[pid];
+  const int n = mn.y;
+  const size_t row = (size_t)mn.x * (a.ns + 1) + n, s1 = row * a.ne + e;
+  const R eig = a.eig_t[row], damp = a.damping[row], dfac = a.dfac[row];
+  // ... and its elements in the fields' order: level gk[i] of column gc[i], at index s[i]
+  const unsigned long long base = row * a.L + (size_t)e * nd;
+  unsigned long long s[NL];
+  int gc[NL];
+  bool on[NL];
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    const int t = lane + 32 * i, c = min(t / nd, 3);
+    gc[i] = c;
+    on[i] = t < 4 * nd && c0 + c < ncol;
+    const unsigned long long bq = __shfl_sync(FULL, base, c);
+    s[i] = bq + (on[i] ? t - c * nd : 0);
+  }
+  auto ld = [&](const V* p, V(&x)[NL]) {
+#pragma unroll
+    for (int i = 0; i < NL; i++) {
+      x[i].x = x[i].y = 0;
+      if (on[i]) x[i] = p[s[i]];
+    }
+  };
+  // between the fields' order and the columns' levels: element t = c nd + k of the buffer
+  const int bo = (lane & 3) * nd + k0;
+  auto to_cols = [&](const V(&x)[NL], R(&yx)[NL], R(&yy)[NL]) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NL; i++) B[lane + 32 * i] = x[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NL; i++) {
+      V v;
+      v.x = v.y = 0;
+      if (k0 + i < nd) v = B[bo + i];
+      yx[i] = v.x;
+      yy[i] = v.y;
+    }
+  };
+  auto to_fields = [&](const R(&yx)[NL], const R(&yy)[NL], V(&x)[NL]) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NL; i++)
+      if (k0 + i < nd) {
+        V v;
+        v.x = yx[i];
+        v.y = yy[i];
+        B[bo + i] = v;
+      }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < NL; i++) x[i] = B[lane + 32 * i];
+  };
+  V divg[NL], tg[NL], p[NL], q[NL], x[NL];
+  ld(a.div_p, p);
+  ld(a.div_c, q);
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    x[i].x = p[i].x - q[i].x;
+    x[i].y = p[i].y - q[i].y;
+  }
+  ld(a.dtend, tg);
+  ld(a.t_p, p);
+  ld(a.t_c, q);
+  ld(a.ddiv, divg);
+  const V l0 = a.dlnps[s1], lp = a.lnps_p[s1], lc0 = a.lnps_c[s1];
+  const R xi = a.xi_t, kap = a.kap_t, Rg = a.rg_t;
+  // Adjust_δlnps_δt_δdiv! :360-404
+  R ux[NL], uy[NL], ex[NL], ey[NL], txk[NL], tyk[NL], tx, ty;
+  to_cols(x, ux, uy);
+  to_cols(tg, txk, tyk);  // δT
+  linear_ps_t_cols<R, NL>(vr, k0, lane, nd, kap, ux, tx, ex);
+  linear_ps_t_cols<R, NL>(vr, k0, lane, nd, kap, uy, ty, ey);
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    txk[i] += ex[i];
+    tyk[i] += ey[i];
+    x[i].x = p[i].x - q[i].x;
+    x[i].y = p[i].y - q[i].y;
+  }
+  R dlx = l0.x - tx * a.rpsr_t, dly = l0.y - ty * a.rpsr_t;
+  const R l2x = lp.x - lc0.x + xi * dlx, l2y = lp.y - lc0.y + xi * dly;
+  to_cols(x, ux, uy);
+  R tmx[NL], tmy[NL];
+#pragma unroll
+  for (int i = 0; i < NL; i++) {  // t2, and Linear_Geopot_δt! :213-241
+    const R dh = k0 + i < nd ? vr.dlnp[k0 + i] : (R)0;
+    ux[i] += xi * txk[i];
+    uy[i] += xi * tyk[i];
+    tmx[i] = Rg * (ux[i] * dh);
+    tmy[i] = Rg * (uy[i] * dh);
+  }
+  L::below(tmx, ex, lane);  // Φ_{k+1/2}
+  L::below(tmy, ey, lane);
+  R dx[NL], dy[NL];
+  to_cols(divg, dx, dy);
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    const int k = min(k0 + i, nd - 1);
+    const R df = vr.dlnpp[k], hk = vr.hk[k];
+    dx[i] -= eig * (ex[i] + Rg * (ux[i] * df) + hk * l2x);
+    dy[i] -= eig * (ey[i] + Rg * (uy[i] * df) + hk * l2y);
+  }
+  // wave-matrix solve, n <= N only (Implicit_Correction! :486-497): the products of row k in the order of c.  A lane
+  // whose levels pass nd takes the last NL rows, `off` of them not its own.
+  {
+    const int kr = min(k0, nd - NL), off = k0 - kr;
+    const size_t wo = (size_t)min(n, a.N) * nd * nd + kr;
+    R sx[NL] = {}, sy[NL] = {}, cx[NL] = {}, cy[NL] = {};
+    const float2* wp = a.W2 + wo;
+    for (int l = 0; l * NL < nd; l++) {
+      const int from = (lane & 3) + 4 * l;
+#pragma unroll
+      for (int q = 0; q < NL; q++) {
+        const R bx = __shfl_sync(FULL, dx[q], from), by = __shfl_sync(FULL, dy[q], from);
+        if (l * NL + q < nd) {
+#pragma unroll
+          for (int i = 0; i < NL; i++) {
+            const float2 wv = wp[i];
+            ds_add_prod(sx[i], cx[i], bx, wv.x, wv.y);
+            ds_add_prod(sy[i], cy[i], by, wv.x, wv.y);
+          }
+          wp += nd;
+        }
+      }
+    }
+    if (n <= a.N) {
+#pragma unroll
+      for (int i = 0; i < NL; i++) {
+        dx[i] = dy[i] = 0;
+#pragma unroll
+        for (int q = i; q < NL; q++)
+          if (q == i + off) {
+            dx[i] = sx[q] + cx[q];
+            dy[i] = sy[q] + cy[q];
+          }
+      }
+    }
+  }
+  linear_ps_t_cols<R, NL>(vr, k0, lane, nd, kap, dx, tx, ex);
+  linear_ps_t_cols<R, NL>(vr, k0, lane, nd, kap, dy, ty, ey);
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    txk[i] += xi * ex[i];
+    tyk[i] += xi * ey[i];
+  }
+  dlx -= a.xipsr_t * tx;
+  dly -= a.xipsr_t * ty;
+  // damping + leapfrog
+  const R rob = a.rob_t;
+  const int ini = a.init_step, Dt = a.dt;
+  R dg[NL], fg[NL];
+#pragma unroll
+  for (int i = 0; i < NL; i++) {
+    dg[i] = __shfl_sync(FULL, damp, gc[i]);
+    fg[i] = __shfl_sync(FULL, dfac, gc[i]);
+  }
+  auto step = [&](V(&dq)[NL], const V* fp, const V* fc, V* on_, V* oc) {
+    ld(fp, p);  // (read again where the algebra took them: held through the products they cost a block per SM)
+    ld(fc, q);
+#pragma unroll
+    for (int i = 0; i < NL; i++) {
+      V qn;
+      lf<R>(ini, Dt, rob, dg[i], fg[i], dq[i].x, p[i].x, q[i].x, qn.x);
+      lf<R>(ini, Dt, rob, dg[i], fg[i], dq[i].y, p[i].y, q[i].y, qn.y);
+      if (on[i]) {
+        on_[s[i]] = qn;
+        oc[s[i]] = q[i];
+      }
+    }
+  };
+  to_fields(dx, dy, divg);
+  step(divg, a.div_p, a.div_c, a.div_n, a.div_c);
+  to_fields(txk, tyk, tg);
+  step(tg, a.t_p, a.t_c, a.t_n, a.t_c);
+  ld(a.dvor, tg);
+  step(tg, a.vor_p, a.vor_c, a.vor_n, a.vor_c);
+  if (lane < 4 && c0 + lane < ncol) {  // lnps: leapfrog without damping (d = 0, f = 1)
+    V ln, lc = lc0;
+    lf<R>(ini, Dt, rob, (R)0, (R)1, dlx, lp.x, lc.x, ln.x);
+    lf<R>(ini, Dt, rob, (R)0, (R)1, dly, lp.y, lc.y, ln.y);
+    a.lnps_n[s1] = ln;
+    a.lnps_c[s1] = lc;
+  }
+  // passive tracers: damping and the filtered leapfrog of T (Time_Integrator.jl:58-101)
+  if (a.nq) {
+    const unsigned long long bq = row * a.LQ + (size_t)e * a.nq * nd;
+    for (int iq = 0; iq < a.nq; iq++) {
+#pragma unroll
+      for (int i = 0; i < NL; i++) {
+        const unsigned long long q0 = __shfl_sync(FULL, bq, gc[i]);
+        s[i] = q0 + (size_t)iq * nd + (on[i] ? lane + 32 * i - gc[i] * nd : 0);
+      }
+      ld(a.dq, tg);
+      step(tg, a.q_p, a.q_c, a.q_n, a.q_c);
+    }
+  }
+}
+
+// From 108 columns per SM on (T42L20: 8 members 21 -> 23 us, 16 members 33 -> 31; 8 members of T63L20 34 -> 31,
+// 32 of T21L20 equal)
+inline bool impl_cols_pay(const jgcm_model* md) {
+  return (size_t)md->npairs * md->ne >= (size_t)108 * md->mesh->sm_count;
+}
+
+int launch_hs_implicit_cols(const ImplArgs<float>& a, const VertT<float>* vt, cudaStream_t st) {
+  const dim3 g((unsigned)(((size_t)a.npairs * a.ne + 4 * IMPL_CW - 1) / (4 * IMPL_CW)));
+  switch ((a.nd + 7) / 8) {
+    case 1: JG_CUDA(launch_pdl(k_hs_implicit_cols<1>, g, 32 * IMPL_CW, 0, st, a, vt)); break;
+    case 2: JG_CUDA(launch_pdl(k_hs_implicit_cols<2>, g, 32 * IMPL_CW, 0, st, a, vt)); break;
+    case 3: JG_CUDA(launch_pdl(k_hs_implicit_cols<3>, g, 32 * IMPL_CW, 0, st, a, vt)); break;
+    default: JG_CUDA(launch_pdl(k_hs_implicit_cols<4>, g, 32 * IMPL_CW, 0, st, a, vt)); break;
+  }
+  return JGCM_OK;
+}
+
 // ------------------------------------------------------------------------------------------
 // Compute_Corrections! (Spectral_Dynamics.jl:30-68): FP64 sums of ps_n and of the column
 // energy (split into the Δa and Δb·ps parts so the mass correction can be applied after the
@@ -2245,15 +2556,20 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
     ia.q_n = (V*)md->spe_q[n];
   }
   // vertical algebra in the state precision (FP64 algebra on the FP32 path measured no more
-  // accurate: its error is set by FP32 storage); the wave-matrix solve is FP64 in both
+  // accurate: its error is set by FP32 storage); the wave-matrix solve to FP64 accuracy in both
   // 4 modes per block: (N+1)(N+2)/2 + N+1 modes at T42 make 248 blocks, every SM's FP64 units busy;
-  // FP64 member ensembles (from 4 members) spread the FP64 products densely over each block
-  if constexpr (std::is_same<T, float>::value)
-    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, (const VertT<T>*)md->d_vt));
-  else if (E >= 4)
-    JG_CUDA(launch_pdl(k_hs_implicit<T, T, true>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, (const VertT<T>*)md->d_vt));
-  else
-    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, dim3((md->npairs + 3) / 4, E), 128, 0, st, ia, (const VertT<T>*)md->d_vt));
+  // FP64 member ensembles (from 4 members) spread the FP64 products densely over each block, FP32 launches of
+  // many columns take four of them per warp
+  const VertT<T>* vt = (const VertT<T>*)md->d_vt;
+  const dim3 gi((md->npairs + 3) / 4, E);
+  if constexpr (std::is_same<T, float>::value) {
+    if (impl_cols_pay(md)) JG_TRY(launch_hs_implicit_cols(ia, vt, st));
+    else JG_CUDA(launch_pdl(k_hs_implicit<T, T>, gi, 128, 0, st, ia, vt));
+  } else if (E >= 4) {
+    JG_CUDA(launch_pdl(k_hs_implicit<T, T, true>, gi, 128, 0, st, ia, vt));
+  } else {
+    JG_CUDA(launch_pdl(k_hs_implicit<T, T>, gi, 128, 0, st, ia, vt));
+  }
   mark(st);
   JG_CUDA(cudaGetLastError());
   // 5. back to the grid: vor, div, u, v, T, lnps (+ ps = exp(lnps)), and the next step's gradients

@@ -59,11 +59,14 @@ def test_one_layer_steps(jg, orc, N, nlat, nlon, prec, tol):
 
 @pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", MIXED_TOL["fp32"])])
 @pytest.mark.parametrize("N,nlat,nlon,nd,members", [(21, 40, 64, 7, 1), (31, 48, 128, 13, 1), (31, 48, 128, 13, 29),
-                                                    (42, 64, 128, 20, 11), (63, 96, 256, 9, 1), (63, 96, 256, 9, 17)])
+                                                    (42, 64, 128, 20, 11), (63, 96, 256, 9, 1), (63, 96, 256, 9, 17),
+                                                    (21, 40, 64, 7, 60), (31, 48, 128, 17, 30), (21, 32, 64, 32, 61),
+                                                    (42, 64, 128, 20, 18)])
 def test_held_suarez_steps(jg, orc, N, nlat, nlon, nd, members, prec, tol):
     """Held-Suarez steps on latitude counts that are no power of two, alone and as ensembles large enough
-    for the tiled Legendre kernels, whose column tiles straddle members: the first and last members against
-    the oracle, at the step tolerances."""
+    for the tiled Legendre kernels, whose column tiles straddle members, and for the semi-implicit kernel of
+    four columns per warp (every number of levels per lane, a ragged last warp): the first and last members
+    against the oracle, at the step tolerances."""
     if prec == "fp64" and members > 1:
         members = 3
     params = configs.PARAMS["hs_t21l20"]
