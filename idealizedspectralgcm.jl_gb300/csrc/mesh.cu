@@ -94,6 +94,14 @@ __global__ void k_legendre(int N, int ns, int nlat, const double* sinth, double*
   }
 }
 
+// w as its FP32 rounding plus that of the remainder
+__global__ void k_weight_pairs(const double* __restrict__ w, float2* __restrict__ p, int n) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const float h = (float)w[j];
+  p[j] = make_float2(h, (float)(w[j] - (double)h));
+}
+
 // Derived kernel tables (FP64 and FP32) in [m][n][jh] / [m][n] layout.
 __global__ void k_derive3(int N, int ns, int nlat, double radius, const double* qnm, const double* dqnm,
                           const double* wts, const double* sinth, double* P, double* PW, double* CA, double* CB,
@@ -188,6 +196,7 @@ int mesh_build_tables(jgcm_mesh* m) {
   JG_CUDA(cudaMalloc(&d_status, sizeof(int)));
   JG_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), st));
   k_gauss<<<(nlat / 2 + 63) / 64, 64, 0, st>>>(nlat, m->d_sinth, m->d_wts, d_status);
+  k_weight_pairs<<<(nlat + 127) / 128, 128, 0, st>>>(m->d_wts, (float2*)(m->d_wts + nlat), nlat);
   JG_CUDA(cudaGetLastError());
   int nt = (N + 1) * nlat;
   k_legendre<<<(nt + 127) / 128, 128, 0, st>>>(N, ns, nlat, m->d_sinth, m->d_qnm, m->d_dqnm);
@@ -325,7 +334,7 @@ extern "C" int jgcm_mesh_create(int num_fourier, int num_spherical, int nlat, in
   }
   size_t T3 = (size_t)(m->N + 1) * (m->ns + 1) * nlat;
   MCHK(cuda(cudaMalloc(&m->d_sinth, nlat * 8), "alloc"));
-  MCHK(cuda(cudaMalloc(&m->d_wts, nlat * 8), "alloc"));
+  MCHK(cuda(cudaMalloc(&m->d_wts, nlat * 16), "alloc"));  // the weights in FP64, then as FP32 pairs
   MCHK(cuda(cudaMalloc(&m->d_costh, nlat * 8), "alloc"));
   MCHK(cuda(cudaMalloc(&m->d_qnm, T3 * 8), "alloc"));
   MCHK(cuda(cudaMalloc(&m->d_dqnm, T3 * 8), "alloc"));

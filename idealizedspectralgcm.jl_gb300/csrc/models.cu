@@ -9,8 +9,9 @@
 // pointer (Time_Advance!, Dyn_Data.jl:326-364, copies instead); steady steps are captured
 // once per rotation phase as CUDA graphs and replayed.  The semi-implicit wave matrices
 // (Semi_Implicit.jl:165-180) are inverted on the device in FP64, the per-(m,n) vertical
-// solve runs in FP64 (one warp per spectral mode, lanes over levels) and the mass/energy
-// fixers (Spectral_Dynamics.jl:5-68) use deterministic FP64 reductions.
+// solve is applied to FP64 accuracy (on the FP32 path as FP32 pairs; a warp per spectral mode, or
+// four columns per warp) and the mass/energy fixers (Spectral_Dynamics.jl:5-68) use deterministic
+// reductions folded in FP64.
 #include <cmath>
 #include <cstddef>
 #include <cstdio>
@@ -140,6 +141,14 @@ __device__ __forceinline__ void ds_add_prod(float& hi, float& lo, float t, float
   lo = __fadd_rn(lo, __fmaf_rn(t, cl, pe));
 }
 
+// (h + l) times the pair (wh, wl), added to the pair (sh, sl): the leading product error-free, the cross
+// terms rounded
+__device__ __forceinline__ void ds_add_mul(float& sh, float& sl, float h, float l, float wh, float wl) {
+  const float p = __fmul_rn(h, wh), pe = __fmaf_rn(h, wh, -p);
+  ds_add(sh, sl, p);
+  sl = __fadd_rn(sl, __fadd_rn(pe, __fmaf_rn(h, wl, __fmul_rn(l, wh))));
+}
+
 // Mercator series of log(1 + d) for |d| <= 2^-12: the remainder after the d^5 term is below
 // |d|^6 / 6 < 2^-62 |d|, under half an ulp of the sum; larger |d| take the library's log
 __device__ __forceinline__ double log_near_one(double f) {
@@ -182,6 +191,7 @@ struct HSColArgs {
   // the physics constants in T, formed on the host with the kernel's own T arithmetic (no FP64 ->
   // FP32 conversion per thread: those run on the FP64 pipe)
   T sb, R, kap, cp_t, rcp, kv0, ka, ks, kt0, dTy, dthz, kappa_t;
+  float cp_hi, cp_lo;  // cp as an FP32 pair
 };
 
 template <typename T>
@@ -199,6 +209,8 @@ void hs_col_consts(HSColArgs<T>& a) {
   a.dTy = (T)a.dT_y;
   a.dthz = (T)a.dtheta_z;
   a.kappa_t = (T)a.kappa;
+  a.cp_hi = (float)a.cp;
+  a.cp_lo = (float)(a.cp - (double)a.cp_hi);
 }
 
 // S lanes per column (S = 1, 2, 4): lane s walks levels [s*len, s*len + len), len = ceil(nd/S); the
@@ -513,45 +525,61 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
       dp = dp1;
     }
   }
-  if constexpr (std::is_same<T, float>::value) {
-    col_ta = (double)ah + (double)al;
-    col_tb = (double)bh + (double)bl;
-  }
+  if (act && seg == 0) a.dlnps[c1] = HYB ? (-tot) / ps : -tot;  // grid_δlnps = grid_δps / ps (Spectral_Dynamics.jl:279)
   if constexpr (!HYB) col_e *= psp;
-  double col_ed = (double)col_e + a.cp * (col_ta + col_tb * (double)psp);
-  col_ed = seg_sum<S>(col_ed);
-  double accp = 0.0, acce = 0.0;
-  if (act && seg == 0) {
-    a.dlnps[c1] = HYB ? (-tot) / ps : -tot;  // grid_δlnps = grid_δps / ps (Spectral_Dynamics.jl:279)
-    accp = (double)psp;
-    acce = col_ed;
-  }
-  // ---- block partials for mean_ps_p and mean_energy_p (fixed order), then the member's fold;
-  // only lanes with seg = 0 hold values, so the butterfly stops at offset S (the skipped levels
-  // would add exact zeros)
+  // ---- block partials for mean ps_p and mean energy_p (fixed order), then the member's fold; only lanes with
+  // seg = 0 hold values of ps, so its butterfly stops at offset S (the skipped levels would add exact zeros).
+  // FP32 on several lanes per column (small grids): all of it as FP32 pairs up to one conversion per warp; as FP64
+  // sums its 34 instructions held the sub-partitions' FP64 pipes for 1 us at the end of the one wave of blocks
+  // (one member of T42L20: step 40.3 -> 39.6 us).  With one lane per column other blocks cover them, and the
+  // pairs' 130 instructions cost more (83 -> 86 us).
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if constexpr (std::is_same<T, float>::value && S > 1) {
+    float ph = __fmul_rn(bh, psp), pl = __fadd_rn(__fmaf_rn(bh, psp, -ph), __fmul_rn(bl, psp));
+    if constexpr (HYB) {
+      ds_add(ph, pl, ah);
+      pl = __fadd_rn(pl, al);
+    }
+    float eh = col_e, el = 0, qh = act && seg == 0 ? psp : 0.f, ql = 0;
+    ds_add_mul(eh, el, ph, pl, a.cp_hi, a.cp_lo);
+    auto fold = [&](float& h, float& l, int o) {
+      const float h2 = __shfl_xor_sync(FULL, h, o), l2 = __shfl_xor_sync(FULL, l, o);
+      ds_add(h, l, h2);
+      l = __fadd_rn(l, l2);
+    };
+    if (!act) eh = el = 0;
 #pragma unroll
-  for (int o = 16; o >= S; o >>= 1) {
-    accp += __shfl_xor_sync(FULL, accp, o);
-    acce += __shfl_xor_sync(FULL, acce, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = accp;
-    red[1][threadIdx.x >> 5] = acce;
+    for (int o = 1; o < 32; o <<= 1) fold(eh, el, o);
+#pragma unroll
+    for (int o = S; o < 32; o <<= 1) fold(qh, ql, o);  // (lane 1 has the energy: any lane does)
+    if (lane < 2) red[lane][wid] = (double)(lane ? eh : qh) + (double)(lane ? el : ql);
+  } else {
+    if constexpr (std::is_same<T, float>::value) {
+      col_ta = (double)ah + (double)al;
+      col_tb = (double)bh + (double)bl;
+    }
+    double acce = seg_sum<S>((double)col_e + a.cp * (col_ta + col_tb * (double)psp)), accp = 0.0;
+    if (act && seg == 0) accp = (double)psp;
+    else acce = 0.0;
+#pragma unroll
+    for (int o = 16; o >= S; o >>= 1) {
+      accp += __shfl_xor_sync(FULL, accp, o);
+      acce += __shfl_xor_sync(FULL, acce, o);
+    }
+    if (lane == 0) {
+      red[0][wid] = accp;
+      red[1][wid] = acce;
+    }
   }
   __syncthreads();
-  double vals[2] = {0, 0};
-  if (threadIdx.x == 0)
-    for (int q = 0; q < HS_CT / 32; q++) {
-      vals[0] += red[0][q];
-      vals[1] += red[1][q];
-    }
   // the block partials only: the fixer reduction, their one consumer, folds them (its last block), so
   // no grid-wide fold sits at this kernel's end
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 2) {
     const int nb = gridDim.x * gridDim.y, bid = blockIdx.y * gridDim.x + blockIdx.x;
-    double* p = a.partials + e * a.pstride;
-    p[bid] = vals[0];
-    p[(size_t)nb + bid] = vals[1];
+    double v = red[threadIdx.x][0];
+#pragma unroll
+    for (int q = 1; q < HS_CT / 32; q++) v += red[threadIdx.x][q];
+    a.partials[e * a.pstride + (size_t)threadIdx.x * nb + bid] = v;
   }
 }
 
@@ -639,8 +667,8 @@ int launch_hs_column(const HSColArgs<T>& a, const jgcm_mesh* m, int ne, int S, c
 // Semi-implicit correction (Adjust_δlnps_δt_δdiv! + Implicit_Correction!, Semi_Implicit.jl:
 // 271-513) followed by Compute_Spectral_Damping! and Filtered_Leapfrog! for vor, div, T, lnps
 // (Spectral_Dynamics.jl:313-327).  One warp per spectral mode (m,n), lane = level.  The
-// per-n solve with W_n = (I - ξ² ∇²_n D)^{-1} runs in FP64; the linearised vertical operators
-// and the time filter run in the state precision T (FP64 on the FP64 path).
+// per-n solve with W_n = (I - ξ² ∇²_n D)^{-1} is formed to FP64 accuracy; the linearised vertical
+// operators and the time filter run in the state precision T (FP64 on the FP64 path).
 template <typename T>
 struct ImplArgs {
   const V2<T>*dvor, *ddiv, *dtend, *dlnps;  // spectral tendencies from the analysis
@@ -1240,6 +1268,7 @@ struct CorrArgs {
   const T *u_n, *v_n, *t_n, *ps_n;
   V2<T>*lnps_n, *t_spec_n;
   const double* wts;
+  const float2* wts2;  // the weights as FP32 pairs
   double *partials, *scalars;  // per member: partials + e * pstride, scalars + 4 e
   T* scal_t;                   // per member: factor and correction rounded to T (for k_hs_corr_apply)
   unsigned* counter;           // a ticket per member
@@ -1474,14 +1503,6 @@ __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const Ver
   corr_finish<T>(a, e, pe + a.col_off, u, nu, ks, lane, x);
 }
 
-// (h + l) times the pair (wh, wl), added to the pair (sh, sl): the leading product error-free, the cross
-// terms rounded
-__device__ __forceinline__ void ds_add_mul(float& sh, float& sl, float h, float l, float wh, float wl) {
-  const float p = __fmul_rn(h, wh), pe = __fmaf_rn(h, wh, -p);
-  ds_add(sh, sl, p);
-  sl = __fadd_rn(sl, __fadd_rn(pe, __fmaf_rn(h, wl, __fmul_rn(l, wh))));
-}
-
 // The same sums for larger grids (member ensembles): a warp takes 32 consecutive columns of a
 // latitude row at a time, a thread one column with all its levels, and keeps the three sums to the end of
 // its columns, so the folds, the barriers and the ticket come once per block.  One block per 32 columns and
@@ -1524,7 +1545,6 @@ __global__ void __launch_bounds__(32 * CORR_WARPS) k_hs_corr_columns(CorrArgs<T>
     if (i >= a.nlon) continue;  // no warp operation in the loop
     const size_t col = (size_t)j * a.nlon + i;
     const T ps = a.ps_n[off1 + col];
-    const double w = a.wts[j];
     float kah = 0, kal = 0, kbh = 0, kbl = 0, tah = 0, tal = 0, tbh = 0, tbl = 0;  // Σ K Δa, K Δb, T Δa, T Δb
     T ka = 0, kb = 0;
     double ta = 0, tb = 0;
@@ -1572,7 +1592,7 @@ __global__ void __launch_bounds__(32 * CORR_WARPS) k_hs_corr_columns(CorrArgs<T>
       }
     }
     if constexpr (F) {
-      const float wh = (float)w, wl = (float)(w - (double)wh);
+      const float wh = a.wts2[j].x, wl = a.wts2[j].y;
       ds_add_mul(kbh, kbl, tbh, tbl, a.cp_hi, a.cp_lo);  // E = K + c_p T
       const float p = __fmul_rn(kbh, ps), pl = __fadd_rn(__fmaf_rn(kbh, ps, -p), __fmul_rn(kbl, ps));
       ds_add_mul(sh[0], sl[0], ps, 0.f, wh, wl);
@@ -1582,13 +1602,16 @@ __global__ void __launch_bounds__(32 * CORR_WARPS) k_hs_corr_columns(CorrArgs<T>
         ds_add_mul(sh[1], sl[1], kah, kal, wh, wl);
       }
     } else {
+      const double w = a.wts[j];
       sd[0] += ps * w;
       sd[1] += (ka + a.cp * ta) * w;
       sd[2] += (kb + a.cp * tb) * ps * w;
     }
   }
-  // the block's values: the butterfly over a warp's columns, then the warps in order
+  // the block's values: the butterfly over a warp's columns, then the warps in order (FP32: as pairs up to one
+  // conversion per value, the FP64 instructions of the eight warps' own had been 5 us of a wave's end)
   __shared__ double s_w[3][CORR_WARPS];
+  __shared__ float2 s_p[3][CORR_WARPS];
 #pragma unroll
   for (int v = 0; v < 3; v++) {
     if constexpr (F) {
@@ -1598,16 +1621,26 @@ __global__ void __launch_bounds__(32 * CORR_WARPS) k_hs_corr_columns(CorrArgs<T>
         ds_add(sh[v], sl[v], h2);
         sl[v] = __fadd_rn(sl[v], l2);
       }
-      sd[v] = (double)sh[v] + (double)sl[v];
+      if (lane == 0) s_p[v][ks] = make_float2(sh[v], sl[v]);
     } else {
       sd[v] = warp_sum(sd[v]);
+      if (lane == 0) s_w[v][ks] = sd[v];
     }
-    if (lane == 0) s_w[v][ks] = sd[v];
   }
   __syncthreads();
   double x = 0.0;
-  if (ks < 3)
-    for (int q = 0; q < CORR_WARPS; q++) x += s_w[ks][q];
+  if (ks < 3) {
+    if constexpr (F) {
+      float h = 0, l = 0;
+      for (int q = 0; q < CORR_WARPS; q++) {
+        ds_add(h, l, s_p[ks][q].x);
+        l = __fadd_rn(l, s_p[ks][q].y);
+      }
+      x = (double)h + (double)l;
+    } else {
+      for (int q = 0; q < CORR_WARPS; q++) x += s_w[ks][q];
+    }
+  }
   else if (ks < 5)
     x = corr_col_share(a, pe, ks - 3, u, nu, lane);
   corr_finish<T>(a, e, pe + a.col_off, u, nu, ks, lane, x);
@@ -2634,6 +2667,7 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
   ca.lnps_n = (V*)md->spe_lnps[n];
   ca.t_spec_n = (V*)md->spe_t[n];
   ca.wts = m->d_wts;
+  ca.wts2 = (const float2*)(m->d_wts + m->nlat);
   ca.partials = md->d_partials;
   ca.scalars = md->d_scalars;
   ca.scal_t = (T*)(md->d_scalars + 4 * E);
