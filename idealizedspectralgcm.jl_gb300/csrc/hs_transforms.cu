@@ -43,9 +43,21 @@ __host__ __device__ constexpr int wpitch(int nh) {
   return nh + 16 / (int)sizeof(T);
 }
 
-// grid (N/2 + 1 pairs, ceil((nd + 1) / LG) level groups, members), blockDim >= rows * LG with rows the
-// largest per-pair thread count (N + 4 for NP = 1)
-template <typename T, int NP>
+// Both values summed over the SP neighbouring lanes of an output, which take the same branches
+template <int SP, typename T>
+__device__ __forceinline__ void pair_sum(T& x, T& y) {
+  const unsigned group = ((1u << SP) - 1) << (threadIdx.x & 31 & ~(SP - 1));
+#pragma unroll
+  for (int o = 1; o < SP; o <<= 1) {
+    x += __shfl_xor_sync(group, x, o);
+    y += __shfl_xor_sync(group, y, o);
+  }
+}
+
+// grid (N/2 + 1 pairs, ceil((nd + 1) / LG) level groups, members), blockDim >= rows * LG * SP with rows the
+// largest per-pair thread count (N + 4 for NP = 1).  SP = 2 (FP64, small launches): two
+// neighbouring lanes share an output's latitudes in turns of four (hs_analysis_shape).
+template <typename T, int NP, int SP>
 __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> tb) {
   using V = V2<T>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -121,8 +133,9 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
   __syncthreads();
   // 3. one thread per (m, level) and NP total wavenumbers of one parity, n and n + 2 (NP = 2:
   //    each folded input loaded from shared memory serves both; rows r = 4 i + b, b < 2)
-  int q = threadIdx.x / LG;
-  const int l = threadIdx.x - q * LG;
+  const int h = threadIdx.x % SP;
+  int q = threadIdx.x / SP / LG;
+  const int l = threadIdx.x / SP - q * LG;
   const int Q1 = NP == 1 ? K1 : 2 * ((K1 + 3) / 4), Q2 = nm == 2 ? (NP == 1 ? K2 : 2 * ((K2 + 3) / 4)) : 0;
   if (q >= Q1 + Q2) return;
   const int s = q < Q1 ? 0 : 1;
@@ -157,7 +170,7 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
     T sr[NP], si[NP];
 #pragma unroll
     for (int u = 0; u < NP; u++) sr[u] = si[u] = 0;
-    for (int jh = 0; jh < nh; jh += 4) {
+    for (int jh = 4 * h; jh < nh; jh += 4 * SP) {
       T w[NP][4];
 #pragma unroll
       for (int u = 0; u < NP; u++) ld4(pw[u] + jh, w[u]);
@@ -174,7 +187,8 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
 #pragma unroll
     for (int u = 0; u < NP; u++) {
       const int n = m + r0 + 2 * u;
-      if (!live[u]) continue;
+      pair_sum<SP>(sr[u], si[u]);
+      if (!live[u] || h) continue;
       V o;
       o.x = n == ns ? (T)0 : sr[u] * (T)0.5;
       o.y = n == ns ? (T)0 : si[u] * (T)0.5;
@@ -194,7 +208,7 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
 #pragma unroll
   for (int u = 0; u < NP; u++)
     var[u] = vai[u] = vbr[u] = vbi[u] = dar[u] = dai[u] = dbr[u] = dbi[u] = er[u] = ei[u] = tr[u] = ti[u] = 0;
-  for (int jh = 0; jh < nh; jh += 4) {
+  for (int jh = 4 * h; jh < nh; jh += 4 * SP) {
     T wP[NP][4], wA[NP][4], wB[NP][4];
 #pragma unroll
     for (int u = 0; u < NP; u++) {
@@ -225,7 +239,13 @@ __global__ void __launch_bounds__(256) k_hs_analysis(HSAnaArgs<T> a, Tables<T> t
   }
 #pragma unroll
   for (int u = 0; u < NP; u++) {
-    if (!live[u]) continue;
+    pair_sum<SP>(var[u], vai[u]);
+    pair_sum<SP>(vbr[u], vbi[u]);
+    pair_sum<SP>(dar[u], dai[u]);
+    pair_sum<SP>(dbr[u], dbi[u]);
+    pair_sum<SP>(er[u], ei[u]);
+    pair_sum<SP>(tr[u], ti[u]);
+    if (!live[u] || h) continue;
     const int n = m + r0 + 2 * u;
     V ov, od, ot;
     if (n == ns) {  // row N+1 of the analysis is zero (Trans_Grid_To_Spherical!, :288-291)
@@ -417,7 +437,7 @@ bool at_fits(const jgcm_mesh* m) {
 // total wavenumbers per thread: two of one parity for member ensembles (each folded input loaded
 // from shared memory serves both: the analysis is shared-memory-bound at that scale), one otherwise
 // (shorter chains for the latency-bound single member)
-static int hs_analysis_np(int E) { return E >= 4 ? 2 : 1; }
+static int hs_analysis_np(const jgcm_mesh* m, int E) { return !is_fp64(m) && E >= 4 ? 2 : 1; }
 
 // threads per level of a block: the largest row count of an m pair (rows r = 4 i + b, b < 2, for
 // two rows per thread)
@@ -431,15 +451,33 @@ static int hs_analysis_rows(const jgcm_mesh* m, int np) {
   return q;
 }
 
-// levels per block of the Held-Suarez analysis: the tuned value when set (clamped to what a block
-// of 256 threads holds), else as many as a block holds (HS T42L20, one member: 5 levels 5.5 us,
-// 2 levels 7.1 us, 1 level 7.6 us per step in a captured graph)
-int hs_analysis_levels(const jgcm_mesh* m, int nd, int E) {
-  (void)nd;
-  const int lg_max = 256 / hs_analysis_rows(m, hs_analysis_np(E));
-  if (lg_max < 1) return 0;
-  if (m->hs_levels > 0) return std::min(m->hs_levels, lg_max);
-  return lg_max;
+// Levels per block and lanes per output (SP) of the Held-Suarez analysis.  The tuned number of levels when set
+// (clamped to what a block of 256 threads holds), else, FP32, as many as a block holds (HS T42L20, one member: 5 levels
+// 5.5 us, 2 levels 7.1 us, 1 level 7.6 us per step in a captured graph).  FP64 is bound by the FP64 pipe of the
+// busiest sub-partition: rounds of blocks over the SMs x (a block's warps on one of its four sub-partitions / SP +
+// half a unit for staging and folds) is least (a block of δ ln ps alone does not count).  Measured, levels x lanes: T42L20
+// 5x1 32.8 us, 4x1 28.7, 2x2 30.8, 3x1 43; T21L20 10x1 20.6, 2x1 16.4, 2x2 12.3; T31L20 7x1 30.8, 4x1 20.6, 3x2 18.5;
+// 4 members of T42L20 5x1 100, 4x1 76, 2x2 83 (two rows per thread 117).
+struct HSAnaShape {
+  int LG, SP;
+};
+static HSAnaShape hs_analysis_shape(const jgcm_mesh* m, int nd, int E) {
+  const int rows = hs_analysis_rows(m, hs_analysis_np(m, E)), lg_max = 256 / rows;
+  if (m->hs_levels > 0) return {std::min(m->hs_levels, lg_max), 1};
+  if (!is_fp64(m)) return {lg_max, 1};
+  HSAnaShape best = {lg_max, 1};
+  double least = 1e30;
+  for (int sp = 2; sp >= 1; sp--)
+    for (int lg = 1; lg <= std::min(256 / (rows * sp), nd + 1); lg++) {
+      const long blocks = (long)(m->N / 2 + 1) * ((nd + lg - 1) / lg) * E;
+      const int warps = (rows * lg * sp + 31) / 32;
+      const double cost = (double)((blocks + m->sm_count - 1) / m->sm_count) * ((double)((warps + 3) / 4) / sp + 0.5);
+      if (cost < least) {
+        least = cost;
+        best = {lg, sp};
+      }
+    }
+  return best;
 }
 
 // The tiled kernel serves an FP32 launch of E members: from five blocks per four SMs on (T42L20, 4 members
@@ -465,7 +503,7 @@ bool hs_analysis_fits(const jgcm_mesh* m, int nd, int E) {
   if (m->hs_levels < 0) return false;  // tuned to the general analysis kernel
   if (m->tc.on && !m->simt_legendre) return false;
   if (m->nh % 4 != 0) return false;  // weights four at a time (and rows of whole 16-byte chunks)
-  const int LG = hs_analysis_levels(m, nd, E);
+  const int LG = hs_analysis_shape(m, nd, E).LG;
   if (LG < 1) return false;
   const size_t sm = is_fp64(m) ? hs_analysis_smem<double>(m, LG) : hs_analysis_smem<float>(m, LG);
   return sm <= kSmemBudget;
@@ -478,12 +516,14 @@ int launch_hs_analysis(jgcm_mesh* m, const FFTPlan& fp, int colU, int colV, int 
                        int E, void* dvor, void* ddiv, void* dt, void* dlnps, cudaStream_t st, void* fbuf, int cap) {
   JG_ARG(hs_analysis_fits(m, nd, E), "the Held-Suarez analysis kernel does not fit this mesh");
   JG_TRY(launch_fft_only<T>(m, fp, st, fbuf, cap));
-  const int LG = hs_analysis_levels(m, nd, E);
+  const auto [LG, sp] = hs_analysis_shape(m, nd, E);
   const size_t sm = hs_analysis_smem<T>(m, LG);
   JG_TRY(g_hs_ana_smem[sizeof(T) == 8 ? 1 : 0].run([]() -> int {
-    JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    if constexpr (std::is_same<T, float>::value) {
+    JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    if constexpr (std::is_same<T, double>::value) {
+      JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    } else {
+      JG_CUDA(cudaFuncSetAttribute(k_hs_analysis<T, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
       JG_CUDA(cudaFuncSetAttribute(k_hs_analysis_tiles<384, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
       JG_CUDA(cudaFuncSetAttribute(k_hs_analysis_tiles<640, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
     }
@@ -522,13 +562,16 @@ int launch_hs_analysis(jgcm_mesh* m, const FFTPlan& fp, int colU, int colV, int 
       return JGCM_OK;
     }
   }
-  const int np = hs_analysis_np(E);
-  const int threads = (hs_analysis_rows(m, np) * LG + 31) / 32 * 32;
+  const int np = hs_analysis_np(m, E);
+  const int threads = (hs_analysis_rows(m, np) * LG * sp + 31) / 32 * 32;
   dim3 grid(m->N / 2 + 1, (nd + 1 + LG - 1) / LG, E);
-  if (np == 2)
-    JG_CUDA(launch_pdl(k_hs_analysis<T, 2>, grid, threads, sm, st, a, tables<T>(m)));
-  else
-    JG_CUDA(launch_pdl(k_hs_analysis<T, 1>, grid, threads, sm, st, a, tables<T>(m)));
+  auto kernel = k_hs_analysis<T, 1, 1>;
+  if constexpr (std::is_same<T, double>::value) {
+    if (sp == 2) kernel = k_hs_analysis<T, 1, 2>;
+  } else {
+    if (np == 2) kernel = k_hs_analysis<T, 2, 1>;
+  }
+  JG_CUDA(launch_pdl(kernel, grid, threads, sm, st, a, tables<T>(m)));
   mark(st);
   JG_CUDA(cudaGetLastError());
   return JGCM_OK;
