@@ -6,7 +6,8 @@
 //                    row N+1 included), a dense (nlat/2 x K) x (K x C) contraction per m,
 //                    mirrored to the northern hemisphere by parity;
 //   k_ifft         : inverse real zonal FFT of every (latitude, column) row as a half-length
-//                    complex FFT, radix-2 in shared memory, fused epilogue (÷cos, exp, ×ps).
+//                    complex FFT, radix-2 in shared memory, fused epilogue (÷cos, exp, ×ps); by size
+//                    also split over registers (zonal_fft.cuh), a warp's lanes, or a row per thread.
 // grid -> spectral (Trans_Grid_To_Spherical!, :221-293; Vor_Div_From_Grid_UV!, :349-459) runs as
 //   k_fft          : forward real zonal FFT (fft/nlon) with fused prologue (×cos, vorticity
 //                    fluxes, kinetic energy, shallow-water height tendency);
@@ -1391,7 +1392,16 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
 #define JG_IFFT_REG(HH) launch_pdl(k_ifft_reg<T, HH>, r.grid, r.threads, r.smem, st, ip, tb, (const V*)fbuf, m->N, m->nlat, r.lcb, r.tiles)
     switch (m->nlon) {
       case 64: JG_CUDA(JG_IFFT_REG(32)); break;
-      case 128: JG_CUDA(JG_IFFT_REG(64)); break;
+      case 128:
+        // FP32: the kernel streams and its time follows the threads in flight; where the launch has more than the
+        // 1024 per SM that the compiler's 64 registers leave room for, 48 registers (no spill) for 1280: 32 members of
+        // T42L20 76.5 -> 71.8 us, against 8.3 -> 9.5 for one member
+        if (std::is_same<T, float>::value && (size_t)r.grid.x * r.grid.y * r.threads > (size_t)1024 * m->sm_count)
+          JG_CUDA(launch_pdl(k_ifft_reg<T, 64, std::is_same<T, float>::value ? 5 : 0>, r.grid, r.threads, r.smem, st, ip, tb,
+                             (const V*)fbuf, m->N, m->nlat, r.lcb, r.tiles));
+        else
+          JG_CUDA(JG_IFFT_REG(64));
+        break;
       case 256: JG_CUDA(JG_IFFT_REG(128)); break;
       case 512: JG_CUDA(JG_IFFT_REG(256)); break;
       default: JG_CUDA(JG_IFFT_REG(512)); break;

@@ -256,10 +256,9 @@ __device__ __forceinline__ void fft_load_row(const FFTPlan& plan, const GridInGr
 // Fourier -> grid.  grid (column tiles or fewer, nlat), CB R2 threads, CB P complex T of shared memory.
 // With X the Hermitian spectrum (0 above N, Im X[0] dropped), D = X[m] - conj X[H-m] and w = e^(2 pi i m / nlon):
 // Z[m] = (X[m] + conj X[H-m]) + i w D, and Z[H-m] is formed from the same sum and product.
-// FP32, nlon 128: 5 blocks of 256 threads per SM (48 registers, no spill; the compiler's choice of 64 holds 4): the
-// kernel streams, its time follows the warps in flight (32 members of T42L20 76.5 -> 71.8 us; 6 blocks spill, 72).
-template <typename T, int H>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 && H == 64) ? 5 : 0) k_ifft_reg(const __grid_constant__ IFFTPlan plan, Tables<T> tb,
+// NB: blocks of 256 threads that the registers leave room for on an SM (0: the compiler's choice).
+template <typename T, int H, int NB = 0>
+__global__ void __launch_bounds__(256, NB) k_ifft_reg(const __grid_constant__ IFFTPlan plan, Tables<T> tb,
                                                   const V2<T>* __restrict__ F, int N, int nlat, int lcb, int ntiles) {
   using V = V2<T>;
   constexpr int R1 = FFTSplit<H>::R1, R2 = FFTSplit<H>::R2, P = FFTSplit<H>::P, L2 = log2_c(R2);
