@@ -451,23 +451,24 @@ static int hs_analysis_rows(const jgcm_mesh* m, int np) {
   return q;
 }
 
-// Levels per block and lanes per output (SP) of the Held-Suarez analysis.  The tuned number of levels when set
-// (clamped to what a block of 256 threads holds), else, FP32, as many as a block holds (HS T42L20, one member: 5 levels
-// 5.5 us, 2 levels 7.1 us, 1 level 7.6 us per step in a captured graph).  FP64 is bound by the FP64 pipe of the
-// busiest sub-partition: rounds of blocks over the SMs x (a block's warps on one of its four sub-partitions / SP +
-// half a unit for staging and folds) is least (a block of δ ln ps alone does not count).  Measured, levels x lanes: T42L20
-// 5x1 32.8 us, 4x1 28.7, 2x2 30.8, 3x1 43; T21L20 10x1 20.6, 2x1 16.4, 2x2 12.3; T31L20 7x1 30.8, 4x1 20.6, 3x2 18.5;
-// 4 members of T42L20 5x1 100, 4x1 76, 2x2 83 (two rows per thread 117).
+// Levels per block and lanes per output (SP) of the Held-Suarez analysis: the tuned number of levels when set
+// (clamped to what a block of 256 threads holds); for FP32 ensembles as many as a block holds; else what makes the
+// load of the busiest sub-partition least: rounds of blocks over the SMs x (a block's warps on one of its four
+// sub-partitions / SP + half a unit for staging and folds), a block of δ ln ps alone not counted, the smaller block
+// at a tie.  Measured in FP64 (levels x lanes; as many as a block holds first): T42L20 5x1 32.8 us, 4x1 28.7, 2x2 30.8,
+// 3x1 43; T21L20 10x1 20.6, 2x1 16.4, 2x2 12.3; T31L20 7x1 30.8, 4x1 20.6, 3x2 18.5; 4 members of T42L20 5x1 100, 4x1 76,
+// 2x2 83 (two rows per thread 117).  In FP32, a member's step: T42L20 5 levels 38.05 us, 4 37.6; T31L13 7 35.35, 2 33.7;
+// T21L20 10 34.7, 2 33.8.
 struct HSAnaShape {
   int LG, SP;
 };
 static HSAnaShape hs_analysis_shape(const jgcm_mesh* m, int nd, int E) {
   const int rows = hs_analysis_rows(m, hs_analysis_np(m, E)), lg_max = 256 / rows;
   if (m->hs_levels > 0) return {std::min(m->hs_levels, lg_max), 1};
-  if (!is_fp64(m)) return {lg_max, 1};
+  if (!is_fp64(m) && E >= 4) return {lg_max, 1};
   HSAnaShape best = {lg_max, 1};
   double least = 1e30;
-  for (int sp = 2; sp >= 1; sp--)
+  for (int sp = is_fp64(m) ? 2 : 1; sp >= 1; sp--)
     for (int lg = 1; lg <= std::min(256 / (rows * sp), nd + 1); lg++) {
       const long blocks = (long)(m->N / 2 + 1) * ((nd + lg - 1) / lg) * E;
       const int warps = (rows * lg * sp + 31) / 32;
