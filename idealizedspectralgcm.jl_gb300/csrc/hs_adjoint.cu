@@ -10,9 +10,9 @@
 //   implicit correction + leapfrog        the transposed semi-implicit kernel (models.cu)
 //   analyses of the tendencies            one synthesis-type launch (G2S^T) + the transposed alpha
 //                                         operator (k_alpha_adjoint + inverse FFT)
-//   column physics and dynamics           k_hs_column_adjoint: a warp per column, lanes over
-//                                         levels (Four_In_One!, Vert_Advection!, geopotential,
-//                                         HS_Forcing!, the p-level energy), FP64 arithmetic
+//   column physics and dynamics           k_hs_column_adjoint: eight lanes per column, up to four
+//                                         levels each (Four_In_One!, Vert_Advection!, geopotential,
+//                                         HS_Forcing!, the p-level energy)
 //   gradients of ln ps and T              one S2G^T launch + k_grad_adjoint
 // In sigma coordinates (a_k = 0) every log-pressure difference is a per-level constant, so the
 // dynamics depend on ps only through grad ln ps; only the Newtonian relaxation (T_eq(p)) and the
@@ -1139,7 +1139,7 @@ int check_model(jgcm_model* md) {
   JG_ARG(md, "NULL model");
   JG_ARG(md->P.kind == JGCM_HELD_SUAREZ, "the step adjoint exists for Held-Suarez models");
   JG_ARG(md->ne == 1, "one-member models only");
-  JG_ARG(md->nd <= 32, "the column adjoint holds one level per lane: nd <= 32");
+  JG_ARG(md->nd <= 32, "the column adjoint holds up to 32 levels: nd <= 32");
   JG_ARG(!md->diag_on, "switch the on-device diagnostics off before differentiating");
   // the reverse column kernel reads the sigma coordinates' per-level log-pressure constants
   JG_ARG(!md->vc.hybrid, "the step adjoint is built for sigma coordinates (a_k = 0), not hybrid ones");

@@ -776,8 +776,9 @@ __device__ __forceinline__ void lf(int init, int Dt, R rob, R d, R f, R& dq, R q
 // result are FP32, W_n as pairs hi + lo and the row sums as pairs (ds_add_prod: error-free products and
 // additions, ~2^-46 of the sum of magnitudes before the result is rounded to FP32).  An FP64 instruction
 // holds a sub-partition for ~64 cycles, the pair's ten FP32 ones for ten: with FP64 products this kernel
-// was bound by them from a few members on (128 x T21L20 95 -> 64 us, 32 x T42L20 90 -> 60 us, one T42L20 member 11.4 -> 9.8 us, event included; the
-// results against 64 bits as before: one member bit for bit, the ensembles 2.4e-6 and 2.5e-6 in the worst field).
+// was bound by them from a few members on (one column per warp, 128 x T21L20 95 -> 64 us, 32 x T42L20 90 -> 60 us,
+// one T42L20 member 11.4 -> 9.8 us, event included; the results against 64 bits as before: one member bit for bit,
+// the ensembles 2.4e-6 and 2.5e-6 in the worst field).
 // DENSE: the FP64 wave-matrix products of the block's modes are spread over all its threads, one
 // (mode, component, row) output each, instead of one mode per warp, whose 32 - nd idle lanes the
 // FP64 pipe executes all the same (for launches with many modes: member ensembles).
@@ -1507,8 +1508,8 @@ __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const Ver
 // latitude row at a time, a thread one column with all its levels, and keeps the three sums to the end of
 // its columns, so the folds, the barriers and the ticket come once per block.  One block per 32 columns and
 // 8 level groups spent 420 instructions and three barriers per warp on 2.5 levels (128 x T21L20 and 32 x T42L20
-// 58 us for 63 MB; 29 and 31 here, 4 levels' loads in flight 40 and 42).  As there: the kinetic part in the state precision over five levels at
-// a time, c_p T and every sum beyond as FP32 pairs (FP64 on the FP64 path).
+// 58 us for 63 MB; 29 here, 4 levels' loads in flight 40 and 42).  As there: the kinetic part in the state
+// precision over five levels at a time, c_p T and every sum beyond as FP32 pairs (FP64 on the FP64 path).
 constexpr int CORR_WARPS = 8;
 template <typename T>
 __global__ void __launch_bounds__(32 * CORR_WARPS) k_hs_corr_columns(CorrArgs<T> a, const VertCoef* __restrict__ vcp,
