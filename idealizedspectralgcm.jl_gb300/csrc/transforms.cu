@@ -1225,6 +1225,16 @@ static inline int fit_ct(int ct, int C) {
   while (ct > 1 && ct / 2 >= C) ct /= 2;
   return ct;
 }
+// And narrower while the launch, `rows` (wavenumbers or latitudes) x tiles, stays within seven blocks per SM: a small
+// launch is as long as its longest block (synthesis, step time with tiles of 8 -> 1 column: shallow water T85 FP32
+// 24.8 -> 19.8 us, FP64 87 -> 68, T42 FP32 17.4 -> 14.9; beyond it the tables staged per block cost more: T42L20 with
+// 774 blocks 37.5 us, 1548 38.3, 3053 40.9).  The FP64 shared-memory FFTs the same way (shallow water T42 48.5 -> 44.7 us,
+// T85 74.1 -> 71.6, barotropic T42 29.9 -> 27.7).
+static inline int spread_ct(const jgcm_mesh* m, int ct, int C, int rows) {
+  ct = fit_ct(ct, C);
+  while (ct > 1 && (size_t)rows * ((C + ct / 2 - 1) / (ct / 2)) <= (size_t)7 * m->sm_count) ct /= 2;
+  return ct;
+}
 
 // threads of a shared-memory FFT block: one per butterfly of a stage, two warps at least
 static inline int fft_threads(const jgcm_mesh* m, int fc) { return std::max(64, std::min(256, fc * m->nlon / 4)); }
@@ -1347,7 +1357,7 @@ static int launch_s2g_into(jgcm_mesh* m, const S2GPlan& sp0, const IFFTPlan& ip,
   const S2GPlan sp = with_f32(sp0);
   JG_TRY(configure_smem<T>());
   Tables<T> tb = tables<T>(m);
-  const int nh = m->nh, ct = m->tune[1] ? s2g_ct(m) : fit_ct(s2g_ct(m), sp.C);
+  const int nh = m->nh, ct = m->tune[1] ? s2g_ct(m) : spread_ct(m, s2g_ct(m), sp.C, m->N + 1);
   if (std::is_same<T, float>::value && m->tc.on && !m->simt_legendre) {
     JG_TRY(launch_s2g_legendre_tc(m, sp, fbuf, st));
   } else if (const int lt = s2g_tile_lats<T>(m, sp.C)) {
@@ -1374,7 +1384,7 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
   using V = V2<T>;
   const IFFTPlan ip = with_f32(ip0);
   Tables<T> tb = tables<T>(m);
-  const int fc = m->tune[3] > 0 ? fft_ct(m) : fit_ct(fft_ct(m), ip.C);
+  const int fc = m->tune[3] > 0 ? fft_ct(m) : spread_ct(m, fft_ct(m), ip.C, m->nlat);
   if (std::is_same<T, float>::value && use_row_fft(m, ip.C)) {  // many rows: a row per thread
     dim3 gr((ip.C + 32 * RF_WARPS - 1) / (32 * RF_WARPS), m->nlat);
     const Tables<float> tf = tables<float>(m);
@@ -1465,7 +1475,7 @@ int launch_fft_only(jgcm_mesh* m, const FFTPlan& fp0, cudaStream_t st, void* fbu
   }
   JG_ARG(fp.C <= cap && fp.C > 0, "bad FFT plan");
   Tables<T> tb = tables<T>(m);
-  const int fc = m->tune[3] > 0 ? fft_ct(m) : fit_ct(fft_ct(m), fp.C);
+  const int fc = m->tune[3] > 0 ? fft_ct(m) : spread_ct(m, fft_ct(m), fp.C, m->nlat);
   if (std::is_same<T, float>::value && use_row_fft(m, fp.C)) {  // many rows: a row per thread
     dim3 gr((fp.C + 32 * RF_WARPS - 1) / (32 * RF_WARPS), m->nlat);
     const Tables<float> tf = tables<float>(m);
