@@ -6,6 +6,7 @@
 // host.  Grids of an FP64 mesh have the host's layout and type: its FFT kernels read and write them
 // without a conversion.
 #include <cstring>
+#include <initializer_list>
 
 #include "jgcm_internal.cuh"
 
@@ -13,9 +14,11 @@ using namespace jgcm;
 
 namespace {
 
-int check_nlev(const jgcm_mesh* m, int nlev) {
+// every argument of a call, before anything is queued
+int check_args(const jgcm_mesh* m, int nlev, std::initializer_list<const double*> arrays) {
   JG_ARG(m != nullptr, "mesh is NULL");
   JG_ARG(nlev == m->nd || nlev == 1, "third dimension must be nd=%d or 1 (got %d)", m->nd, nlev);
+  for (const double* a : arrays) JG_ARG(a != nullptr, "an array of the call is NULL");
   return JGCM_OK;
 }
 
@@ -63,8 +66,9 @@ int spec_done(jgcm_mesh* m, int i, double* dst, int nlev) {
   JG_TRY(spec_dev_to_host(m, m->d_spec[i], p, nlev, m->stream));
   return host_out_done(dst, p, n, m->stream);
 }
-int finish(jgcm_mesh* m) {
+int finish(jgcm_mesh* m, HostCall& call) {
   JG_CUDA(cudaStreamSynchronize(m->stream));
+  call.done = true;
   JG_CUDA(cudaGetLastError());
   if (m->tc.on) JG_TRY(tc_status(m));  // a tensor-core kernel whose bounded wait gave up
   return JGCM_OK;
@@ -151,7 +155,8 @@ __global__ void k_adv_update(const T* gl, const T* gt, const double* u, const do
 namespace {
 // one group of a synthesis / of an analysis: plan, kernels, host arrays
 int synthesis(jgcm_mesh* m, int op, int epi, const double* spec, int nlev, double* grid) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {spec, grid}));
+  HostCall call(m->stream);
   const void* a;
   GridOut o;
   JG_TRY(spec_in(m, 0, spec, nlev, &a));
@@ -168,10 +173,11 @@ int synthesis(jgcm_mesh* m, int op, int epi, const double* spec, int nlev, doubl
   ip.g[0] = out_group(epi, o.dev, nlev, 0);
   JG_TRY(s2g(m, sp, ip));
   JG_TRY(grid_done(m, o, nlev));
-  return finish(m);
+  return finish(m, call);
 }
 int analysis(jgcm_mesh* m, int op, const double* grid, int nlev, double* spec) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {grid, spec}));
+  HostCall call(m->stream);
   const void* x;
   JG_TRY(grid_in(m, 1, grid, nlev, &x));
   FFTPlan fp;
@@ -187,7 +193,7 @@ int analysis(jgcm_mesh* m, int op, const double* grid, int nlev, double* spec) {
   gp.g[0].scale = m->nlon;
   JG_TRY(g2s(m, fp, gp));
   JG_TRY(spec_done(m, 0, spec, nlev));
-  return finish(m);
+  return finish(m, call);
 }
 }  // namespace
 
@@ -210,7 +216,8 @@ extern "C" int jgcm_trans_grid_to_spherical_adjoint(jgcm_mesh* m, const double* 
 }
 
 extern "C" int jgcm_trans_grid_to_fourier(jgcm_mesh* m, const double* pfield, int nlev, double* fourier) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {pfield, fourier}));
+  HostCall call(m->stream);
   const size_t nf = 2 * grid_elems(m, nlev);  // complex [nlev][nlat][nlon]: staging slots 1 and 2
   const void* x;
   double* f;
@@ -218,12 +225,13 @@ extern "C" int jgcm_trans_grid_to_fourier(jgcm_mesh* m, const double* pfield, in
   JG_TRY(host_out(m, fourier, nf, slot(m, 1), &f));
   JG_TRY(fourier_full_to_host(m, x, nlev, f, m->stream));
   JG_TRY(host_out_done(fourier, f, nf, m->stream));
-  return finish(m);
+  return finish(m, call);
 }
 
 extern "C" int jgcm_vor_div_from_grid_uv(jgcm_mesh* m, const double* u, const double* v, int nlev, double* vor,
                                          double* div) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {u, v, vor, div}));
+  HostCall call(m->stream);
   const void *gu, *gv;
   JG_TRY(grid_in(m, 0, u, nlev, &gu));
   JG_TRY(grid_in(m, 1, v, nlev, &gv));
@@ -242,12 +250,13 @@ extern "C" int jgcm_vor_div_from_grid_uv(jgcm_mesh* m, const double* u, const do
   JG_TRY(g2s(m, fp, gp));
   JG_TRY(spec_done(m, 0, vor, nlev));
   JG_TRY(spec_done(m, 1, div, nlev));
-  return finish(m);
+  return finish(m, call);
 }
 
 extern "C" int jgcm_uv_grid_from_vor_div(jgcm_mesh* m, const double* vor, const double* div, int nlev, double* u,
                                          double* v) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {vor, div, u, v}));
+  HostCall call(m->stream);
   const void *sv, *sd;
   GridOut ou, ov;
   JG_TRY(spec_in(m, 0, vor, nlev, &sv));
@@ -269,11 +278,12 @@ extern "C" int jgcm_uv_grid_from_vor_div(jgcm_mesh* m, const double* vor, const 
   JG_TRY(s2g(m, sp, ip));
   JG_TRY(grid_done(m, ou, nlev));
   JG_TRY(grid_done(m, ov, nlev));
-  return finish(m);
+  return finish(m, call);
 }
 
 extern "C" int jgcm_compute_gradients(jgcm_mesh* m, const double* hs, int nlev, double* gdl, double* gdt) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {hs, gdl, gdt}));
+  HostCall call(m->stream);
   const void* a;
   GridOut ol, ot;
   JG_TRY(spec_in(m, 0, hs, nlev, &a));
@@ -282,12 +292,13 @@ extern "C" int jgcm_compute_gradients(jgcm_mesh* m, const double* hs, int nlev, 
   JG_TRY(gradients_dev(m, a, nlev, ol.dev, ot.dev));
   JG_TRY(grid_done(m, ol, nlev));
   JG_TRY(grid_done(m, ot, nlev));
-  return finish(m);
+  return finish(m, call);
 }
 
 extern "C" int jgcm_add_horizontal_advection(jgcm_mesh* m, const double* hs, const double* u, const double* v,
                                              int nlev, double* dh) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {hs, u, v, dh}));
+  HostCall call(m->stream);
   const size_t ng = grid_elems(m, nlev);
   const void* a;
   const double *pu, *pv, *ph;
@@ -308,23 +319,25 @@ extern "C" int jgcm_add_horizontal_advection(jgcm_mesh* m, const double* hs, con
                                                          out, ng);
   JG_CUDA(cudaGetLastError());
   JG_TRY(host_out_done(dh, out, ng, m->stream));
-  return finish(m);
+  return finish(m, call);
 }
 
 extern "C" int jgcm_apply_laplacian(jgcm_mesh* m, double* spe, int nlev) {
-  JG_TRY(check_nlev(m, nlev));
+  JG_TRY(check_args(m, nlev, {spe}));
+  HostCall call(m->stream);
   const void* a;
   JG_TRY(spec_in(m, 0, spe, nlev, &a));
   JG_TRY(apply_laplacian(m, m->d_spec[0], nlev, m->stream));
   JG_TRY(spec_done(m, 0, spe, nlev));
-  return finish(m);
+  return finish(m, call);
 }
 
 extern "C" int jgcm_area_weighted_global_mean(jgcm_mesh* m, const double* grid, double* out) {
-  JG_ARG(m && grid && out, "NULL argument");
+  JG_TRY(check_args(m, 1, {grid, out}));
+  HostCall call(m->stream);
   const void* x;
   JG_TRY(grid_in(m, 0, grid, 1, &x));
   JG_TRY(area_mean(m, x, m->d_red, m->stream));
   JG_CUDA(cudaMemcpyAsync(out, m->d_red, 8, cudaMemcpyDeviceToHost, m->stream));
-  return finish(m);
+  return finish(m, call);
 }

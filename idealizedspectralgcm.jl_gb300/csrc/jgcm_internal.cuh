@@ -358,6 +358,19 @@ int launch_ifft_only(jgcm_mesh* m, const IFFTPlan& ip, cudaStream_t st, void* fb
 int host_in(jgcm_mesh* m, const double* src, size_t n, double* stage, cudaStream_t st, const double** use);
 int host_out(jgcm_mesh* m, double* dst, size_t n, double* stage, double** use);
 int host_out_done(double* dst, const double* use, size_t n, cudaStream_t st);
+// Held by an entry point from before it hands a caller's array to a kernel or a copy until it returns: a return
+// before `done` is set (an error) first waits for what is queued on the stream, so that nothing reads or
+// writes the arrays when they are the caller's again.
+struct HostCall {
+  cudaStream_t st;
+  bool done = false;
+  explicit HostCall(cudaStream_t s) : st(s) {}
+  HostCall(const HostCall&) = delete;
+  HostCall& operator=(const HostCall&) = delete;
+  ~HostCall() {
+    if (!done) cudaStreamSynchronize(st);
+  }
+};
 int spec_host_to_dev(jgcm_mesh* m, const double* d_host_layout, void* d_native, int L, cudaStream_t st);
 int spec_dev_to_host(jgcm_mesh* m, const void* d_native, double* d_host_layout, int L, cudaStream_t st);
 int grid_host_to_dev(jgcm_mesh* m, const double* d_src, void* d_native, size_t n, cudaStream_t st);

@@ -3227,6 +3227,7 @@ extern "C" int jgcm_model_get_field(jgcm_model* md, const char* name, double* ho
   JG_ARG(cap >= (long)n, "buffer too small for '%s'", name);
   cudaStream_t st = m->stream;
   double* stage = n <= 4 * m->stage_slot ? m->d_stage : md->q_stage;  // tracer fields may need their own
+  HostCall call(st);
   if (f.derived) {
     size_t G = grid_elems(m, 1);
     int nb = (int)((G + 127) / 128);
@@ -3248,6 +3249,7 @@ extern "C" int jgcm_model_get_field(jgcm_model* md, const char* name, double* ho
     JG_TRY(host_out_done(host, dst, n, st));
   }
   JG_CUDA(cudaStreamSynchronize(st));
+  call.done = true;
   return JGCM_OK;
 }
 
@@ -3264,14 +3266,16 @@ extern "C" int jgcm_model_set_field(jgcm_model* md, const char* name, const doub
   double* stage = n <= 4 * m->stage_slot ? m->d_stage : md->q_stage;  // tracer fields may need their own
   JG_CUDA(cudaStreamSynchronize(st));
   const double* src;
+  HostCall call(st);
+  md->grad_ready = 0;  // the gradients of the current level are recomputed by the next step
   JG_TRY(host_in(m, host, n, stage, st, &src));
   if (f.spec)
     JG_TRY(spec_host_to_dev(m, src, f.ptr, f.L, st));
   else
     JG_TRY(grid_host_to_dev(m, src, f.ptr, n, st));
   if (!strcmp(name, "spe_lnps_n")) md->sw_adv_from_n = 1;
-  md->grad_ready = 0;  // the gradients of the current level are recomputed by the next step
   JG_CUDA(cudaStreamSynchronize(st));
+  call.done = true;
   return JGCM_OK;
 }
 

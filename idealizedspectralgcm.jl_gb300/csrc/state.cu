@@ -208,14 +208,16 @@ extern "C" int jgcm_model_set_state(jgcm_model* md, const double* packed) {
   size_t n = 0;
   JG_TRY(pack_list(md, &p, &n));
   const double* src;
+  HostCall call(st);
+  md->grad_ready = 0;  // the gradients of the new c level are recomputed by the next step
   JG_TRY(host_in(m, packed, n, md->state_stage, st, &src));
   const dim3 g(64, NSTATE);
   const size_t G1 = grid_elems(m, 1);
   if (is_fp64(m)) k_state_h2d<double><<<g, 256, 0, st>>>(p, src, m->N, m->ns, G1);
   else k_state_h2d<float><<<g, 256, 0, st>>>(p, src, m->N, m->ns, G1);
   JG_CUDA(cudaGetLastError());
-  md->grad_ready = 0;  // the gradients of the new c level are recomputed by the next step
   JG_CUDA(cudaStreamSynchronize(st));
+  call.done = true;
   return JGCM_OK;
 }
 
@@ -228,6 +230,7 @@ extern "C" int jgcm_model_get_state(jgcm_model* md, double* packed) {
   size_t n = 0;
   JG_TRY(pack_list(md, &p, &n));
   double* dst;
+  HostCall call(st);
   JG_TRY(host_out(m, packed, n, md->state_stage, &dst));
   const dim3 g(64, NSTATE);
   const size_t G1 = grid_elems(m, 1);
@@ -236,5 +239,6 @@ extern "C" int jgcm_model_get_state(jgcm_model* md, double* packed) {
   JG_CUDA(cudaGetLastError());
   JG_TRY(host_out_done(packed, dst, n, st));
   JG_CUDA(cudaStreamSynchronize(st));
+  call.done = true;
   return JGCM_OK;
 }
