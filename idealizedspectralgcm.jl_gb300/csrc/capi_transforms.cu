@@ -144,12 +144,6 @@ int gradients_dev(jgcm_mesh* m, const void* d_spec, int nlev, void* d_gl, void* 
   return s2g(m, sp, ip);
 }
 
-template <typename T>
-__global__ void k_adv_update(const T* gl, const T* gt, const double* u, const double* v, double* dh, size_t n) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-    dh[t] = dh[t] - (u[t] * (double)gl[t] + v[t] * (double)gt[t]);
-}
-
 }  // namespace
 
 namespace {
@@ -309,15 +303,7 @@ extern "C" int jgcm_add_horizontal_advection(jgcm_mesh* m, const double* hs, con
   JG_TRY(host_in(m, dh, ng, slot(m, 3), m->stream, &ph));
   double* out;  // dh itself or its staged copy, updated in place
   JG_TRY(host_out(m, dh, ng, slot(m, 3), &out));
-  size_t nb = (ng + 255) / 256;
-  if (nb > 1184) nb = 1184;
-  if (is_fp64(m))
-    k_adv_update<double><<<(int)nb, 256, 0, m->stream>>>((const double*)m->d_grid[0], (const double*)m->d_grid[1], pu,
-                                                          pv, out, ng);
-  else
-    k_adv_update<float><<<(int)nb, 256, 0, m->stream>>>((const float*)m->d_grid[0], (const float*)m->d_grid[1], pu, pv,
-                                                         out, ng);
-  JG_CUDA(cudaGetLastError());
+  JG_TRY(advection_update(m, m->d_grid[0], m->d_grid[1], pu, pv, out, ng, m->stream));
   JG_TRY(host_out_done(dh, out, ng, m->stream));
   return finish(m, call);
 }

@@ -1771,6 +1771,22 @@ int apply_laplacian(jgcm_mesh* m, void* d_spec, int L, cudaStream_t st) {
   return JGCM_OK;
 }
 
+// Add_Horizontal_Advection! (Spectral_Spherical_Mesh.jl:694-718) from the gradients of the advected field
+template <typename T>
+__global__ void k_adv_update(const T* gl, const T* gt, const double* u, const double* v, double* dh, size_t n) {
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
+    dh[t] = dh[t] - (u[t] * (double)gl[t] + v[t] * (double)gt[t]);
+}
+int advection_update(jgcm_mesh* m, const void* gl, const void* gt, const double* u, const double* v, double* dh, size_t n,
+                     cudaStream_t st) {
+  if (is_fp64(m))
+    k_adv_update<double><<<nblk(n), 256, 0, st>>>((const double*)gl, (const double*)gt, u, v, dh, n);
+  else
+    k_adv_update<float><<<nblk(n), 256, 0, st>>>((const float*)gl, (const float*)gt, u, v, dh, n);
+  JG_CUDA(cudaGetLastError());
+  return JGCM_OK;
+}
+
 // Area_Weighted_Global_Mean (Spectral_Spherical_Mesh.jl:746-760): one block, FP64, fixed order.
 template <typename T>
 __global__ void k_area_mean(const T* __restrict__ g, const double* __restrict__ w, int nlat, int nlon, double* out) {

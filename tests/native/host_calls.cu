@@ -1,6 +1,7 @@
 // The host-pointer entry points of capi_transforms.cu over stand-ins for everything they queue, for tests on the
 // CPU: each stand-in records 'q' (work queued that may touch the caller's arrays) and can be told to fail; a
-// stream synchronisation records 's'.  No kernel runs and no device is needed.
+// stream synchronisation records 's'.  capi_transforms.cu launches no kernel itself, and the process that loads
+// this sees no device.
 #include "capi_transforms.cu"
 
 #include <cstdio>
@@ -46,6 +47,9 @@ int grid_host_to_dev(jgcm_mesh*, const double*, void*, size_t, cudaStream_t) { r
 int grid_dev_to_host(jgcm_mesh*, const void*, double*, size_t, cudaStream_t) { return queue(); }
 int fourier_full_to_host(jgcm_mesh*, const void*, int, double*, cudaStream_t) { return queue(); }
 int apply_laplacian(jgcm_mesh*, void*, int, cudaStream_t) { return queue(); }
+int advection_update(jgcm_mesh*, const void*, const void*, const double*, const double*, double*, size_t, cudaStream_t) {
+  return queue();
+}
 int area_mean(jgcm_mesh*, const void*, double*, cudaStream_t) { return queue(); }
 int tc_status(jgcm_mesh*) { return JGCM_OK; }
 template <typename T>

@@ -1,14 +1,16 @@
 """The host-pointer transforms leave the caller's arrays alone once they return, in failure too (CPU).
 
-Their kernels read and write the arrays in place, so a call that returns with work in flight would let a
+Their kernels read and write the arrays in place, so a call that returned with work in flight would let a
 program free memory that the device still reads or writes.  The entry points are compiled over stand-ins
-(native/host_calls.cu) that record what is queued and fail on request; nothing runs on a device.
+(native/host_calls.cu) that record what is queued and fail on request.  The stand-ins run in a process of their
+own that sees no CUDA device: nothing can be launched, whatever machine this runs on.
 """
 import ctypes as C
+import json
 import os
 import subprocess
+import sys
 
-import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -22,55 +24,68 @@ CALLS = {"jgcm_trans_spherical_to_grid": "ana", "jgcm_trans_grid_to_spherical": 
          "jgcm_area_weighted_global_mean": "aa"}
 
 
+def _run(so):
+    """every call of both precisions: {"name/precision": {what: [status, events]}}"""
+    lib = C.CDLL(so)
+    lib.stub_mesh.restype = C.c_void_p
+    lib.stub_events.restype = C.c_char_p
+
+    def call(name, mesh, fail_at=0, null=None, nlev=3):
+        arrays, args = [], [C.c_void_p(mesh)]
+        for c in CALLS[name]:
+            if c == "n":
+                args.append(C.c_int(nlev))
+                continue
+            arrays.append((C.c_double * (2 * 16 * 10 * 3))())
+            args.append(C.c_void_p(None if len(arrays) - 1 == null else C.addressof(arrays[-1])))
+        lib.stub_begin(fail_at)
+        return [getattr(lib, name)(*args), lib.stub_events().decode()]
+
+    out = {}
+    for precision in (0, 1):
+        mesh = lib.stub_mesh(precision)
+        for name, args in CALLS.items():
+            good = call(name, mesh)
+            r = {"good": good, "bad": [call(name, mesh, null=k) for k in range(args.count("a"))] + [call(name, None)],
+                 "failing": [call(name, mesh, fail_at=k) for k in range(1, good[1].count("q") + 1)]}
+            if "n" in args:
+                r["bad"].append(call(name, mesh, nlev=2))
+            out[f"{name}/{precision}"] = r
+    return out
+
+
 @pytest.fixture(scope="module")
-def stub(built, tmp_path_factory):
+def results(built, tmp_path_factory):
     import build_lib
 
     so = str(tmp_path_factory.mktemp("native") / "libhostcalls.so")
     wrap = [f"-Xlinker=--wrap={f}" for f in ("cudaStreamSynchronize", "cudaGetLastError", "cudaMemcpyAsync")]
-    cmd = [build_lib.NVCC] + build_lib.ARCH + build_lib.FLAGS + ["-Xcompiler", "-fvisibility=default", "-shared",
-           "-o", so, os.path.join(HERE, "native", "host_calls.cu")] + wrap
+    cmd = [build_lib.NVCC] + build_lib.ARCH + build_lib.FLAGS + ["-Xcompiler", "-fvisibility=default", "-shared", "-o", so,
+           os.path.join(HERE, "native", "host_calls.cu")] + wrap
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
-    lib = C.CDLL(so)
-    lib.stub_mesh.restype = C.c_void_p
-    lib.stub_events.restype = C.c_char_p
-    return lib
-
-
-def _call(stub, name, mesh, fail_at, null=None, nlev=3):
-    f = getattr(stub, name)
-    arrays, args, k = [], [C.c_void_p(mesh)], 0
-    for c in CALLS[name]:
-        if c == "n":
-            args.append(C.c_int(nlev))
-            continue
-        arrays.append(np.zeros(2 * 16 * 10 * 3))
-        args.append(C.c_void_p(None if k == null else arrays[-1].ctypes.data))
-        k += 1
-    stub.stub_begin(fail_at)
-    status = f(*args)
-    return status, stub.stub_events().decode()
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), so], capture_output=True, text=True,
+                       env=dict(os.environ, CUDA_VISIBLE_DEVICES=""))
+    assert r.returncode == 0, r.stderr
+    return json.loads(r.stdout)
 
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("name", sorted(CALLS))
-def test_arguments_are_checked_before_anything_is_queued(stub, name, precision):
-    mesh = stub.stub_mesh(precision)
-    for null in range(CALLS[name].count("a")):
-        assert _call(stub, name, mesh, 0, null=null) == (-1, ""), null
-    if "n" in CALLS[name]:
-        assert _call(stub, name, mesh, 0, nlev=2) == (-1, "")
-    assert _call(stub, name, None, 0) == (-1, "")
+def test_arguments_are_checked_before_anything_is_queued(results, name, precision):
+    for r in results[f"{name}/{precision}"]["bad"]:
+        assert r == [-1, ""]
 
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("name", sorted(CALLS))
-def test_a_failing_call_waits_for_what_it_queued(stub, name, precision):
+def test_a_failing_call_waits_for_what_it_queued(results, name, precision):
     """whichever launch or copy fails: a synchronisation follows the last thing queued"""
-    mesh = stub.stub_mesh(precision)
-    status, events = _call(stub, name, mesh, 0)
-    assert status == 0 and events.endswith("s") and "q" in events
-    for k in range(1, events.count("q") + 1):
-        status, ev = _call(stub, name, mesh, k)
-        assert status == -2 and ev == "q" * (k - 1) + "s", (k, ev)
+    r = results[f"{name}/{precision}"]
+    assert r["good"][0] == 0 and r["good"][1].strip("q") == "s" and r["failing"]
+    for k, f in enumerate(r["failing"]):
+        assert f == [-2, "q" * k + "s"], k
+
+
+if __name__ == "__main__":
+    print(json.dumps(_run(sys.argv[1])))
