@@ -1287,7 +1287,8 @@ static bool reg_fft(const jgcm_mesh* m, int C) {
   if (sizeof(T) == 4) return m->nd > 1 && C > 2;
   return (size_t)C * m->nlat * reg_fft_threads(m->nlon) >= (size_t)2 * 32 * m->sm_count;
 }
-// They move pairs of values: every field has to start on a pair's boundary (a caller's device grid may not).
+// The FFTs other than those in shared memory move pairs of values: every field has to start on a pair's
+// boundary.  A caller's device grid may not, and takes the shared-memory kernel.
 template <typename T>
 static bool pairs_aligned(const IFFTPlan& p) {
   uintptr_t a = 0;
@@ -1385,7 +1386,8 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
   const IFFTPlan ip = with_f32(ip0);
   Tables<T> tb = tables<T>(m);
   const int fc = m->tune[3] > 0 ? fft_ct(m) : spread_ct(m, fft_ct(m), ip.C, m->nlat);
-  if (std::is_same<T, float>::value && use_row_fft(m, ip.C)) {  // many rows: a row per thread
+  const bool pairs = pairs_aligned<T>(ip);
+  if (std::is_same<T, float>::value && use_row_fft(m, ip.C) && pairs) {  // many rows: a row per thread
     dim3 gr((ip.C + 32 * RF_WARPS - 1) / (32 * RF_WARPS), m->nlat);
     const Tables<float> tf = tables<float>(m);
     const float2* Ff = (const float2*)fbuf;
@@ -1397,7 +1399,7 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
     JG_CUDA(cudaGetLastError());
     return JGCM_OK;
   }
-  if (reg_fft<T>(m, ip.C) && pairs_aligned<T>(ip)) {
+  if (reg_fft<T>(m, ip.C) && pairs) {
     const RegFFT r = reg_fft_shape<T>(m, ip.C);
 #define JG_IFFT_REG(HH) launch_pdl(k_ifft_reg<T, HH>, r.grid, r.threads, r.smem, st, ip, tb, (const V*)fbuf, m->N, m->nlat, r.lcb, r.tiles)
     switch (m->nlon) {
@@ -1421,7 +1423,7 @@ static int launch_ifft_stage(jgcm_mesh* m, const IFFTPlan& ip0, cudaStream_t st,
     JG_CUDA(cudaGetLastError());
     return JGCM_OK;
   }
-  if (std::is_same<T, float>::value && m->nlon >= 64 && m->nlon <= 1024 && m->tune[3] == 0) {
+  if (std::is_same<T, float>::value && m->nlon >= 64 && m->nlon <= 1024 && m->tune[3] == 0 && pairs) {
     const size_t smw = (size_t)(m->N + 1) * FW_COLS * sizeof(V);
     dim3 gw((ip.C + FW_COLS - 1) / FW_COLS, m->nlat);
     switch (m->nlon) {
@@ -1857,6 +1859,8 @@ extern "C" int jgcm_trans_spherical_to_grid_noalloc(jgcm_mesh* m, const void* d_
   using namespace jgcm;
   JG_ARG(m != nullptr && d_snm != nullptr && d_grid != nullptr, "NULL argument");
   JG_ARG(nlev == m->nd || nlev == 1, "third dimension must be nd=%d or 1 (got %d)", m->nd, nlev);
+  JG_ARG((uintptr_t)d_snm % (2 * tsize(m)) == 0 && (uintptr_t)d_grid % tsize(m) == 0,
+         "d_snm must be aligned to its complex values (%zu bytes), d_grid to its values (%zu bytes)", 2 * tsize(m), tsize(m));
   const size_t need = (size_t)(m->N + 1) * m->nlat * nlev * 2 * tsize(m);
   JG_ARG(need <= kNoAllocScratchBytes,
          "jgcm_trans_spherical_to_grid_noalloc: needs %zu bytes of scratch for (N+1)=%d x nlat=%d x nlev=%d, the "

@@ -111,8 +111,10 @@ int jgcm_area_weighted_global_mean(jgcm_mesh* mesh, const double* grid, double* 
  * while a stream is captured into a CUDA graph, hosts whose device memory belongs to their own
  * pool allocator, and loops that forbid allocation after start-up.
  *   d_snm   device array, mesh precision, library layout: complex [m][n][k] (N+1 x N+2 x nlev,
- *           levels innermost; entries n < m are ignored)
- *   d_grid  device array, mesh precision: [k][nlat][nlon]
+ *           levels innermost; entries n < m are ignored), aligned to its complex values (16 bytes in
+ *           FP64, 8 bytes otherwise), else JGCM_E_ARG
+ *   d_grid  device array, mesh precision: [k][nlat][nlon], aligned to its values (8 or 4 bytes), else
+ *           JGCM_E_ARG; twice that is faster
  *   stream  cudaStream_t to run on, or NULL for the mesh's stream; the call is asynchronous.
  * Same result as jgcm_trans_spherical_to_grid.  The Fourier coefficients are staged in a static
  * 8 MiB device array owned by the library (every GPU that loads it holds it until exit), so
