@@ -136,16 +136,20 @@ __device__ __forceinline__ void leapfrog_c(const StepParams& sp, T d, V2<T>& dq,
 // Input of the synthesis for total wavenumber n (>= m) of column k of group g: the field itself,
 // cos(lat) x its gradient (Compute_Gradient_Cos!, Spectral_Spherical_Mesh.jl:655-692) or ucos / vcos
 // from vorticity and divergence (Compute_Ucos_Vcos_From_Vor_Div!, :517-580; these fill row N+1).
-template <typename T, int OP>
-__device__ __forceinline__ V2<T> s2g_input_op(const S2GGroup& g, const Tables<T>& tb, int m, int n, int ns, size_t mrow,
-                                                int k) {
+// OP: the group's operator, S2G_ANY = looked up per call.  The tensor-core kernel looks it up: with a call of its
+// own per operator it compiled to 40 registers instead of 48, fewer loads in flight (T85, 8 barotropic
+// members, BF16x3: 18.4 -> 22.3 us).
+constexpr int S2G_ANY = -1;
+template <typename T, int OP = S2G_ANY>
+__device__ __forceinline__ V2<T> s2g_input(const S2GGroup& g, const Tables<T>& tb, int m, int n, int ns, size_t mrow,
+                                             int k) {
   using V = V2<T>;
-  const int L = g.L;
+  const int L = g.L, op = OP == S2G_ANY ? g.op : OP;
   const V* a = (const V*)g.a;
   V x;
   x.x = 0;
   x.y = 0;
-  switch (OP) {
+  switch (op) {
     case S2G_PLAIN:
       x = a[(mrow + n) * L + k];
       if (m == 0 && n == 0) x.x = x.x - pick<T>(g.shift, g.shiftf);
@@ -189,7 +193,7 @@ __device__ __forceinline__ V2<T> s2g_input_op(const S2GGroup& g, const Tables<T>
       // vcos = uvc (i vor) + uvm div_{n-1} + uvp div_{n+1}
       const V* vor = a;
       const V* dv = (const V*)g.b;
-      const bool u = OP == S2G_UCOS;
+      const bool u = op == S2G_UCOS;
       const V* ic = u ? dv : vor;  // term multiplied by i*uvc
       const V* nb = u ? vor : dv;  // neighbour terms
       T sg = u ? (T)-1 : (T)1;
@@ -214,26 +218,13 @@ __device__ __forceinline__ V2<T> s2g_input_op(const S2GGroup& g, const Tables<T>
   return x;
 }
 
-template <typename T>
-__device__ __forceinline__ V2<T> s2g_input(const S2GGroup& g, const Tables<T>& tb, int m, int n, int ns, size_t mrow,
-                                             int k) {
-  switch (g.op) {
-    case S2G_PLAIN: return s2g_input_op<T, S2G_PLAIN>(g, tb, m, n, ns, mrow, k);
-    case S2G_DLAM: return s2g_input_op<T, S2G_DLAM>(g, tb, m, n, ns, mrow, k);
-    case S2G_DTH: return s2g_input_op<T, S2G_DTH>(g, tb, m, n, ns, mrow, k);
-    case S2G_UCOS: return s2g_input_op<T, S2G_UCOS>(g, tb, m, n, ns, mrow, k);
-    case S2G_VCOS: return s2g_input_op<T, S2G_VCOS>(g, tb, m, n, ns, mrow, k);
-    case S2G_ADJ_G2S: return s2g_input_op<T, S2G_ADJ_G2S>(g, tb, m, n, ns, mrow, k);
-    default: return s2g_input_op<T, S2G_ANOM>(g, tb, m, n, ns, mrow, k);
-  }
-}
 // Rows n = m + r, r = r0, r0 + rstep, ... < K of one column into X[r * CT]; the group's operator is chosen
 // once, so several rows' loads are in flight
 template <typename T, int OP>
 __device__ __forceinline__ void s2g_column_op(const S2GGroup& g, const Tables<T>& tb, int m, int ns, size_t mrow, int k,
                                               V2<T>* X, int CT, int r0, int rstep, int K) {
 #pragma unroll 4
-  for (int r = r0; r < K; r += rstep) X[r * CT] = s2g_input_op<T, OP>(g, tb, m, m + r, ns, mrow, k);
+  for (int r = r0; r < K; r += rstep) X[r * CT] = s2g_input<T, OP>(g, tb, m, m + r, ns, mrow, k);
 }
 template <typename T>
 __device__ __forceinline__ void s2g_column(const S2GGroup& g, const Tables<T>& tb, int m, int ns, size_t mrow, int k,
