@@ -28,6 +28,8 @@ namespace jgcm {
 
 // Dynamic shared memory the transform kernels may use per block (the SM allows 227 KB).
 constexpr size_t kSmemBudget = 200 * 1024;
+// ... and may use if an SM is to hold two of them
+constexpr size_t kSmemPair = 112 * 1024;
 
 // Largest dynamic shared memory the unconditional parts of the transform kernels need for a mesh
 // whose tables hold `ts`-byte reals: the synthesis stages all P rows of one m plus one spectral

@@ -964,15 +964,17 @@ constexpr int FFT_BLOCKS_PER_SM = 4;  // the column tiles' (reg_fft_shape)
 // the tile no wider than the launch's columns 12.2, 12.3 and 31.6 us, launch and event included).  The weight rows are constants: they are staged by asynchronous copies before the
 // dependency wait, at a pitch one 16-byte chunk longer than a row, so that the rows read by a warp's
 // quads start in different banks.  Only the tables (`tabs`) and input slots (`slots`) that the plan
-// uses are staged.
+// uses are staged.  STAGE: as launch_g2s chooses; without it the weights come from L2 row by row, and the FP32
+// kernel of four lanes per output keeps more of them in flight in 64 registers than in the compiler's 48 (shallow
+// water T170, 8 members 157 -> 128 us; staged, 48 are enough).
 enum { G2S_TAB_PW = 1, G2S_TAB_AB = 2, G2S_TAB_P = 4 };
 __host__ __device__ inline int g2s_ntab(int tabs) { return (tabs & G2S_TAB_PW ? 1 : 0) + (tabs & G2S_TAB_AB ? 2 : 0) + (tabs & G2S_TAB_P ? 1 : 0); }
 __host__ __device__ inline int bits4(int x) { return (x & 1) + (x >> 1 & 1) + (x >> 2 & 1) + (x >> 3 & 1); }
 
-template <typename T, int QL>
-__global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb, const V2<T>* __restrict__ F,
-                                                      int ns, int nlat, int Cin, int CT, int RC, int slots, int tabs,
-                                                      int stage) {
+template <typename T, int QL, bool STAGE>
+__global__ void __launch_bounds__(256, !STAGE && QL == 4 && sizeof(T) == 4 ? 4 : 0)
+    k_g2s_legendre(G2SPlan plan, Tables<T> tb, const V2<T>* __restrict__ F, int ns, int nlat, int Cin, int CT, int RC,
+                   int slots, int tabs) {
   using V = V2<T>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int m = blockIdx.y;
@@ -989,7 +991,7 @@ __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb
   // quadrature rows of this block ([K][pitch]); staged once per block when they fit
   const T *tPW = tb.PW + toff, *tCA = tb.CA + toff, *tCB = tb.CB + toff, *tP = tb.P + toff;
   int wp = nh;
-  if (stage) {
+  if constexpr (STAGE) {
     constexpr int ce = 16 / (int)sizeof(T);
     wp = nh + ce;
     T* dst = (T*)(A + nslot * CT * nh);
@@ -1037,7 +1039,7 @@ __global__ void __launch_bounds__(256) k_g2s_legendre(G2SPlan plan, Tables<T> tb
     S[i] = s;
     A[i] = a;
   }
-  if (stage) cp_async_wait_all();
+  if constexpr (STAGE) cp_async_wait_all();
   __syncthreads();
   // each output is summed by QL threads (latitudes jh = q, q+QL, ...), then combined with masked
   // shuffles; the QL lanes never straddle loop iterations (blockDim is a multiple of 4)
@@ -1190,8 +1192,10 @@ static int configure_smem() {
     JG_CUDA(cudaFuncSetAttribute(k_ifft<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     JG_CUDA(cudaFuncSetAttribute(k_fft<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     JG_CUDA(cudaFuncSetAttribute(k_fourier_full<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+    JG_CUDA(cudaFuncSetAttribute(k_g2s_legendre<T, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
     if (idx == 0) {
       JG_CUDA(cudaFuncSetAttribute(k_s2g_tiles<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
       JG_CUDA(cudaFuncSetAttribute(k_s2g_tiles<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
@@ -1581,14 +1585,18 @@ int launch_g2s(jgcm_mesh* m, const FFTPlan& fp, const G2SPlan& gp0, cudaStream_t
     rc = (rc + 1) / 2;
   size_t sm = (size_t)2 * bits4(slots) * ct * nh * sizeof(V);
   const size_t tab = (size_t)g2s_ntab(tabs) * rc * (nh + 16 / sizeof(T)) * sizeof(T);
-  const int stage = sm + tab <= kSmemBudget;
+  // staged where the rows fit beside another block's; in FP32 a block that would have its SM to itself keeps them
+  // only if its outputs take a few passes (shallow water T170, one member, 2 passes: 32 us, unstaged 37), since with
+  // more the SM waits on eight warps (us, staged and not: barotropic T170, 8 members 47, 43, 32 members 144, 98;
+  // shallow water T106, 32 members 158, 73).  FP64 is bound by its arithmetic (T106, 8 members 257, 282).
+  const int passes = (rc * ct * ql + 255) / 256;
+  const bool stage = sm + tab <= (sizeof(T) == 8 || (ql == 4 && passes <= 4) ? kSmemBudget : kSmemPair);
   if (stage) sm += tab;
   dim3 g(tiles, m->N + 1, (K0 + rc - 1) / rc);
   const int threads = std::min(256, (rc * ct * ql + 31) / 32 * 32);
-  if (ql == 1)
-    JG_CUDA(launch_pdl(k_g2s_legendre<T, 1>, g, threads, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, rc, slots, tabs, stage));
-  else
-    JG_CUDA(launch_pdl(k_g2s_legendre<T, 4>, g, threads, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, rc, slots, tabs, stage));
+  auto kernel = ql == 1 ? (stage ? k_g2s_legendre<T, 1, true> : k_g2s_legendre<T, 1, false>)
+                        : (stage ? k_g2s_legendre<T, 4, true> : k_g2s_legendre<T, 4, false>);
+  JG_CUDA(launch_pdl(kernel, g, threads, sm, st, gp, tb, (const V*)fbuf, m->ns, m->nlat, fp.C, ct, rc, slots, tabs));
   mark(st);
   JG_CUDA(cudaGetLastError());
   return JGCM_OK;
