@@ -453,10 +453,12 @@ __global__ void __launch_bounds__(256) k_fft(FFTPlan plan, Tables<T> tb, V2<T>* 
 // interleaved, i fastest: Julia's Array{ComplexF64,3}(nλ, nθ, L)).  Modes m < h as k_fft forms them,
 // the Nyquist mode X[h] = Re Z[0] - Im Z[0], and the modes above h by the Hermitian symmetry of a
 // real row, X[nλ - m] = conj X[m].  Same shared-memory transform and block shape as k_fft; this
-// serves the entry point only (the model steps read modes m <= N from k_fft and its variants).
+// serves the entry point only (the model steps read modes m <= N from k_fft and its variants).  A mode is
+// one 16-byte store: `out` may be the host's array, and two stores of 8 leave gaps in its sectors
+// (FP32, T63L20 132 -> 86 us, T85L20 159 -> 108).
 template <typename T>
 __global__ void __launch_bounds__(256) k_fourier_full(const T* __restrict__ grid, Tables<T> tb,
-                                                      double* __restrict__ out, int C, int nlat, int nlon,
+                                                      double2* __restrict__ out, int C, int nlat, int nlon,
                                                       int logh, int CT) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int h = nlon >> 1;
@@ -496,9 +498,7 @@ __global__ void __launch_bounds__(256) k_fourier_full(const T* __restrict__ grid
       xi = (ei + (tc * oi - ts * orr)) * scale;
     }
     if (t > h) xi = -xi;
-    const size_t o = (((size_t)c * nlat + j) * nlon + t) * 2;
-    out[o] = (double)xr;
-    out[o + 1] = (double)xi;
+    out[((size_t)c * nlat + j) * nlon + t] = make_double2((double)xr, (double)xi);
   }
 }
 
@@ -1748,11 +1748,11 @@ int fourier_full_to_host(jgcm_mesh* m, const void* d_grid, int L, double* d_dst,
   dim3 g((L + fc - 1) / fc, m->nlat);
   if (is_fp64(m)) {
     JG_TRY(configure_smem<double>());
-    k_fourier_full<double><<<g, 256, sm, st>>>((const double*)d_grid, tables<double>(m), d_dst, L, m->nlat,
+    k_fourier_full<double><<<g, 256, sm, st>>>((const double*)d_grid, tables<double>(m), (double2*)d_dst, L, m->nlat,
                                                m->nlon, m->logn - 1, fc);
   } else {
     JG_TRY(configure_smem<float>());
-    k_fourier_full<float><<<g, 256, sm, st>>>((const float*)d_grid, tables<float>(m), d_dst, L, m->nlat, m->nlon,
+    k_fourier_full<float><<<g, 256, sm, st>>>((const float*)d_grid, tables<float>(m), (double2*)d_dst, L, m->nlat, m->nlon,
                                               m->logn - 1, fc);
   }
   mark(st);
