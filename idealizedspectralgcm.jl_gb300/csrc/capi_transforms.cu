@@ -216,7 +216,10 @@ extern "C" int jgcm_trans_grid_to_fourier(jgcm_mesh* m, const double* pfield, in
   const size_t nf = 2 * grid_elems(m, nlev);  // complex [nlev][nlat][nlon]: staging slots 1 and 2
   const void* x;
   double* f;
-  JG_TRY(grid_in(m, 0, pfield, nlev, &x));
+  // the kernel reads rows and writes modes at once: a field that lies in the output array is copied first (the
+  // other calls write in place after everything has been read)
+  const bool overlap = pfield < fourier + nf && fourier < pfield + nf / 2;
+  JG_TRY(grid_in(m, 0, pfield, nlev, &x, overlap));
   JG_TRY(host_out(m, fourier, nf, slot(m, 1), &f));
   JG_TRY(fourier_full_to_host(m, x, nlev, f, m->stream));
   JG_TRY(host_out_done(fourier, f, nf, m->stream));
