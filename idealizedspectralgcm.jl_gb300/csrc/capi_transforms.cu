@@ -305,9 +305,9 @@ extern "C" int jgcm_add_horizontal_advection(jgcm_mesh* m, const double* hs, con
   JG_TRY(host_in(m, u, ng, slot(m, 1), m->stream, &pu));
   JG_TRY(host_in(m, v, ng, slot(m, 2), m->stream, &pv));
   JG_TRY(host_in(m, dh, ng, slot(m, 3), m->stream, &ph));
-  double* out;  // dh itself or its staged copy, updated in place
+  double* out;
   JG_TRY(host_out(m, dh, ng, slot(m, 3), &out));
-  JG_TRY(advection_update(m, m->d_grid[0], m->d_grid[1], pu, pv, out, ng, m->stream));
+  JG_TRY(advection_update(m, m->d_grid[0], m->d_grid[1], pu, pv, ph, out, ng, m->stream));
   JG_TRY(host_out_done(dh, out, ng, m->stream));
   return finish(m, call);
 }

@@ -381,9 +381,9 @@ int fourier_dev_to_host(jgcm_mesh* m, int L, double* d_dst, cudaStream_t st);
 // all nλ modes of fft/nλ of L device grid levels, FP64 host layout [L][nlat][nlon] complex
 int fourier_full_to_host(jgcm_mesh* m, const void* d_grid, int L, double* d_dst, cudaStream_t st);
 int apply_laplacian(jgcm_mesh* m, void* d_spec, int L, cudaStream_t st);
-// dh -= u gl + v gt, n values (gl, gt in the mesh's precision)
-int advection_update(jgcm_mesh* m, const void* gl, const void* gt, const double* u, const double* v, double* dh, size_t n,
-                     cudaStream_t st);
+// out = dh - (u gl + v gt), n values (gl, gt in the mesh's precision; out may be dh)
+int advection_update(jgcm_mesh* m, const void* gl, const void* gt, const double* u, const double* v, const double* dh,
+                     double* out, size_t n, cudaStream_t st);
 int area_mean(jgcm_mesh* m, const void* d_grid, double* d_out, cudaStream_t st);
 template <typename T>
 Tables<T> tables(const jgcm_mesh* m);

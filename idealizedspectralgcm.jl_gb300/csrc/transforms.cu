@@ -1685,16 +1685,21 @@ int grid_dev_to_host(jgcm_mesh* m, const void* src, double* dst, size_t n, cudaS
 // T21 31 -> 22 us).  Every page of the array is touched by this thread first: pages that were never written are mapped before the device
 // meets them, and an address that is not the process's to read or write faults here, in the calling
 // thread, as it did in the copy, and never on the device.  Arrays that are not 16-byte aligned (the
-// kernels move pairs), device pointers and other devices keep the copy.
-static bool host_direct(const jgcm_mesh* m, const void* p) {
-  if (!m->host_direct || ((uintptr_t)p & 15)) return false;
+// kernels move pairs), device pointers and other devices keep the copy; so do pageable results of more than
+// HOST_WRITE_MAX bytes, whose pages cost more, touched and translated, than the copy engine's pass (states, us,
+// copied and in place: 14 MB 104 and 100, 18 MB 126 and 126, 26 MB 166 and 170, 57 MB 339 and 369; in pinned
+// memory in place is faster throughout, 336 and 331 at 57 MB; as inputs too, 376 and 274).
+constexpr size_t HOST_WRITE_MAX = (size_t)16 << 20;
+enum class Host { other, pageable, pinned };  // other: not in place
+static Host host_direct(const jgcm_mesh* m, const void* p) {
+  if (!m->host_direct || ((uintptr_t)p & 15)) return Host::other;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return Host::other;
   }
-  return at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeManaged ||
-         (at.type == cudaMemoryTypeHost && at.devicePointer == p);
+  if (at.type == cudaMemoryTypeUnregistered || at.type == cudaMemoryTypeManaged) return Host::pageable;
+  return at.type == cudaMemoryTypeHost && at.devicePointer == p ? Host::pinned : Host::other;
 }
 static size_t page_bytes() {
   static const size_t b = (size_t)sysconf(_SC_PAGESIZE);
@@ -1702,7 +1707,7 @@ static size_t page_bytes() {
 }
 int host_in(jgcm_mesh* m, const double* src, size_t n, double* stage, cudaStream_t st, const double** use) {
   JG_ARG(src != nullptr, "input array is NULL");
-  if (host_direct(m, src)) {
+  if (host_direct(m, src) != Host::other) {
     const volatile char* p = (const volatile char*)src;
     for (size_t o = 0; o < n * 8; o += page_bytes()) (void)p[o];
     (void)p[n * 8 - 1];
@@ -1715,7 +1720,8 @@ int host_in(jgcm_mesh* m, const double* src, size_t n, double* stage, cudaStream
 }
 int host_out(jgcm_mesh* m, double* dst, size_t n, double* stage, double** use) {
   JG_ARG(dst != nullptr, "output array is NULL");
-  if (host_direct(m, dst)) {
+  const Host kind = host_direct(m, dst);
+  if (kind == Host::pinned || (kind == Host::pageable && n * 8 <= HOST_WRITE_MAX)) {
     volatile char* p = (volatile char*)dst;
     for (size_t o = 0; o < n * 8; o += page_bytes()) p[o] = p[o];
     p[n * 8 - 1] = p[n * 8 - 1];
@@ -1783,16 +1789,17 @@ int apply_laplacian(jgcm_mesh* m, void* d_spec, int L, cudaStream_t st) {
 
 // Add_Horizontal_Advection! (Spectral_Spherical_Mesh.jl:694-718) from the gradients of the advected field
 template <typename T>
-__global__ void k_adv_update(const T* gl, const T* gt, const double* u, const double* v, double* dh, size_t n) {
+__global__ void k_adv_update(const T* gl, const T* gt, const double* u, const double* v, const double* dh, double* out,
+                             size_t n) {
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-    dh[t] = dh[t] - (u[t] * (double)gl[t] + v[t] * (double)gt[t]);
+    out[t] = dh[t] - (u[t] * (double)gl[t] + v[t] * (double)gt[t]);
 }
-int advection_update(jgcm_mesh* m, const void* gl, const void* gt, const double* u, const double* v, double* dh, size_t n,
-                     cudaStream_t st) {
+int advection_update(jgcm_mesh* m, const void* gl, const void* gt, const double* u, const double* v, const double* dh,
+                     double* out, size_t n, cudaStream_t st) {
   if (is_fp64(m))
-    k_adv_update<double><<<nblk(n), 256, 0, st>>>((const double*)gl, (const double*)gt, u, v, dh, n);
+    k_adv_update<double><<<nblk(n), 256, 0, st>>>((const double*)gl, (const double*)gt, u, v, dh, out, n);
   else
-    k_adv_update<float><<<nblk(n), 256, 0, st>>>((const float*)gl, (const float*)gt, u, v, dh, n);
+    k_adv_update<float><<<nblk(n), 256, 0, st>>>((const float*)gl, (const float*)gt, u, v, dh, out, n);
   JG_CUDA(cudaGetLastError());
   return JGCM_OK;
 }

@@ -47,7 +47,8 @@ int grid_host_to_dev(jgcm_mesh*, const double*, void*, size_t, cudaStream_t) { r
 int grid_dev_to_host(jgcm_mesh*, const void*, double*, size_t, cudaStream_t) { return queue(); }
 int fourier_full_to_host(jgcm_mesh*, const void*, int, double*, cudaStream_t) { return queue(); }
 int apply_laplacian(jgcm_mesh*, void*, int, cudaStream_t) { return queue(); }
-int advection_update(jgcm_mesh*, const void*, const void*, const double*, const double*, double*, size_t, cudaStream_t) {
+int advection_update(jgcm_mesh*, const void*, const void*, const double*, const double*, const double*, double*, size_t,
+                     cudaStream_t) {
   return queue();
 }
 int area_mean(jgcm_mesh*, const void*, double*, cudaStream_t) { return queue(); }
