@@ -1243,10 +1243,10 @@ __global__ void __launch_bounds__(32 * IMPL_CW) k_hs_implicit_cols(const __grid_
   }
 }
 
-// From 108 columns per SM on (T42L20: 8 members 21 -> 23 us, 16 members 33 -> 31; 8 members of T63L20 34 -> 31,
-// 32 of T21L20 equal)
+// From 100 columns per SM on (kernel, us: T42L20, 8 members, 52 per SM, 21 -> 23, 16 members, 104 per SM, 32.6 -> 30.9;
+// 8 members of T63L20, 113 per SM, 34 -> 31; step: 56 members of T21L20, 101 per SM, 157.8 -> 156.6)
 inline bool impl_cols_pay(const jgcm_model* md) {
-  return (size_t)md->npairs * md->ne >= (size_t)108 * md->mesh->sm_count;
+  return (size_t)md->npairs * md->ne >= (size_t)100 * md->mesh->sm_count;
 }
 
 int launch_hs_implicit_cols(const ImplArgs<float>& a, const VertT<float>* vt, cudaStream_t st) {
