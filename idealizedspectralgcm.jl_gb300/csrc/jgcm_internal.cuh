@@ -402,7 +402,6 @@ size_t simt_smem_need(const jgcm_mesh* m, int s2g, int g2s, int fft);
 // member); the forward FFT of the plan first
 bool hs_analysis_fits(const jgcm_mesh* m, int nd, int E);
 int hs_tables_build(jgcm_mesh* m, int nd, int E);
-int hs_analysis_levels(const jgcm_mesh* m, int nd, int E);
 template <typename T>
 int launch_hs_analysis(jgcm_mesh* m, const FFTPlan& fp, int colU, int colV, int colE, int colT, int colP, int nd,
                        int E, void* dvor, void* ddiv, void* dt, void* dlnps, cudaStream_t st, void* fbuf, int cap);
