@@ -134,9 +134,18 @@ __device__ __forceinline__ void fft_row(T (&re)[FFTSplit<H>::R1], T (&im)[FFTSpl
   }
 }
 
+// x / c with rc = 1 / c at hand.  FP32: the product, within an ulp of the quotient.  FP64: the product corrected by
+// its residual, which the fused operation forms exactly (P. Markstein, IBM J. Res. Dev. 34, 1990): the quotient's own
+// rounding (none of 2e8 random pairs differed; the product alone differs in 27 %).  A product that is not finite
+// stays as it is.  T42L20's inverse 51 us, 47 with the bare product, 60 with divisions.
+__device__ __forceinline__ float quotient(float x, float, float rc) { return x * rc; }
+__device__ __forceinline__ double quotient(double x, double c, double rc) {
+  const double q = x * rc, z = fma(fma(-q, c, x), rc, q);
+  return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : z;
+}
+
 // The epilogue of a run of a row: x(λ_2i) = re[r], x(λ_2i+1) = im[r] for i = i0 + step r, the group's epilogue
-// chosen once per run and each pair of longitudes stored as one 8- or 16-byte word.  ÷cos θ as a product
-// with 1/cos θ (within an ulp of the quotient).
+// chosen once per run and each pair of longitudes stored as one 8- or 16-byte word.
 template <typename T, int V>
 __device__ __forceinline__ void ifft_store_row(const GridOutGroup& g, const Tables<T>& tb, int k, int j, int nlat,
                                                int nlon, const T (&re)[V], const T (&im)[V], int i0, int step) {
@@ -149,16 +158,17 @@ __device__ __forceinline__ void ifft_store_row(const GridOutGroup& g, const Tabl
     v.y = b;
     d[step * r] = v;
   };
+  const T c = tb.cosj[j], rc = (T)1 / c;
+  auto div_cos = [&](T x) -> T { return quotient(x, c, rc); };
   switch (g.epi) {
     case EPI_NONE:
 #pragma unroll
       for (int r = 0; r < V; r++) put(dst, r, re[r], im[r]);
       break;
-    case EPI_DIVCOS: {
-      const T rc = (T)1 / tb.cosj[j];
+    case EPI_DIVCOS:
 #pragma unroll
-      for (int r = 0; r < V; r++) put(dst, r, re[r] * rc, im[r] * rc);
-    } break;
+      for (int r = 0; r < V; r++) put(dst, r, div_cos(re[r]), div_cos(im[r]));
+      break;
     case EPI_EXP2: {
       const T sh = pick<T>(g.shift, g.shiftf), es = pick<T>(g.eshift, g.eshiftf);
       P* d2 = reinterpret_cast<P*>((T*)g.dst2 + row) + i0;
@@ -169,12 +179,11 @@ __device__ __forceinline__ void ifft_store_row(const GridOutGroup& g, const Tabl
       }
     } break;
     case EPI_DIVCOS_MULPS: {  // level k of ps
-      const T rc = (T)1 / tb.cosj[j];
       const P* ps = reinterpret_cast<const P*>((const T*)g.ps + row) + i0;
 #pragma unroll
       for (int r = 0; r < V; r++) {
         const P q = ps[step * r];
-        put(dst, r, (re[r] * rc) * q.x, (im[r] * rc) * q.y);
+        put(dst, r, div_cos(re[r]) * q.x, div_cos(im[r]) * q.y);
       }
     } break;
     case EPI_ADJ_G2S: {
