@@ -711,8 +711,9 @@ def run_jgcm(args):
         "dtype": "f32" if args.precision != "fp64" else "f64", "data": "synthetic",
         "config": {"workload": "Held-Suarez T42L20 (128x64 Gaussian, 20 sigma levels), dt 1200 s; 1 step = 1 "
                                "sim-day = 72 model steps",
-                   "precision": f"{args.precision} state/transforms/tendencies, fp64 semi-implicit solve and "
-                                f"global mass/energy sums",
+                   "precision": "fp64" if args.precision == "fp64" else
+                                f"{args.precision} state/transforms/tendencies; wave matrices and tables formed in "
+                                f"fp64, wave-matrix product and global mass/energy sums as fp32 pairs, folded in fp64",
                    "initial_state": "isothermal 264 K at rest, ps 1e5 Pa, reference vorticity seed, seeded "
                                     "N(0,0.1^2) K grid noise",
                    "l2": "flushed (256 MiB write) before every timed sim-day; working set ~20 MB is otherwise "

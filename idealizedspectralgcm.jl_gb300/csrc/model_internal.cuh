@@ -22,7 +22,7 @@ struct VertCoef {  // Vert_Coordinate (even_sigma) and the semi-implicit referen
   double dlp_m[JGCM_MAX_ND];   // ln p_k - ln p_{k-1/2}   (k >= 1)
   double dlp[JGCM_MAX_ND];     // ln p_{k+1/2} - ln p_{k-1/2}   (k >= 1)
   // Δa_k, Δb_k as FP32 pairs hi + lo (hi the FP32 rounding, lo that of the remainder): the FP32
-  // path forms the column sums of T_k Δa_k, T_k Δb_k to FP64 accuracy from them
+  // path forms the column sums of T_k Δa_k, T_k Δb_k as FP32 pairs (2^-48) from them
   float dak_hi[JGCM_MAX_ND], dak_lo[JGCM_MAX_ND], dbk_hi[JGCM_MAX_ND], dbk_lo[JGCM_MAX_ND];
 };
 // The same in the state precision T, rounded once on the host: a conversion in a kernel, like every FP64

@@ -9,7 +9,7 @@
 // pointer (Time_Advance!, Dyn_Data.jl:326-364, copies instead); steady steps are captured
 // once per rotation phase as CUDA graphs and replayed.  The semi-implicit wave matrices
 // (Semi_Implicit.jl:165-180) are inverted on the device in FP64, the per-(m,n) vertical
-// solve is applied to FP64 accuracy (on the FP32 path as FP32 pairs; a warp per spectral mode, or
+// solve is applied in FP64 (on the FP32 path as FP32 pairs, to ~2^-46; a warp per spectral mode, or
 // four columns per warp) and the mass/energy fixers (Spectral_Dynamics.jl:5-68) use deterministic
 // reductions folded in FP64.
 #include <cmath>
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(HS_CT, (sizeof(T) == 4 && S == 1) ? 14 : sizeo
     }
   // ---- pass 2, top-down within the segment
   // the column's energy integral (Compute_Corrections_Init): its kinetic part in the state precision,
-  // its c_p T part (~99 % of it) to FP64 accuracy (on the FP32 path the state precision's rounding of
+  // its c_p T part (~99 % of it) beyond it (on the FP32 path the state precision's rounding of
   // c_p T, the same at nearly every point of a near-uniform temperature, biased the energy correction
   // by up to 1e-6 K per step): FP64 sums of T_k Δa_k and T_k Δb_k on the FP64 path, the same sums as
   // FP32 pairs (error-free products and additions, ds_add_prod) on the FP32 path
@@ -667,7 +667,7 @@ int launch_hs_column(const HSColArgs<T>& a, const jgcm_mesh* m, int ne, int S, c
 // Semi-implicit correction (Adjust_δlnps_δt_δdiv! + Implicit_Correction!, Semi_Implicit.jl:
 // 271-513) followed by Compute_Spectral_Damping! and Filtered_Leapfrog! for vor, div, T, lnps
 // (Spectral_Dynamics.jl:313-327).  One warp per spectral mode (m,n), lane = level.  The
-// per-n solve with W_n = (I - ξ² ∇²_n D)^{-1} is formed to FP64 accuracy; the linearised vertical
+// per-n solve with W_n = (I - ξ² ∇²_n D)^{-1} is formed in FP64 or FP32 pairs; the linearised vertical
 // operators and the time filter run in the state precision T (FP64 on the FP64 path).
 template <typename T>
 struct ImplArgs {
@@ -771,14 +771,15 @@ __device__ __forceinline__ void lf(int init, int Dt, R rob, R d, R f, R& dq, R q
   }
 }
 
-// R is the precision of the vertical algebra, the state's.  The wave-matrix product is formed to FP64
-// accuracy in both: FP64 products and sums on the FP64 path; on the FP32 path, whose right-hand side and
-// result are FP32, W_n as pairs hi + lo and the row sums as pairs (ds_add_prod: error-free products and
-// additions, ~2^-46 of the sum of magnitudes before the result is rounded to FP32).  An FP64 instruction
+// R is the precision of the vertical algebra, the state's.  The wave-matrix product has FP64 products and
+// sums on the FP64 path; on the FP32 path, whose right-hand side and result are FP32, W_n as pairs
+// hi + lo and the row sums as pairs (ds_add_prod: error-free products and additions, ~2^-46 of the sum
+// of magnitudes before the result is rounded to FP32).  An FP64 instruction
 // holds a sub-partition for ~64 cycles, the pair's ten FP32 ones for ten: with FP64 products this kernel
 // was bound by them from a few members on (one column per warp, 128 x T21L20 95 -> 64 us, 32 x T42L20 90 -> 60 us,
-// one T42L20 member 11.4 -> 9.8 us, event included; the results against 64 bits as before: one member bit for bit,
-// the ensembles 2.4e-6 and 2.5e-6 in the worst field).
+// one T42L20 member 11.4 -> 9.8 us, event included).  Errors of a single step's outputs against the FP64 path, FP32
+// inputs, T21 to T63 with 7 to 32 levels, 60 runs: equal to four digits with FP64 products and with pairs (δ
+// divergence, the field that the product forms, 9.97e-8 rms and 1.245e-7 at most).
 // DENSE: the FP64 wave-matrix products of the block's modes are spread over all its threads, one
 // (mode, component, row) output each, instead of one mode per warp, whose 32 - nd idle lanes the
 // FP64 pipe executes all the same (for launches with many modes: member ensembles).
@@ -830,7 +831,7 @@ __global__ void __launch_bounds__(256) k_hs_implicit(ImplArgs<T> a, const VertT<
   R hk = vr.hk[k];
   ddiv.x = ddiv.x - eig * (gx + hk * l2.x);
   ddiv.y = ddiv.y - eig * (gy + hk * l2.y);
-  // wave-matrix solve in FP64, n <= N only (Implicit_Correction! :486-497)
+  // wave-matrix solve, n <= N only (Implicit_Correction! :486-497)
   if (DENSE) {
     __shared__ double s_b[8][2][JGCM_MAX_ND], s_o[8][2][JGCM_MAX_ND];
     if (act) {
@@ -1381,7 +1382,7 @@ __global__ void __launch_bounds__(256) k_hs_corr_reduce(CorrArgs<T> a, const Ver
   const size_t G = (size_t)a.nlat * a.nlon, col = (size_t)j * a.nlon + (act ? i : 0);
   const size_t offL = (size_t)e * nd * G, off1 = (size_t)e * G;
   // the energy integrals sum_k E_k Δa_k, sum_k E_k Δb_k (E = |u|²/2 + c_p T): the kinetic part in
-  // the state precision, the c_p T part (~99 %) to FP64 accuracy (the state precision's rounding of
+  // the state precision, the c_p T part (~99 %) beyond it (the state precision's rounding of
   // c_p T biased the energy correction by up to 1e-6 K per step): FP64 sums of the products T_k Δa_k,
   // T_k Δb_k on the FP64 path; on the FP32 path the same sums as FP32 pairs (error-free products
   // against Δ_hi + Δ_lo, error-free additions), each column's pair converted to FP64 once
@@ -2590,7 +2591,7 @@ int step_held_suarez(jgcm_model* md, cudaStream_t st) {
     ia.q_n = (V*)md->spe_q[n];
   }
   // vertical algebra in the state precision (FP64 algebra on the FP32 path measured no more
-  // accurate: its error is set by FP32 storage); the wave-matrix solve to FP64 accuracy in both
+  // accurate: its error is set by FP32 storage); the wave-matrix solve in FP64, on the FP32 path in pairs
   // 4 modes per block: (N+1)(N+2)/2 + N+1 modes at T42 make 248 blocks, every SM's FP64 units busy;
   // FP64 member ensembles (from 4 members) spread the FP64 products densely over each block, FP32 launches of
   // many columns take four of them per warp

@@ -1283,8 +1283,7 @@ static inline int reg_fft_threads(int nlon) { return nlon == 64 ? 4 : nlon <= 25
 // shared memory 35 and 66, split 27 and 47.  With few rows the split threads' longer chains show (T85 shallow
 // water FP32 a warp per row 8.3 and 8.3, split 11.9 and 10.2 us; FP64 shared 16 and 21, split 39 and 25):
 // FP64 launches of less than two warps an SM keep the shared-memory kernels, and in FP32 fields of one level
-// a warp per row -- whatever their number, so that the members of an ensemble are transformed by the kernel
-// of a model of one, rounding for rounding.
+// a warp per row, for an ensemble's members as for one (at nlon 64 until the rows ask for use_row_fft's kernels).
 template <typename T>
 static bool reg_fft(const jgcm_mesh* m, int C) {
   if (m->nlon < 64 || m->tune[3] != 0) return false;

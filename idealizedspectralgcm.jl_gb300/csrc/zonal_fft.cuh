@@ -158,17 +158,16 @@ __device__ __forceinline__ void ifft_store_row(const GridOutGroup& g, const Tabl
     v.y = b;
     d[step * r] = v;
   };
-  const T c = tb.cosj[j], rc = (T)1 / c;
-  auto div_cos = [&](T x) -> T { return quotient(x, c, rc); };
   switch (g.epi) {
     case EPI_NONE:
 #pragma unroll
       for (int r = 0; r < V; r++) put(dst, r, re[r], im[r]);
       break;
-    case EPI_DIVCOS:
+    case EPI_DIVCOS: {
+      const T c = tb.cosj[j], rc = (T)1 / c;
 #pragma unroll
-      for (int r = 0; r < V; r++) put(dst, r, div_cos(re[r]), div_cos(im[r]));
-      break;
+      for (int r = 0; r < V; r++) put(dst, r, quotient(re[r], c, rc), quotient(im[r], c, rc));
+    } break;
     case EPI_EXP2: {
       const T sh = pick<T>(g.shift, g.shiftf), es = pick<T>(g.eshift, g.eshiftf);
       P* d2 = reinterpret_cast<P*>((T*)g.dst2 + row) + i0;
@@ -179,11 +178,12 @@ __device__ __forceinline__ void ifft_store_row(const GridOutGroup& g, const Tabl
       }
     } break;
     case EPI_DIVCOS_MULPS: {  // level k of ps
+      const T c = tb.cosj[j], rc = (T)1 / c;
       const P* ps = reinterpret_cast<const P*>((const T*)g.ps + row) + i0;
 #pragma unroll
       for (int r = 0; r < V; r++) {
         const P q = ps[step * r];
-        put(dst, r, div_cos(re[r]) * q.x, div_cos(im[r]) * q.y);
+        put(dst, r, quotient(re[r], c, rc) * q.x, quotient(im[r], c, rc) * q.y);
       }
     } break;
     case EPI_ADJ_G2S: {

@@ -41,7 +41,8 @@ extern "C" {
 
 /* Precision modes (jgcm_mesh_create). */
 #define JGCM_FP64 0       /* all device arithmetic FP64 (the FP64 GPU path) */
-#define JGCM_FP32 1       /* FP32 state/transforms, FP64 tables, implicit solve and sums */
+#define JGCM_FP32 1       /* FP32 state/transforms; tables formed in FP64; wave-matrix product and global
+                             sums as FP32 pairs (kinetic energy FP32 within a column), folded in FP64 */
 #define JGCM_TF32X3 2     /* as FP32, Legendre contraction on tcgen05 tensor cores, 3xTF32 split */
 #define JGCM_BF16X3 3     /* as FP32, Legendre contraction on tcgen05, 3-term split-BF16 */
 
