@@ -1280,7 +1280,7 @@ static inline int reg_fft_threads(int nlon) { return nlon == 64 ? 4 : nlon <= 25
 // Which kernels transform the rows of a launch of C columns (tile knob 0): the register-split FFTs (nlon 64
 // to 1024) for fields of several levels.  T42L20, one member, FP32: a warp per row 9.0 and 12.4 us (forward and
 // inverse), split 8.8 and 8.5; 32 members 76 and 180, 38 and 76; T21L7, one member, equal (6.6 and 8.2).  FP64: in
-// shared memory 35 and 66, split 27 and 47.  With few rows the split threads' longer chains show (T85 shallow
+// shared memory 35 and 66, split 27 and 51.  With few rows the split threads' longer chains show (T85 shallow
 // water FP32 a warp per row 8.3 and 8.3, split 11.9 and 10.2 us; FP64 shared 16 and 21, split 39 and 25):
 // FP64 launches of less than two warps an SM keep the shared-memory kernels, and in FP32 fields of one level
 // a warp per row, for an ensemble's members as for one (at nlon 64 until the rows ask for use_row_fft's kernels).
@@ -1321,7 +1321,7 @@ static RegFFT reg_fft_shape(const jgcm_mesh* m, int C) {
   RegFFT r;
   // columns per block: 32 (256-byte runs of FP32 pairs), fewer where the rows would take more than 48 KB, the
   // grid would leave SMs without a block, or, in FP64 (bound by its arithmetic: small blocks spread evenly,
-  // T63L20 140 -> 133 us), a block would hold more than two warps; a warp at least
+  // T63L20 140 -> 133 us, 143 with the quotients), a block would hold more than two warps; a warp at least
   r.lcb = 5;
   while ((row << r.lcb) > 48 * 1024 || (sizeof(T) == 8 && (R2 << r.lcb) > 64)) r.lcb--;
   while ((R2 << r.lcb) > 32 && (size_t)((C + (1 << r.lcb) - 1) >> r.lcb) * m->nlat < (size_t)FFT_BLOCKS_PER_SM * m->sm_count)

@@ -11,8 +11,8 @@
 // dependency wait.  A block holds CB columns of one latitude, so that the Fourier side is read and written
 // in runs of CB consecutive columns, and walks column tiles.
 // Why this split: radix-2 in shared memory spent a pass, a barrier and full complex products per stage (FP64
-// T42L20 step: forward 35, inverse 66 us, bound by the FP64 pipe at 2300 FP64 instructions a row; 27 and 47
-// us here at 1650); a warp per row spent 20 shuffles per pair of points (FP32 T42L20, 32 members: forward 76
+// T42L20 step: forward 35, inverse 66 us, bound by the FP64 pipe at 2300 FP64 instructions a row; 27 and 51
+// us here at 1650 and the quotients); a warp per row spent 20 shuffles per pair of points (FP32 T42L20, 32 members: forward 76
 // us with the load-store pipe 97 % busy, 405 instructions a row; 38 us here, 75); a row per thread needs 152
 // registers at nlon 128 (inverse 90 us at 17 % of the warps; 76 us here).  Separate, conflict-free pitches
 // for the exchange, and the next tile's coefficients loaded ahead, measured no better (76 and 80 us).
