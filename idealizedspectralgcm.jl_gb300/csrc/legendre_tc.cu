@@ -747,6 +747,7 @@ int tc_status(jgcm_mesh* m) {
   JG_CUDA(cudaMemcpy(&s, m->d_status, sizeof(s), cudaMemcpyDeviceToHost));
   if (s) {
     JG_CUDA(cudaMemset(m->d_status, 0, sizeof(s)));
+    JG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // before a kernel on the mesh's (non-blocking) stream sets it
     set_error("tensor-core Legendre kernel gave up waiting (%s%s)", (s & 1u) ? "table copy " : "",
               (s & 2u) ? "MMA completion" : "");
     return JGCM_E_CUDA;

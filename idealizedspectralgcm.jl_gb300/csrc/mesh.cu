@@ -338,8 +338,9 @@ extern "C" int jgcm_mesh_create(int num_fourier, int num_spherical, int nlat, in
   MCHK(cuda(cudaMalloc(&m->d_costh, nlat * 8), "alloc"));
   MCHK(cuda(cudaMalloc(&m->d_qnm, T3 * 8), "alloc"));
   MCHK(cuda(cudaMalloc(&m->d_dqnm, T3 * 8), "alloc"));
-  MCHK(cuda(cudaMemset(m->d_qnm, 0, T3 * 8), "memset"));
-  MCHK(cuda(cudaMemset(m->d_dqnm, 0, T3 * 8), "memset"));
+  // (on the mesh's stream, like everything that follows: it does not wait for the legacy stream)
+  MCHK(cuda(cudaMemsetAsync(m->d_qnm, 0, T3 * 8, m->stream), "memset"));
+  MCHK(cuda(cudaMemsetAsync(m->d_dqnm, 0, T3 * 8, m->stream), "memset"));
   MCHK(alloc_store(m->t64, m->N, m->ns, nlat, nlon));
   MCHK(alloc_store(m->t32, m->N, m->ns, nlat, nlon));
   MCHK(mesh_build_tables(m));
@@ -353,15 +354,16 @@ extern "C" int jgcm_mesh_create(int num_fourier, int num_spherical, int nlat, in
   for (int i = 0; i < 4; i++) {
     MCHK(cuda(cudaMalloc(&m->d_grid[i], sg * ts), "alloc grid scratch"));
     MCHK(cuda(cudaMalloc(&m->d_spec[i], spec_elems(m, nd) * 2 * ts), "alloc spec scratch"));
-    MCHK(cuda(cudaMemset(m->d_spec[i], 0, spec_elems(m, nd) * 2 * ts), "memset"));
+    MCHK(cuda(cudaMemsetAsync(m->d_spec[i], 0, spec_elems(m, nd) * 2 * ts, m->stream), "memset"));
   }
   MCHK(cuda(cudaMalloc(&m->d_red, (size_t)(4 * nlat + 64) * 8), "alloc red"));
   MCHK(cuda(cudaMalloc(&m->d_counter, 64 * sizeof(unsigned int)), "alloc counter"));
-  MCHK(cuda(cudaMemset(m->d_counter, 0, 64 * sizeof(unsigned int)), "memset"));
+  MCHK(cuda(cudaMemsetAsync(m->d_counter, 0, 64 * sizeof(unsigned int), m->stream), "memset"));
   MCHK(cuda(cudaMalloc(&m->d_ref2, T3 * 8), "alloc ref2"));
   MCHK(cuda(cudaMalloc(&m->d_status, sizeof(unsigned int)), "alloc status"));
-  MCHK(cuda(cudaMemset(m->d_status, 0, sizeof(unsigned int)), "memset"));
+  MCHK(cuda(cudaMemsetAsync(m->d_status, 0, sizeof(unsigned int), m->stream), "memset"));
   if (precision == JGCM_TF32X3 || precision == JGCM_BF16X3) MCHK(tc_tables_build(m));
+  MCHK(cuda(cudaStreamSynchronize(m->stream), "mesh set-up"));
 #undef MCHK
   m->refs = 1;
   cudaGetDevice(&m->device);

@@ -1982,7 +1982,13 @@ __global__ void k_fill_coriolis(const double* sinth, T* f, int nlat, double omeg
   if (t < nlat) f[t] = (T)(2 * omega * sinth[t]);
 }
 
-int alloc(void** p, size_t bytes) {
+// Zeros and copies of alloc and cudaMemcpy are queued on the legacy stream, for which the meshes' (non-blocking) streams
+// do not wait: complete before a kernel on one of them may use what they fill
+int filled() {
+  JG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return JGCM_OK;
+}
+int alloc(void** p, size_t bytes) {  // zero-filled, once filled() has returned
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     set_error("cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
@@ -2047,6 +2053,7 @@ int build_wave(jgcm_model* md) {
   for (int n = 0; n <= N; n++) eig0[n] = (double)(-n * (n + 1)) / (m->radius * m->radius);
   JG_CUDA(cudaMemcpy(d_div, md->div_mat, nd * nd * 8, cudaMemcpyHostToDevice));
   JG_CUDA(cudaMemcpy(d_eig0, eig0.data(), (N + 1) * 8, cudaMemcpyHostToDevice));
+  JG_TRY(filled());
   const double a = md->P.implicit_coef;
   double xis[2] = {md->P.dt * a, (2 * md->P.dt) * a};  // Get_ξ for the init step and afterwards
   for (int s = 0; s < 2; s++) {
@@ -2130,6 +2137,7 @@ int model_alloc(jgcm_model* md) {
   JG_TRY(alloc(&md->dfac[1], (size_t)nt * ts));
   const double cf = md->P.damping_coef, dt1 = md->P.dt, dt2 = 2.0 * md->P.dt;
   const int od = md->P.damping_order, nb = (nt + 127) / 128;
+  JG_TRY(filled());
   if (is_fp64(m)) {
     k_fill_damping<double><<<nb, 128, 0, m->stream>>>(m->t64.eig, (double*)md->damping, N, ns, cf, od, 0.0);
     k_fill_damping<double><<<nb, 128, 0, m->stream>>>(m->t64.eig, (double*)md->dfac[0], N, ns, cf, od, dt1);
@@ -2153,6 +2161,7 @@ int model_alloc(jgcm_model* md) {
     JG_TRY(hs_tables_build(m, nd, ne));
     JG_TRY(build_wave(md));
   }
+  JG_TRY(filled());
   JG_CUDA(cudaStreamSynchronize(m->stream));
   return JGCM_OK;
 }
@@ -4077,6 +4086,7 @@ int adj_mats(jgcm_model* md, AdjMats* out) {
   *out = adj_mats_view(d, nd);
   JG_CUDA(cudaMemcpy(d, host.data(), nall * 8, cudaMemcpyHostToDevice));
   JG_CUDA(cudaMemcpy(out->Aptf, hostf.data(), nall * 4, cudaMemcpyHostToDevice));
+  JG_TRY(filled());
   return JGCM_OK;
 }
 
@@ -4227,6 +4237,7 @@ int si_alloc(jgcm_model* md, SIBuffers* b) {
   jgcm_mesh* m = md->mesh;
   const size_t ts = tsize(m), S = spec_elems(m, md->nd) * 2 * ts, S1 = spec_elems(m, 1) * 2 * ts;
   JG_TRY(alloc(&b->base, 20 * S));
+  JG_TRY(filled());
   for (int i = 0; i < 20; i++) b->f[i] = (char*)b->base + (size_t)i * S;
   (void)S1;
   return JGCM_OK;
@@ -4282,7 +4293,10 @@ ImplArgs<T> si_args(jgcm_model* md, void* const* in, void* const* out) {
 }  // namespace
 
 namespace jgcm {
-int dev_alloc(void** p, size_t bytes) { return alloc(p, bytes); }
+int dev_alloc(void** p, size_t bytes) {
+  JG_TRY(alloc(p, bytes));
+  return filled();
+}
 
 int model_step_async(jgcm_model* md) { return model_step(md); }
 
@@ -4458,6 +4472,7 @@ extern "C" int jgcm_model_diagnostics(jgcm_model* md, int on) {
   if (on) {
     if (!md->diag) JG_TRY(alloc((void**)&md->diag, n * 8));
     JG_CUDA(cudaMemset(md->diag, 0, n * 8));
+    JG_TRY(filled());
     md->diag_steps = 0;
   }
   if ((on != 0) != (md->diag_on != 0)) drop_graphs(md);  // the step graphs gain / lose the reduction
