@@ -4363,14 +4363,16 @@ extern "C" int jgcm_model_semi_implicit_step(jgcm_model* md, const double* const
     void* p;
     ~Free() { cudaFree(p); }
   } fr{b.base};
+  HostCall call(st);
   void* din[12];
   void* dout[8];
   for (int i = 0; i < 12; i++) din[i] = b.f[i];
   for (int i = 0; i < 8; i++) dout[i] = b.f[12 + i];
   for (int i = 0; i < 12; i++) {
     const size_t nn = 2 * spec_elems(m, si_levels_in(md, i));
-    JG_CUDA(cudaMemcpyAsync(m->d_stage, in[i], nn * 8, cudaMemcpyHostToDevice, st));
-    JG_TRY(spec_host_to_dev(m, m->d_stage, din[i], si_levels_in(md, i), st));
+    const double* p;
+    JG_TRY(host_in(m, in[i], nn, m->d_stage, st, &p));
+    JG_TRY(spec_host_to_dev(m, p, din[i], si_levels_in(md, i), st));
   }
   const size_t ts = tsize(m);
   JG_CUDA(cudaMemcpyAsync(dout[1], din[5], spec_elems(m, md->nd) * 2 * ts, cudaMemcpyDeviceToDevice, st));
@@ -4384,10 +4386,13 @@ extern "C" int jgcm_model_semi_implicit_step(jgcm_model* md, const double* const
   JG_CUDA(cudaGetLastError());
   for (int i = 0; i < 8; i++) {
     const size_t nn = 2 * spec_elems(m, si_levels_out(md, i));
-    JG_TRY(spec_dev_to_host(m, dout[i], m->d_stage, si_levels_out(md, i), st));
-    JG_CUDA(cudaMemcpyAsync(out[i], m->d_stage, nn * 8, cudaMemcpyDeviceToHost, st));
-    JG_CUDA(cudaStreamSynchronize(st));
+    double* p;
+    JG_TRY(host_out(m, out[i], nn, m->d_stage, &p));
+    JG_TRY(spec_dev_to_host(m, dout[i], p, si_levels_out(md, i), st));
+    JG_TRY(host_out_done(out[i], p, nn, st));
   }
+  JG_CUDA(cudaStreamSynchronize(st));
+  call.done = true;
   return JGCM_OK;
 }
 
@@ -4411,14 +4416,16 @@ extern "C" int jgcm_model_semi_implicit_step_adjoint(jgcm_model* md, const doubl
       cudaFree(q);
     }
   } fr{b.base, am.Apt};
+  HostCall call(st);
   void* dob[8];
   void* dib[12];
   for (int i = 0; i < 8; i++) dob[i] = b.f[i];
   for (int i = 0; i < 12; i++) dib[i] = b.f[8 + i];
   for (int i = 0; i < 8; i++) {
     const size_t nn = 2 * spec_elems(m, si_levels_out(md, i));
-    JG_CUDA(cudaMemcpyAsync(m->d_stage, out_bar[i], nn * 8, cudaMemcpyHostToDevice, st));
-    JG_TRY(spec_host_to_dev(m, m->d_stage, dob[i], si_levels_out(md, i), st));
+    const double* p;
+    JG_TRY(host_in(m, out_bar[i], nn, m->d_stage, st, &p));
+    JG_TRY(spec_host_to_dev(m, p, dob[i], si_levels_out(md, i), st));
   }
   auto launch = [&](auto tag) {
     using T = decltype(tag);
@@ -4453,10 +4460,13 @@ extern "C" int jgcm_model_semi_implicit_step_adjoint(jgcm_model* md, const doubl
   JG_CUDA(cudaGetLastError());
   for (int i = 0; i < 12; i++) {
     const size_t nn = 2 * spec_elems(m, si_levels_in(md, i));
-    JG_TRY(spec_dev_to_host(m, dib[i], m->d_stage, si_levels_in(md, i), st));
-    JG_CUDA(cudaMemcpyAsync(in_bar[i], m->d_stage, nn * 8, cudaMemcpyDeviceToHost, st));
-    JG_CUDA(cudaStreamSynchronize(st));
+    double* p;
+    JG_TRY(host_out(m, in_bar[i], nn, m->d_stage, &p));
+    JG_TRY(spec_dev_to_host(m, dib[i], p, si_levels_in(md, i), st));
+    JG_TRY(host_out_done(in_bar[i], p, nn, st));
   }
+  JG_CUDA(cudaStreamSynchronize(st));
+  call.done = true;
   return JGCM_OK;
 }
 
